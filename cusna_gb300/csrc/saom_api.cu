@@ -118,14 +118,17 @@ struct Facts {
   std::string spec, spec_w;
   JitPlan jplan;
   int flags = 0;
-  std::vector<int> kind, cfn, offd, offt;  // effect plan, k each
+  std::vector<int> kind, cfn, offd, offt;  // effect plan, k each (cfn packed: cfn_pack)
+  CounterSet cnt{};                        // two-path counters of the plan
   std::vector<int> tsize;                  // theta-table length per effect (0: none)
   // multi-network problems: one network's effects as a problem of their own
   bool multi = false;
   std::vector<int> cross_src;              // source network per effect (cross effects)
   std::vector<int> dci;                    // dyadic covariate index per effect (-1 none)
   std::vector<double> dyc;                 // the dyadic covariate, n*n (empty: none)
-  std::vector<double> pool;                // its tables
+  std::vector<double> pool;                // its tables (after 256 entries, exp_fx's in fixed point)
+  std::vector<uint64_t> poolq;             // the same in fixed point
+  std::vector<double> bound;               // bound on |d_e|, k
   int zlo = 0, zR = 1;
 };
 
@@ -202,7 +205,15 @@ cusna_status build_plan(const cusna_saom_problem *p, bool dev, Facts &F, bool on
   F.zR = (int)std::max<long long>(1, std::min<long long>(zR, 65536));
   F.kind.assign(k, K_GEN); F.cfn.assign(k, 0); F.offd.assign(k, 0); F.offt.assign(k, 0);
   F.tsize.assign(k, 0);
-  F.pool.clear();
+  F.pool.assign(256, 0.0);
+  F.poolq.assign(256, 0);
+  F.bound.assign(k, 1.0);
+  for (int x = 0; x < 256; ++x) {
+    const int2 t = exp_fx_entry(std::exp2(x / 256.0));
+    F.poolq[x] = (uint64_t)(uint32_t)t.x | (uint64_t)(uint32_t)t.y << 32;
+  }
+  std::vector<int> pk(k);
+  plan_counters(F.tid.data(), k, F.multi, F.multi ? F.cross_src.data() : nullptr, F.cnt, pk.data());
   auto add = [&](size_t cnt) { const size_t o = F.pool.size(); F.pool.resize(o + cnt, 0.0); return (int)o; };
   auto cnt_table = [&](int e, int cfn, size_t size) {
     F.kind[e] = K_CNT; F.cfn[e] = cfn;
@@ -215,7 +226,19 @@ cusna_status build_plan(const cusna_saom_problem *p, bool dev, Facts &F, bool on
   auto look_table = [&](int e, int cfn, size_t size, auto value) {
     F.kind[e] = K_LOOK; F.cfn[e] = cfn;
     F.offd[e] = add(size);
-    for (size_t x = 0; x < size; ++x) F.pool[F.offd[e] + x] = value(x);
+    double top = 0.0;
+    bool finite = true;
+    for (size_t x = 0; x < size; ++x) {
+      const double v = F.pool[F.offd[e] + x] = value(x);
+      top = std::max(top, std::fabs(v));
+      finite = finite && std::isfinite(v);
+    }
+    F.bound[e] = finite ? top : INFINITY;   // not finite: the chains run in float64
+    const double scale = std::ldexp(1.0, fx_scale(finite ? top : 1.0));
+    F.poolq.resize(F.pool.size(), 0);
+    for (size_t x = 0; x < size; ++x)
+      F.poolq[F.offd[e] + x] =
+          finite ? (uint64_t)(std::llrint(F.pool[F.offd[e] + x] * scale) + (1LL << 62)) : 0;
     if (uniform) {
       F.offt[e] = add(size);
       F.tsize[e] = (int)size;
@@ -227,6 +250,21 @@ cusna_status build_plan(const cusna_saom_problem *p, bool dev, Facts &F, bool on
   for (int e = 0; e < k; ++e) {
     const int t = F.tid[e];
     const double *v = &vm[(size_t)e * n];
+    double vmax = 0.0, wmax = 0.0;
+    bool finite = std::isfinite(p1[e]) && std::isfinite(p2[e]);
+    if (dyn[e]) {
+      vmax = std::max(std::fabs((double)lo - zbar), std::fabs((double)hi - zbar));
+    } else {
+      for (int j = 0; j < n; ++j) {
+        vmax = std::max(vmax, std::fabs(v[j]));
+        finite = finite && std::isfinite(v[j]);
+      }
+    }
+    for (int j = 0; j <= n; ++j) {
+      wmax = std::max(wmax, std::fabs(wt[(size_t)e * (n + 1) + j]));
+      finite = finite && std::isfinite(wt[(size_t)e * (n + 1) + j]);
+    }
+    F.bound[e] = finite ? effect_bound(t, n, vmax, wmax, p1[e], p2[e]) : INFINITY;
     switch (t) {
       case 0: cnt_table(e, 0, 2); break;
       case 1: cnt_table(e, 1, 2); break;
@@ -276,23 +314,41 @@ cusna_status build_plan(const cusna_saom_problem *p, bool dev, Facts &F, bool on
         // cross-network effects read another network of a multi-network
         // problem; a single-network problem has none, and the reference's
         // change statistic of these types there is 0
-        if (F.multi) { F.kind[e] = K_CROSS; F.cfn[e] = t; F.offd[e] = F.cross_src[e]; }
+        if (F.multi && t == 36 && p1[e] >= 2.0) {   // the square root of the count
+          look_table(e, 8, N + 1, [](size_t c) { return std::sqrt((double)c); });
+        } else if (F.multi) { F.kind[e] = K_CROSS; F.cfn[e] = t; F.offd[e] = F.cross_src[e]; }
         else F.kind[e] = K_ZERO;
         break;
       case 24: look_table(e, 8, N + 1, [&](size_t c) { return wt[(size_t)e * (n + 1) + c]; }); break;
-      case 26: look_table(e, 9, N + 1, [&](size_t c) { return wt[(size_t)e * (n + 1) + c]; }); break;
-      case 27: look_table(e, 10, N + 1, [&](size_t c) { return wt[(size_t)e * (n + 1) + c]; }); break;
-      case 28: look_table(e, 11, N + 1, [&](size_t c) { return wt[(size_t)e * (n + 1) + c]; }); break;
+      case 26: look_table(e, 8, N + 1, [&](size_t c) { return wt[(size_t)e * (n + 1) + c]; }); break;
+      case 27: look_table(e, 8, N + 1, [&](size_t c) { return wt[(size_t)e * (n + 1) + c]; }); break;
+      case 28: look_table(e, 8, N + 1, [&](size_t c) { return wt[(size_t)e * (n + 1) + c]; }); break;
       case 32:
         // interactions are formed from their components in the single-network
         // engine; the multi-network change statistic of the type is 0
         if (F.multi) F.kind[e] = K_ZERO;
         break;
-      case 13: case 29: case 30: break;  // K_GEN
+      case 29: case 30:
+        // K_GEN with the differences of the weights in fixed point (gw_fixed)
+        if (finite) {
+          F.cfn[e] = 16;
+          F.offd[e] = add(N);
+          F.poolq.resize(F.pool.size(), 0);
+          double top = 0.0;
+          const double *w = &wt[(size_t)e * (n + 1)];
+          for (size_t x = 0; x < N; ++x) top = std::max(top, std::fabs(w[x + 1] - w[x]));
+          F.bound[e] = 1.001 * top * (double)N;
+          const double scale = std::ldexp(1.0, fx_scale(F.bound[e]));
+          for (size_t x = 0; x < N; ++x)
+            F.poolq[F.offd[e] + x] = (uint64_t)(int64_t)std::llrint((w[x + 1] - w[x]) * scale);
+        }
+        break;
+      case 13: break;  // K_GEN
       default: F.kind[e] = K_ZERO; break;       // unknown ids: the reference's 0
     }
   }
-  if (F.pool.empty()) F.pool.push_back(0.0);
+  // the counters each effect reads beside its count function or table index
+  for (int e = 0; e < k; ++e) F.cfn[e] = (pk[e] & ~0xFF) | F.cfn[e];
   if (uniform) fl |= F_THETA_TAB;
   if (has_z) fl |= F_HAS_Z;
   F.flags |= fl;
@@ -351,19 +407,12 @@ cusna_status validate(const cusna_saom_problem *p, const cusna_saom_result *r, b
   for (int e = 0; e < k; ++e) {
     const int t = F.tid[e];
     switch (t) {
-      case 2: fl |= F_PC_RI_CJ | F_PC_RI_RJ; break;
-      case 3: case 23: fl |= F_PC_RJ_CI; break;
       case 5: fl |= F_NEED_TP; break;
-      case 6: fl |= F_PC_RI_CJ | F_PC_RICIRJ; break;
       case 19:
         // the multi-network engine passes a reciprocated degree of 0
         // (src/libcusna_saom_cpu.cpp:510)
         if (!F.multi) fl |= F_NEED_RDEG;
         break;
-      case 24: fl |= F_PC_RI_CJ; break;
-      case 26: fl |= F_PC_RI_RJ; break;
-      case 27: fl |= F_PC_CI_CJ; break;
-      case 28: fl |= F_PC_CI_RJ; break;
       case 29: fl |= F_NEED_GW29; break;
       case 30: fl |= F_NEED_GW30; break;
       case 32:
@@ -381,16 +430,8 @@ cusna_status validate(const cusna_saom_problem *p, const cusna_saom_result *r, b
   if ((s = build_plan(p, dev, F, one_row)) != CUSNA_OK) return s;
   {
     JitPlan &J = F.jplan;
-    J.pc_flags = F.flags & (F_PC_RI_CJ | F_PC_RI_RJ | F_PC_RJ_CI | F_PC_CI_CJ | F_PC_CI_RJ |
-                            F_PC_RICIRJ);
     J.kind = F.kind; J.cfn = F.cfn; J.tid = F.tid; J.ety = F.ety;
     J.i0 = F.i0; J.i1 = F.i1; J.i2 = F.i2;
-    if (!F.multi) {
-      F.spec = jit_spec_source(J);
-      J.n = p->n;
-      F.spec_w = jit_spec_source(J);
-      J.n = 0;
-    }
   }
   // gwdsp change statistics index the weight table at p+1 with p <= n-2 on a
   // network without self-ties; a self-tie in the start network could push p to
@@ -420,10 +461,10 @@ struct RawSizes {
 
 // Device layout of one prepared problem.
 struct ProbBufs {
-  size_t x0T, x0cT, simT, simcT, kdistT, permT, keepT, forceT, keepcT, forcecT;
+  size_t x0r, x0c, simr, simc, kdistr, permr, keepr, forcer, keepc, forcec;
   size_t vmat, wtab, p1, p2, vb, ralpha, ru;
   size_t etypes, dyn, i0, i1, i2, act, z0, bkdist, inact, vmiss;
-  size_t ekind, ecfn, eoffd, eofft, pool, pool2;
+  size_t ekind, ecfn, eoffd, eofft, pool, poolq, bound, c0;
   // raw copies (host mode)
   size_t r_x0, r_sim, r_kd, r_pm, r_keep, r_force, r_theta, r_lam, r_lamb, r_thetab, r_tid,
       r_ety, r_dyn, r_i0, r_i1, r_i2, r_vmat64, r_vmat32, r_wtab64, r_wtab32, r_p164, r_p132,
@@ -435,6 +476,11 @@ struct ProbBufs {
 };
 
 const size_t NONE = ~(size_t)0;
+
+// Counts of a problem's matrices.
+size_t counts_words(const CounterSet &C, int n) {
+  return __builtin_popcount(C.mask) * cm_size(n);
+}
 
 struct Job {
   const cusna_saom_problem *p;
@@ -453,9 +499,9 @@ void plan_problem(Planner &pl, Job &J, bool dev) {
   const size_t n = p->n, W = p->W, k = p->k, M = p->M, kb = p->kb, nr = p->nrate;
   const size_t bits = W * n * 4;
   ProbBufs &B = J.B;
-  B.x0T = pl.take(bits); B.x0cT = pl.take(bits); B.simT = pl.take(bits); B.simcT = pl.take(bits);
-  B.kdistT = pl.take(bits); B.permT = pl.take(bits); B.keepT = pl.take(bits);
-  B.forceT = pl.take(bits); B.keepcT = pl.take(bits); B.forcecT = pl.take(bits);
+  B.x0r = pl.take(bits); B.x0c = pl.take(bits); B.simr = pl.take(bits); B.simc = pl.take(bits);
+  B.kdistr = pl.take(bits); B.permr = pl.take(bits); B.keepr = pl.take(bits);
+  B.forcer = pl.take(bits); B.keepc = pl.take(bits); B.forcec = pl.take(bits);
   B.vmat = pl.take(k * n * 8); B.wtab = pl.take(k * (n + 1) * 8);
   B.p1 = pl.take(k * 8); B.p2 = pl.take(k * 8); B.vb = pl.take(n * 8);
   B.ralpha = pl.take((nr + 1) * 8); B.ru = pl.take((nr + 1) * n * 8);
@@ -465,7 +511,9 @@ void plan_problem(Planner &pl, Job &J, bool dev) {
   B.vmiss = NONE;
   B.ekind = pl.take(k * 4); B.ecfn = pl.take(k * 4); B.eoffd = pl.take(k * 4);
   B.eofft = pl.take(k * 4); B.pool = pl.take(J.F.pool.size() * 8);
-  B.pool2 = pl.take(J.F.pool.size() * 8);
+  B.poolq = pl.take(J.F.pool.size() * 8);
+  B.bound = pl.take(k * 8);
+  B.c0 = J.F.cnt.mask ? pl.take(counts_words(J.F.cnt, p->n) * 2) : NONE;
   if (!dev) {
     B.r_x0 = pl.take(n * W * 4);
     B.r_sim = maybe(pl, p->sim_out, n * W * 4);
@@ -583,12 +631,12 @@ cusna_status prepare(Job &J, bool dev, DevProblem &D, uint32_t chain_offset) {
   if (s != CUSNA_OK) return s;
 
   // canonical word-major networks
-  CU(launch_prep_bits(x0, n, W, at<uint32_t>(B.x0T), at<uint32_t>(B.x0cT), 0, st));
-  CU(launch_prep_bits(sim ? sim : x0, n, W, at<uint32_t>(B.simT), at<uint32_t>(B.simcT), 0, st));
-  CU(launch_prep_bits(kd, n, W, at<uint32_t>(B.kdistT), nullptr, 1, st));
-  CU(launch_prep_bits(pm, n, W, at<uint32_t>(B.permT), nullptr, 1, st));
-  CU(launch_prep_bits(kp, n, W, at<uint32_t>(B.keepT), at<uint32_t>(B.keepcT), 1, st));
-  CU(launch_prep_bits(fo, n, W, at<uint32_t>(B.forceT), at<uint32_t>(B.forcecT), 2, st));
+  CU(launch_prep_bits(x0, n, W, at<uint32_t>(B.x0r), at<uint32_t>(B.x0c), 0, st));
+  CU(launch_prep_bits(sim ? sim : x0, n, W, at<uint32_t>(B.simr), at<uint32_t>(B.simc), 0, st));
+  CU(launch_prep_bits(kd, n, W, at<uint32_t>(B.kdistr), nullptr, 1, st));
+  CU(launch_prep_bits(pm, n, W, at<uint32_t>(B.permr), nullptr, 1, st));
+  CU(launch_prep_bits(kp, n, W, at<uint32_t>(B.keepr), at<uint32_t>(B.keepc), 1, st));
+  CU(launch_prep_bits(fo, n, W, at<uint32_t>(B.forcer), at<uint32_t>(B.forcec), 2, st));
   // float64 descriptors
   CU(launch_prep_desc(vm64, vm32, (size_t)k * n, at<double>(B.vmat), st));
   CU(launch_prep_desc(wt64, wt32, (size_t)k * (n + 1), at<double>(B.wtab), st));
@@ -638,11 +686,11 @@ cusna_status prepare(Job &J, bool dev, DevProblem &D, uint32_t chain_offset) {
   D.ralpha = at<double>(B.ralpha); D.ru = at<double>(B.ru);
   D.act = at<int>(B.act); D.inact = at<uint32_t>(B.inact);
   D.z0 = at<int>(B.z0); D.bkdist = at<int>(B.bkdist);
-  D.x0T = at<uint32_t>(B.x0T); D.x0cT = at<uint32_t>(B.x0cT);
-  D.simT = at<uint32_t>(B.simT); D.simcT = at<uint32_t>(B.simcT);
-  D.kdistT = at<uint32_t>(B.kdistT); D.permT = at<uint32_t>(B.permT);
-  D.keepT = at<uint32_t>(B.keepT); D.forceT = at<uint32_t>(B.forceT);
-  D.keepcT = at<uint32_t>(B.keepcT); D.forcecT = at<uint32_t>(B.forcecT);
+  D.x0r = at<uint32_t>(B.x0r); D.x0c = at<uint32_t>(B.x0c);
+  D.simr = at<uint32_t>(B.simr); D.simc = at<uint32_t>(B.simc);
+  D.kdistr = at<uint32_t>(B.kdistr); D.permr = at<uint32_t>(B.permr);
+  D.keepr = at<uint32_t>(B.keepr); D.forcer = at<uint32_t>(B.forcer);
+  D.keepc = at<uint32_t>(B.keepc); D.forcec = at<uint32_t>(B.forcec);
   D.lam = lam; D.theta = theta; D.lamb = lamb; D.thetab = thetab;
   D.prow = 1;
   CU(cudaMemcpyAsync(at<int>(B.ekind), J.F.kind.data(), (size_t)k * 4, cudaMemcpyHostToDevice, st));
@@ -650,20 +698,13 @@ cusna_status prepare(Job &J, bool dev, DevProblem &D, uint32_t chain_offset) {
   CU(cudaMemcpyAsync(at<int>(B.eoffd), J.F.offd.data(), (size_t)k * 4, cudaMemcpyHostToDevice, st));
   CU(cudaMemcpyAsync(at<int>(B.eofft), J.F.offt.data(), (size_t)k * 4, cudaMemcpyHostToDevice, st));
   CU(cudaMemcpyAsync(at<double>(B.pool), J.F.pool.data(), J.F.pool.size() * 8, cudaMemcpyHostToDevice, st));
-  {
-    // lookup values as double-float pairs: the float32 rounding (the float32
-    // pass) and the float32 rounding of the remainder (the score sums); a
-    // pageable copy is staged before cudaMemcpyAsync returns, so the local
-    // vector may go
-    std::vector<float> p2(2 * J.F.pool.size());
-    for (size_t x = 0; x < J.F.pool.size(); ++x) {
-      p2[2 * x] = (float)J.F.pool[x];
-      p2[2 * x + 1] = (float)(J.F.pool[x] - (double)p2[2 * x]);
-    }
-    CU(cudaMemcpyAsync(at<float>(B.pool2), p2.data(), p2.size() * 4, cudaMemcpyHostToDevice, st));
-  }
+  J.F.poolq.resize(J.F.pool.size(), 0);
+  CU(cudaMemcpyAsync(at<uint64_t>(B.poolq), J.F.poolq.data(), J.F.poolq.size() * 8, cudaMemcpyHostToDevice, st));
+  CU(cudaMemcpyAsync(at<double>(B.bound), J.F.bound.data(), (size_t)k * 8, cudaMemcpyHostToDevice, st));
   D.ekind = at<int>(B.ekind); D.ecfn = at<int>(B.ecfn); D.eoffd = at<int>(B.eoffd);
-  D.eofft = at<int>(B.eofft); D.tab = at<double>(B.pool); D.tab2 = at<float2>(B.pool2);
+  D.eofft = at<int>(B.eofft); D.cnt = J.F.cnt;
+  D.c0 = B.c0 == NONE ? nullptr : at<uint16_t>(B.c0); D.tab = at<double>(B.pool);
+  D.tabq = at<uint64_t>(B.poolq); D.ebound = at<double>(B.bound);
   auto out = [&](void *user, size_t off) -> void * {
     if (!user) return nullptr;
     return dev ? user : (off == NONE ? nullptr : at<char>(off));
@@ -719,6 +760,59 @@ cusna_status fetch_outputs(Job &J) {
   return CUSNA_OK;
 }
 
+// Chooses which two-path counters the chains hold as matrices. A popcount takes
+// W words per alter, a matrix one read per alter and, per toggle, one update for
+// each tie of the two actors: from kCountsMinW words on the matrices win (the figures
+// below), if the resident teams' matrices stay within
+// kCountsMaxBytes of device memory.
+constexpr int kCountsMinW = 12;
+constexpr size_t kCountsMaxBytes = (size_t)8 << 30;
+constexpr size_t kResidentTeams = 152 * 32;
+void choose_counts(std::vector<Job> &jobs, long long total_units, int nets) {
+  size_t per_team = 0;
+  for (Job &J : jobs) {
+    CounterSet &C = J.F.cnt;
+    C.mask = 0;
+    if (J.p->W >= kCountsMinW)
+      for (int c = 0; c < C.n; ++c)
+        if (C.list[c] == CL_OUT || C.list[c] == CL_IN || C.list[c] >= CL_NET) C.mask |= 1u << c;
+    per_team = std::max(per_team, counts_words(C, J.p->n) * 2 * nets);
+  }
+  const size_t teams = std::min<size_t>((size_t)total_units, kResidentTeams);
+  const bool fits = per_team * teams <= kCountsMaxBytes;
+  if (!fits)
+    for (Job &J : jobs) J.F.cnt.mask = 0;
+  std::vector<const CounterSet *> all;
+  for (Job &J : jobs) all.push_back(&J.F.cnt);
+  for (size_t q = 0; q < jobs.size(); ++q) {
+    Job &J = jobs[q];
+    if (nets > 1) {
+      counter_tasks(all.data(), nets, (int)q, J.F.cnt);
+    } else {
+      counter_tasks(&all[q], 1, 0, J.F.cnt);
+    }
+    JitPlan &P = J.F.jplan;
+    P.cnt = J.F.cnt;
+    if (J.F.multi) continue;
+    J.F.spec = jit_spec_source(P);
+    P.n = J.p->n;
+    J.F.spec_w = jit_spec_source(P);
+    P.n = 0;
+  }
+}
+
+// What the problems of a launch need in a team's slice beside their sizes.
+struct Needs {
+  bool tp = false, gw = false, tq = false;
+  size_t counts = 0;   // count matrices per team, in counts
+  void add(const Facts &F, int n) {
+    tp |= (F.flags & F_NEED_TP) != 0;
+    gw |= (F.flags & F_NEED_GW29) != 0;
+    tq |= (F.flags & F_NEED_GW30) != 0;
+    counts = std::max(counts, counts_words(F.cnt, n));
+  }
+};
+
 // ---- launch-shape autotuner ---------------------------------------------------
 // The simulator is bound by the float64 pipe, whose instructions have long
 // latencies, so the shape that wins keeps the most warps resident per SM while
@@ -728,8 +822,8 @@ cusna_status fetch_outputs(Job &J) {
 // memory, registers and warps all count). The score is the number of warps that
 // will be busy: min(resident teams, chains) * G per SM, capped at 48; ties go to
 // smaller teams (fewer barriers) and to in-rows in shared memory.
-std::vector<LaunchShape> rank_shapes(int nmax, int Wmax, int kmax, int kbmax, int nrmax, bool tp,
-                                     bool gw, bool tq, long long total_units, int force_G,
+std::vector<LaunchShape> rank_shapes(int nmax, int Wmax, int kmax, int kbmax, int nrmax,
+                                     const Needs &nd, long long total_units, int force_G,
                                      int force_tpc, int nets = 1,
                                      const JitKernel *jk = nullptr, bool valid = false) {
   const Ctx &c = g_ctx;
@@ -738,21 +832,20 @@ std::vector<LaunchShape> rank_shapes(int nmax, int Wmax, int kmax, int kbmax, in
   for (int gi = 0; gi < 5; ++gi) {
     const int G = Gs[gi];
     if (force_G && G != force_G) continue;
-    // placements: everything in shared memory; the in-rows in global scratch
-    // (L1-cached; a candidate even when shared memory suffices, as it frees
-    // shared memory for more chains per SM); the out-rows too, only when
-    // neither of the first two fits
-    bool placed = false;
+    // placements: everything in shared memory; the in-rows in global scratch;
+    // the out-rows too (both L1- and L2-cached: a ministep reads the focal
+    // actor's rows and one row per neighbour, so leaving them outside frees
+    // shared memory for more chains per SM, which pays most where a chain's
+    // rows alone fill an SM)
     for (int place = 0; place < 3; ++place) {
-      if (place == 2 && placed) break;
       const bool rows_smem = place < 2, cols_smem = place == 0;
       LaunchShape sh{};
       sh.G = G;
       sh.cols_in_smem = cols_smem;
       sh.rows_in_smem = rows_smem;
-      sh.lay = make_layout(nmax, Wmax, kmax, kbmax, nrmax, G, rows_smem, cols_smem, tp, gw, tq);
+      sh.lay = make_layout(nmax, Wmax, kmax, kbmax, nrmax, G, rows_smem, cols_smem, nd.tp, nd.gw,
+                           nd.tq);
       if (sh.lay.bytes * nets > (size_t)c.smem_optin) continue;
-      bool any = false;
       for (int tpc = 1; tpc <= 16; tpc *= 2) {
         if (force_tpc && tpc != force_tpc) continue;
         const int threads = 32 * G * tpc;
@@ -774,9 +867,7 @@ std::vector<LaunchShape> rank_shapes(int nmax, int Wmax, int kmax, int kbmax, in
         const long long want = (total_units + tpc - 1) / tpc;
         x.ctas = (int)std::max<long long>(1, std::min<long long>((long long)c.sms * per_sm, want));
         all.push_back({score, x});
-        any = true;
       }
-      placed |= any;
     }
   }
   std::stable_sort(all.begin(), all.end(),
@@ -819,12 +910,13 @@ bool tuning_enabled() {
   return on;
 }
 
-TuneKey tune_key(int nmax, int Wmax, int kmax, int kbmax, int nrmax, bool tp, bool gw, bool tq,
+TuneKey tune_key(int nmax, int Wmax, int kmax, int kbmax, int nrmax, const Needs &nd,
                  long long units, bool jit = false) {
   TuneKey k;
   std::memset(&k, 0, sizeof k);
   k.dev = g_ctx.device; k.nmax = nmax; k.Wmax = Wmax; k.kmax = kmax; k.kbmax = kbmax;
-  k.nrmax = nrmax; k.flags = (tp ? 1 : 0) | (gw ? 2 : 0) | (tq ? 4 : 0) | (jit ? 8 : 0);
+  k.nrmax = nrmax; k.flags = (nd.tp ? 1 : 0) | (nd.gw ? 2 : 0) | (nd.tq ? 4 : 0) | (jit ? 8 : 0) |
+                              (nd.counts ? 16 : 0);
   k.units = units;
   return k;
 }
@@ -860,8 +952,8 @@ bool jit_for(const std::vector<Job> &jobs, int spec_mode, JitKernel *jk) {
 
 // the model's two best shapes of each team size, in the model's order
 // Two candidates per team size G, in the model's order: its best shape for
-// that G and the best with the other placement of the in-rows (shared memory
-// or global scratch), or without one its second best.
+// that G and the best with another placement of the rows and in-rows (shared
+// memory or global scratch), or without one its second best.
 std::vector<LaunchShape> tuning_candidates(const std::vector<LaunchShape> &ranked) {
   std::vector<LaunchShape> c;
   for (size_t i = 0; i < ranked.size(); ++i) {
@@ -872,7 +964,8 @@ std::vector<LaunchShape> tuning_candidates(const std::vector<LaunchShape> &ranke
     c.push_back(first);
     const LaunchShape *second = nullptr;
     for (size_t j = i + 1; j < ranked.size() && !second; ++j)
-      if (ranked[j].G == first.G && ranked[j].cols_in_smem != first.cols_in_smem)
+      if (ranked[j].G == first.G && (ranked[j].cols_in_smem != first.cols_in_smem ||
+                                     ranked[j].rows_in_smem != first.rows_in_smem))
         second = &ranked[j];
     for (size_t j = i + 1; j < ranked.size() && !second; ++j)
       if (ranked[j].G == first.G) second = &ranked[j];
@@ -935,14 +1028,12 @@ cusna_status run_jobs(std::vector<Job> &jobs, bool dev, cusna_gpu_options *opts,
   const uint32_t off0 = opts ? opts->chain_offset : 0;
   const long long launches0 = kernel_launches();
   int nmax = 0, Wmax = 0, kmax = 0, kbmax = 0, nrmax = 0;
-  bool tp = false, gw = false, tq = false;
+  Needs nd;
   long long total = 0;
   for (auto &J : jobs) {
     nmax = std::max(nmax, J.p->n); Wmax = std::max(Wmax, J.p->W); kmax = std::max(kmax, J.p->k);
     kbmax = std::max(kbmax, J.p->kb); nrmax = std::max(nrmax, J.p->nrate);
-    tp |= (J.F.flags & F_NEED_TP) != 0;
-    gw |= (J.F.flags & (F_NEED_GW29 | F_NEED_TP)) != 0;
-    tq |= (J.F.flags & F_NEED_GW30) != 0;
+    nd.add(J.F, J.p->n);
     total += J.p->M;
   }
   const bool valid = vo != nullptr;
@@ -952,7 +1043,7 @@ cusna_status run_jobs(std::vector<Job> &jobs, bool dev, cusna_gpu_options *opts,
   // the validation build is the library kernel's
   const bool use_jit = !valid && jit_for(jobs, opts ? opts->specialise : 0, &jk);
   std::vector<LaunchShape> ranked =
-      rank_shapes(nmax, Wmax, kmax, kbmax, nrmax, tp, gw, tq, total, fG, fT, 1,
+      rank_shapes(nmax, Wmax, kmax, kbmax, nrmax, nd, total, fG, fT, 1,
                   use_jit ? &jk : nullptr, valid);
   if (ranked.empty()) {
     set_err("no launch shape fits n=%d in shared memory", nmax);
@@ -961,7 +1052,7 @@ cusna_status run_jobs(std::vector<Job> &jobs, bool dev, cusna_gpu_options *opts,
   // a forced shape is used as given; otherwise the autotuner picks (and may be
   // timing one of its candidates in this call)
   int trial = -1;
-  const TuneKey tkey = tune_key(nmax, Wmax, kmax, kbmax, nrmax, tp, gw, tq, total, use_jit);
+  const TuneKey tkey = tune_key(nmax, Wmax, kmax, kbmax, nrmax, nd, total, use_jit);
   const LaunchShape sh = (fG || fT || valid) ? ranked[0]
                                              : tuner_pick(tkey, tuning_candidates(ranked), &trial);
   Planner pl;
@@ -979,6 +1070,7 @@ cusna_status run_jobs(std::vector<Job> &jobs, bool dev, cusna_gpu_options *opts,
   const size_t cols_words = (size_t)Wmax * nmax;
   const size_t o_cols = sh.cols_in_smem ? NONE : pl.take(teams * cols_words * 4);
   const size_t o_rows = sh.rows_in_smem ? NONE : pl.take(teams * cols_words * 4);
+  const size_t o_counts = nd.counts ? pl.take(teams * nd.counts * 2) : NONE;
   if ((s = ensure_arena(pl.off)) != CUSNA_OK) return s;
 
   std::vector<DevProblem> hp(jobs.size());
@@ -1009,17 +1101,17 @@ cusna_status run_jobs(std::vector<Job> &jobs, bool dev, cusna_gpu_options *opts,
   CU(cudaMemcpyAsync(at<char>(o_units), units.data(), sizeof(long long) * units.size(),
                      cudaMemcpyHostToDevice, st));
   CU(cudaMemsetAsync(at<char>(o_counter), 0, sizeof(unsigned long long), st));
+  const Scratch sc{o_cols == NONE ? nullptr : at<uint32_t>(o_cols),
+                   o_rows == NONE ? nullptr : at<uint32_t>(o_rows),
+                   o_counts == NONE ? nullptr : at<uint16_t>(o_counts), cols_words, nd.counts};
+  if (nd.counts) CU(launch_counts_init(at<DevProblem>(o_probs), (int)jobs.size(), nmax, false, st));
   CU(cudaEventRecord(g_ctx.ev0, st));
   if (use_jit)
     CU(launch_period_jit(jk, sh, at<DevProblem>(o_probs), at<long long>(o_units), (int)jobs.size(),
-                         total, at<unsigned long long>(o_counter),
-                         o_cols == NONE ? nullptr : at<uint32_t>(o_cols),
-                         o_rows == NONE ? nullptr : at<uint32_t>(o_rows), cols_words, st));
+                         total, at<unsigned long long>(o_counter), sc, st));
   else
     CU(launch_period(sh, at<DevProblem>(o_probs), at<long long>(o_units), (int)jobs.size(), total,
-                     at<unsigned long long>(o_counter),
-                     o_cols == NONE ? nullptr : at<uint32_t>(o_cols),
-                     o_rows == NONE ? nullptr : at<uint32_t>(o_rows), cols_words, st, valid));
+                     at<unsigned long long>(o_counter), sc, st, valid));
   CU(cudaEventRecord(g_ctx.ev1, st));
   if (!dev)
     for (auto &J : jobs)
@@ -1042,6 +1134,12 @@ cusna_status run_jobs(std::vector<Job> &jobs, bool dev, cusna_gpu_options *opts,
 
 void order_longest_first(std::vector<Job> &jobs);
 
+long long total_chains(const std::vector<Job> &jobs) {
+  long long t = 0;
+  for (const Job &J : jobs) t += J.p->M;
+  return t;
+}
+
 cusna_status simulate(const cusna_saom_problem *problems, cusna_saom_result *results, int count,
                       cusna_gpu_options *opts) {
   if (!problems || !results) { set_err("problem or result is NULL"); return CUSNA_ERR_NULL_ARG; }
@@ -1063,6 +1161,7 @@ cusna_status simulate(const cusna_saom_problem *problems, cusna_saom_result *res
   }
   if ((s = ensure_ctx()) != CUSNA_OK) return s;
   order_longest_first(jobs);
+  choose_counts(jobs, total_chains(jobs), 1);
   s = run_jobs(jobs, dev, opts);
   if (s == CUSNA_OK && opts) {
     long long tot = 0;
@@ -1150,7 +1249,7 @@ cusna_status simulate_multi(const cusna_saom_multi_problem *pb, cusna_saom_multi
   }
   std::vector<Job> jobs(D);
   int kmax = 0;
-  bool tp = false, gw = false, tq = false;
+  Needs nd;
   for (int d = 0; d < D; ++d) {
     MultiNet &N = nets[d];
     goff[d + 1] = goff[d] + (int)N.eidx.size();
@@ -1200,10 +1299,9 @@ cusna_status simulate_multi(const cusna_saom_multi_problem *pb, cusna_saom_multi
     cusna_status s = validate(&N.q, &N.r, false, F);
     if (s != CUSNA_OK) return s;
     kmax = std::max(kmax, kd);
-    tp |= (F.flags & F_NEED_TP) != 0;
-    gw |= (F.flags & (F_NEED_GW29 | F_NEED_TP)) != 0;
-    tq |= (F.flags & F_NEED_GW30) != 0;
   }
+  choose_counts(jobs, M, D);
+  for (const Job &J : jobs) nd.add(J.F, n);
   // the multi-network kernel specialised to the networks' effect plans
   std::vector<JitPlan> jplans;
   for (int d = 0; d < D; ++d) {
@@ -1224,14 +1322,14 @@ cusna_status simulate_multi(const cusna_saom_multi_problem *pb, cusna_saom_multi
   JitKernel jk;
   const bool use_jit = jit_get(mspec, &jk);
   const std::vector<LaunchShape> ranked =
-      rank_shapes(n, W, kmax, 0, 0, tp, gw, tq, M, 0, 0, D, use_jit ? &jk : nullptr);
+      rank_shapes(n, W, kmax, 0, 0, nd, M, 0, 0, D, use_jit ? &jk : nullptr);
   if (ranked.empty()) {
     set_err("no launch shape fits %d networks of n=%d", D, n);
     return CUSNA_ERR_UNSUPPORTED;
   }
   // the autotuner as for single networks, under a key of its own (the
   // network count in the flags)
-  TuneKey tkey = tune_key(n, W, kmax, 0, 0, tp, gw, tq, M, use_jit);
+  TuneKey tkey = tune_key(n, W, kmax, 0, 0, nd, M, use_jit);
   tkey.flags |= (D << 8) | (1 << 7);
   int trial = -1;
   const LaunchShape sh = tuner_pick(tkey, tuning_candidates(ranked), &trial);
@@ -1250,6 +1348,7 @@ cusna_status simulate_multi(const cusna_saom_multi_problem *pb, cusna_saom_multi
   const size_t cols_words = (size_t)W * n;
   const size_t o_cols = sh.cols_in_smem ? NONE : pl.take(teams * D * cols_words * 4);
   const size_t o_rows = sh.rows_in_smem ? NONE : pl.take(teams * D * cols_words * 4);
+  const size_t o_counts = nd.counts ? pl.take(teams * D * nd.counts * 2) : NONE;
   if ((s = ensure_arena(pl.off)) != CUSNA_OK) return s;
   std::vector<DevProblem> hp(D);
   for (int d = 0; d < D; ++d)
@@ -1272,15 +1371,15 @@ cusna_status simulate_multi(const cusna_saom_multi_problem *pb, cusna_saom_multi
   CU(cudaMemcpyAsync(at<char>(o_lam), pb->lam, (size_t)M * D * 4, cudaMemcpyHostToDevice, st));
   CU(cudaMemcpyAsync(at<char>(o_gidx), gidx.data(), (size_t)k * 4, cudaMemcpyHostToDevice, st));
   CU(cudaMemsetAsync(at<char>(o_counter), 0, sizeof(unsigned long long), st));
+  const Scratch sc{o_cols == NONE ? nullptr : at<uint32_t>(o_cols),
+                   o_rows == NONE ? nullptr : at<uint32_t>(o_rows),
+                   o_counts == NONE ? nullptr : at<uint16_t>(o_counts), cols_words, nd.counts};
+  if (nd.counts) CU(launch_counts_init(at<DevProblem>(o_probs), (int)jobs.size(), n, true, st));
   CU(cudaEventRecord(g_ctx.ev0, st));
   if (use_jit)
-    CU(launch_multi_jit(jk, sh, at<DevProblem>(o_probs), md, M, at<unsigned long long>(o_counter),
-                        o_cols == NONE ? nullptr : at<uint32_t>(o_cols),
-                        o_rows == NONE ? nullptr : at<uint32_t>(o_rows), cols_words, st));
+    CU(launch_multi_jit(jk, sh, at<DevProblem>(o_probs), md, M, at<unsigned long long>(o_counter), sc, st));
   else
-    CU(launch_multi(sh, at<DevProblem>(o_probs), md, M, at<unsigned long long>(o_counter),
-                    o_cols == NONE ? nullptr : at<uint32_t>(o_cols),
-                    o_rows == NONE ? nullptr : at<uint32_t>(o_rows), cols_words, st));
+    CU(launch_multi(sh, at<DevProblem>(o_probs), md, M, at<unsigned long long>(o_counter), sc, st));
   CU(cudaEventRecord(g_ctx.ev1, st));
   auto get = [&](void *dst, size_t off, size_t bytes) -> cusna_status {
     if (!dst || off == NONE) return CUSNA_OK;
@@ -1319,8 +1418,7 @@ struct cusna_saom_plan {
   cusna::PlanTable *tabs = nullptr;
   int count = 0, n_tabs = 0;
   long long total = 0;
-  uint32_t *cols = nullptr, *rows = nullptr;
-  size_t cols_words = 0;
+  cusna::Scratch sc;   // the parts that some candidate shape keeps in global memory
   cudaGraphExec_t graph = nullptr;
   // autotuning over the first launches (one timed trial per candidate shape)
   std::vector<cusna::LaunchShape> cand;
@@ -1364,24 +1462,23 @@ cusna_status plan_create(const cusna_saom_problem *problems, cusna_saom_result *
     if (!one) jobs[q].F.flags &= ~F_THETA_TAB;
   }
   order_longest_first(jobs);
+  choose_counts(jobs, total_chains(jobs), 1);
   int nmax = 0, Wmax = 0, kmax = 0, kbmax = 0, nrmax = 0;
-  bool tp = false, gw = false, tq = false;
+  Needs nd;
   long long total = 0;
   for (auto &J : jobs) {
     nmax = std::max(nmax, J.p->n); Wmax = std::max(Wmax, J.p->W); kmax = std::max(kmax, J.p->k);
     kbmax = std::max(kbmax, J.p->kb); nrmax = std::max(nrmax, J.p->nrate);
-    tp |= (J.F.flags & F_NEED_TP) != 0;
-    gw |= (J.F.flags & (F_NEED_GW29 | F_NEED_TP)) != 0;
-    tq |= (J.F.flags & F_NEED_GW30) != 0;
+    nd.add(J.F, J.p->n);
     total += J.p->M;
   }
   const std::vector<LaunchShape> ranked =
-      rank_shapes(nmax, Wmax, kmax, kbmax, nrmax, tp, gw, tq, total, 0, 0);
+      rank_shapes(nmax, Wmax, kmax, kbmax, nrmax, nd, total, 0, 0);
   if (ranked.empty()) { set_err("no launch shape fits n=%d", nmax); return CUSNA_ERR_UNSUPPORTED; }
   std::vector<LaunchShape> cand = tuning_candidates(ranked);
   {
     // a signature the tuner has settled needs no exploration
-    const TuneKey key = tune_key(nmax, Wmax, kmax, kbmax, nrmax, tp, gw, tq, total);
+    const TuneKey key = tune_key(nmax, Wmax, kmax, kbmax, nrmax, nd, total);
     std::lock_guard<std::mutex> lk(g_tune_mu);
     for (auto &e : g_tune)
       if (std::memcmp(&e.key, &key, sizeof key) == 0 && e.next >= e.cand.size() && e.best >= 0)
@@ -1412,6 +1509,7 @@ cusna_status plan_create(const cusna_saom_problem *problems, cusna_saom_result *
   const size_t cols_words = (size_t)Wmax * nmax;
   const size_t o_cols = cols_global ? pl.take(teams * cols_words * 4) : NONE;
   const size_t o_rows = rows_global ? pl.take(teams * cols_words * 4) : NONE;
+  const size_t o_counts = nd.counts ? pl.take(teams * nd.counts * 2) : NONE;
 
   cusna_saom_plan *P = new cusna_saom_plan();
   P->cand = cand;
@@ -1459,6 +1557,8 @@ cusna_status plan_create(const cusna_saom_problem *problems, cusna_saom_result *
   if (e == cudaSuccess && !tabs.empty()) e = up(o_tabs, tabs.data(), sizeof(PlanTable) * tabs.size());
   if (e == cudaSuccess) e = cudaMemsetAsync(at<char>(o_counter), 0, 8, st);
   if (e == cudaSuccess) e = cudaMemsetAsync(at<char>(o_epoch), 0, 8, st);
+  if (e == cudaSuccess && nd.counts)
+    e = launch_counts_init(at<DevProblem>(o_probs), count, nmax, false, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) {
     set_err("plan: staging failed: %s", cudaGetErrorString(e));
@@ -1475,9 +1575,9 @@ cusna_status plan_create(const cusna_saom_problem *problems, cusna_saom_result *
   P->count = count;
   P->n_tabs = (int)tabs.size();
   P->total = total;
-  P->cols = o_cols == NONE ? nullptr : at<uint32_t>(o_cols);
-  P->rows = o_rows == NONE ? nullptr : at<uint32_t>(o_rows);
-  P->cols_words = cols_words;
+  P->sc = Scratch{o_cols == NONE ? nullptr : at<uint32_t>(o_cols),
+                  o_rows == NONE ? nullptr : at<uint32_t>(o_rows),
+                  o_counts == NONE ? nullptr : at<uint16_t>(o_counts), cols_words, nd.counts};
   P->spec = launch_spec(jobs);
   *out = P;
   return CUSNA_OK;
@@ -1488,14 +1588,13 @@ cusna_status plan_create(const cusna_saom_problem *problems, cusna_saom_result *
 cusna_status plan_enqueue(cusna_saom_plan *P, const LaunchShape &sh, cudaStream_t st) {
   CU(launch_plan_prologue(P->probs, P->seeds, P->count, P->epoch, P->tabs, P->n_tabs, st));
   CU(cudaMemsetAsync(P->counter, 0, sizeof(unsigned long long), st));
+  Scratch sc = P->sc;
+  if (sh.cols_in_smem) sc.cols = nullptr;
+  if (sh.rows_in_smem) sc.rows = nullptr;
   if (P->jit)
-    CU(launch_period_jit(P->jk, sh, P->probs, P->units, P->count, P->total, P->counter,
-                         sh.cols_in_smem ? nullptr : P->cols, sh.rows_in_smem ? nullptr : P->rows,
-                         P->cols_words, st));
+    CU(launch_period_jit(P->jk, sh, P->probs, P->units, P->count, P->total, P->counter, sc, st));
   else
-    CU(launch_period(sh, P->probs, P->units, P->count, P->total, P->counter,
-                     sh.cols_in_smem ? nullptr : P->cols, sh.rows_in_smem ? nullptr : P->rows,
-                     P->cols_words, st));
+    CU(launch_period(sh, P->probs, P->units, P->count, P->total, P->counter, sc, st));
   return CUSNA_OK;
 }
 
@@ -1630,6 +1729,7 @@ CUSNA_API cusna_status cusna_saom_simulate_period_validate(const cusna_saom_prob
   if (s != CUSNA_OK) return s;
   if ((s = ensure_ctx()) != CUSNA_OK) return s;
   std::vector<Job> jobs(1, J);
+  choose_counts(jobs, total_chains(jobs), 1);
   return run_jobs(jobs, false, nullptr, vo);
 }
 
@@ -1648,12 +1748,15 @@ CUSNA_API cusna_status cusna_saom_specialise_check(const cusna_saom_problem *pro
   cusna_saom_result dummy;
   std::memset(&dummy, 0, sizeof dummy);
   dummy.struct_version = CUSNA_ABI_VERSION;
-  Facts F;
-  cusna_status s = validate(problem, &dummy, false, F);
+  std::vector<Job> jobs(1);
+  jobs[0].p = problem;
+  jobs[0].r = &dummy;
+  cusna_status s = validate(problem, &dummy, false, jobs[0].F);
   if (s != CUSNA_OK) return s;
+  choose_counts(jobs, problem->M, 1);
   std::string text;
   double sec = 0.0;
-  const int st = jit_compile_only(F.spec_w, &text, &sec);
+  const int st = jit_compile_only(jobs[0].F.spec_w, &text, &sec);
   if (seconds) *seconds = sec;
   if (log && log_len) {
     const size_t m = std::min(log_len - 1, text.size());

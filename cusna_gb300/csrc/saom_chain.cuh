@@ -1,23 +1,52 @@
 // saom_chain.cuh -- one chain of one period, run by a team of G warps.
 // Restates src/libcusna_saom_cpu.cpp:142-303 (simulate_one) and :394-422 (the
-// per-chain outputs) over word-major bitsets.
+// per-chain outputs) over bitsets.
 #pragma once
 #include "saom_kernel.cuh"
 #include "saom_stats.cuh"
 
 namespace cusna {
 
+// The actor and word counts: constants where a specialised build fixes them.
+__device__ __forceinline__ int prob_n(const DevProblem &P) {
+#ifdef CUSNA_JIT_N
+  return CUSNA_JIT_N;
+#else
+  return P.n;
+#endif
+}
+__device__ __forceinline__ int prob_w(const DevProblem &P) {
+#ifdef CUSNA_JIT_N
+  return (CUSNA_JIT_N + 31) / 32;
+#else
+  return P.W;
+#endif
+}
+__device__ __forceinline__ int prob_k(const DevProblem &P) {
+#ifdef CUSNA_JIT_K
+  return CUSNA_JIT_K;
+#else
+  return P.k;
+#endif
+}
+
+// exp_fx's table into the CTA's shared memory (every thread of the CTA calls).
+__device__ __forceinline__ void load_exp_table(int2 *etab, const DevProblem *probs) {
+  const int2 *src = reinterpret_cast<const int2 *>(probs[0].tabq);
+  for (int x = threadIdx.x; x < 256; x += blockDim.x) etab[x] = src[x];
+  __syncthreads();
+}
+
 // Load the chain's start state and parameters into the team slice.
 __device__ __forceinline__ void chain_init(const Team &T, const DevProblem &P, const Slice &S,
                                            int c) {
   const int n = P.n, W = P.W, k = P.k, L = T.L;
   for (int x = T.tl; x < W * n; x += L) {
-    S.rowsT[x] = P.simT[x];
-    S.colsT[x] = P.simcT[x];
+    S.rows[x] = P.simr[x];
+    S.cols[x] = P.simc[x];
   }
   for (int e = T.tl; e < k; e += L) {
-    S.th32[e] = P.theta[(size_t)c * P.prow * k + e];
-    S.th[e] = (double)S.th32[e];
+    S.th[e] = (double)P.theta[(size_t)c * P.prow * k + e];
     S.sc[e] = 0.0;
     S.tid[e] = P.type_ids[e];
     S.ety[e] = P.etypes[e];
@@ -41,55 +70,103 @@ __device__ __forceinline__ void chain_init(const Team &T, const DevProblem &P, c
     S.rsc[q] = 0.0;
     S.rkind[q] = P.rkind[q];
   }
+  if (P.cnt.mask) {
+    // the count matrices' start values, 16 bytes per access
+    const size_t words = __popc(P.cnt.mask) * cm_size(n) / 8;
+    const uint4 *src = reinterpret_cast<const uint4 *>(P.c0);
+    uint4 *dst = reinterpret_cast<uint4 *>(S.cm);
+    size_t x = T.tl;
+    for (; x + 3 * (size_t)L < words; x += 4 * (size_t)L) {
+      const uint4 a = src[x], b = src[x + L], c4 = src[x + 2 * L], e4 = src[x + 3 * L];
+      dst[x] = a;
+      dst[x + L] = b;
+      dst[x + 2 * L] = c4;
+      dst[x + 3 * L] = e4;
+    }
+    for (; x < words; x += L) dst[x] = src[x];
+  }
   if (P.flags & F_HAS_Z)
     for (int x = T.tl; x < n; x += L) S.z[x] = P.z0[x];
   if (P.nrate > 0)
     for (int x = T.tl; x < n; x += L) S.crate[x] = 1.0;
-  if (T.tl == 0) {
-    S.misc[12] = -1;  // last ministep whose score sums need the float64 path
-    S.misc[13] = c;   // the chain's index within its problem (validation words)
-  }
+  if (T.tl == 0) S.misc[13] = c;   // the chain's index within its problem (validation words)
   T.sync();
+  if (T.tl == 0) {
+    // fixed-point scales, classes and parameters; the pass over the alters needs
+    // every |f_j| < 2^14 (S.fx[1]), else the chain runs on the float64 path
+    int64_t f0 = 0;
+    double range = 0.0;
+    for (int e = 0; e < k; ++e) {
+      const int kind = S.ekind[e];
+      const int cls = fx_class(kind, S.ecfn[e] & 0xFF, S.tid[e], S.ety[e]);
+      double bound = P.ebound[e];
+      int sd = fx_scale(bound);
+      if (S.tid[e] == 32 && kind != K_ZERO) {   // products: bounds and scales of the components
+        bound = __dmul_rn(S.dstar[S.i0[e]], S.dstar[S.i1[e]]);
+        sd = S.esd[S.i0[e]] + S.esd[S.i1[e]] - 64;
+        if (S.i2[e] >= 0) {
+          bound = __dmul_rn(bound, S.dstar[S.i2[e]]);
+          sd += S.esd[S.i2[e]] - 64;
+        }
+      }
+      S.dstar[e] = bound;
+      S.esd[e] = sd;
+      S.ecls[e] = cls | (S.th[e] < 0.0 ? 256 : 0);
+      if (cls != FX_ZERO) range = __dadd_rn(range, __dmul_rn(fabs(S.th[e]), bound));
+    }
+    const bool in_range = range < 16384.0;      // false for a NaN
+    if (in_range)
+      for (int e = 0; e < k; ++e) {
+        S.thq[e] = theta_fx(S.th[e], S.ecls[e] & 0xFF, S.esd[e]);
+        if ((S.ecls[e] & 0xFF) == FX_DELTA) f0 += (int64_t)S.thq[e];
+        // the part of a real magnitude's 2^62, for every alter alike
+        if ((S.ecls[e] & 0xFF) == FX_UNI || ((S.ecls[e] & 0xFF) == FX_REAL && S.ety[e] == 0))
+          f0 += base_fx(S.thq[e], S.ecls[e]);
+      }
+    S.fx[0] = f0;
+    S.fx[1] = in_range;
+  }
   for (int x = T.tl; x < n; x += L) {
     int od = 0, id = 0;
     for (int w = 0; w < W; ++w) {
-      od += __popc(S.rowsT[w * n + x]);
-      id += __popc(S.colsT[w * n + x]);
+      od += __popc(S.rows[w * n + x]);
+      id += __popc(S.cols[w * n + x]);
     }
     S.outdeg[x] = od;
     S.indeg[x] = id;
   }
   T.sync();
-}
-
-// Per-ministep helper arrays: transTies two-path counts and masks, gwdsp counts.
-__device__ __forceinline__ void step_helpers(const Team &T, const DevProblem &P, const Slice &S,
-                                             int i) {
-  const int n = P.n, W = P.W;
-  const bool tp = (P.flags & (F_NEED_TP | F_NEED_GW29)) != 0;
-  const bool tq = (P.flags & F_NEED_GW30) != 0;
-  if (!tp && !tq) return;
-  for (int h = T.tl; h < n; h += T.L) {
-    int a = 0, b = 0;
-    for (int w = 0; w < W; ++w) {
-      const uint32_t ri = S.rowsT[w * n + i];
-      if (tp) a += __popc(ri & S.colsT[w * n + h]);
-      if (tq) b += __popc(ri & S.rowsT[w * n + h]);
-    }
-    if (tp) S.tp[h] = a;
-    if (tq) S.tq[h] = b;
+  // largest degrees, kept up (never lowered) by the toggles: the bound on a
+  // count in step_guard
+  int mo = 0, mi = 0;
+  for (int x = T.tl; x < n; x += L) {
+    mo = max(mo, (int)S.outdeg[x]);
+    mi = max(mi, (int)S.indeg[x]);
+  }
+  mo = (int)team_max_ll(T, mo, S.red);
+  mi = (int)team_max_ll(T, mi, S.red);
+  if (T.tl == 0) {
+    S.misc[10] = mi;
+    S.misc[11] = mo;
   }
   T.sync();
-  if (P.flags & F_NEED_TP) {
-    // masks {h : tp_h == 0} and {h : tp_h == 1}, word-parallel via ballots
-    for (int hb = 32 * T.warp; hb < W * 32; hb += T.L) {
-      const int h = hb + T.lane;
-      const int v = h < n ? S.tp[h] : -1;
-      const uint32_t z0 = __ballot_sync(kFull, v == 0), z1 = __ballot_sync(kFull, v == 1);
-      if (T.lane == 0) { S.tpeq[hb >> 5] = z0; S.tpeq[W + (hb >> 5)] = z1; }
-    }
-    T.sync();
+}
+
+// Per-ministep helper arrays: transTies masks, gwdsp counts as integers per
+// actor. Complete for the whole team on return.
+__device__ __forceinline__ void step_helpers(const Team &T, const DevProblem &P, const Slice &S,
+                                             const StepCtx &X) {
+  const int n = prob_n(P), W = prob_w(P), fl = P.flags;
+  if (fl & F_NEED_TP) tp_masks(T, P, S, X, n, W, P.cnt.tp);
+  if (fl & F_NEED_GW29) {
+    const CountRow R = count_row(P, S, X, n, W, P.cnt.tp);
+    for (int h = T.tl; h < n; h += T.L) S.tp[h] = count_of(R, n, W, h);
   }
+  if (fl & F_NEED_GW30) {
+    const CountRow R = count_row(P, S, X, n, W, P.cnt.tq);
+    for (int h = T.tl; h < n; h += T.L) S.tq[h] = count_of(R, n, W, h);
+  }
+  if (fl & (F_NEED_TP | F_NEED_GW29 | F_NEED_GW30)) T.sync();
 }
 
 // The four Philox words of ministep ms, counter (ms, chain, 0, 0) as the
@@ -111,12 +188,12 @@ __device__ __forceinline__ void step_words(const DevProblem &P, const Slice &S, 
 // (ms, chain, 1, j) (src/libcusna_saom_cpu.cpp:266), or the caller's word.
 template <bool VALID>
 __device__ __forceinline__ uint32_t alter_word(const DevProblem &P, const Slice &S, long long ms,
-                                               uint32_t chain, int j) {
+                                               uint32_t chain, int j, uint32_t k0, uint32_t k1) {
   if (VALID && P.ustream && ms < P.ustream_steps)
     return P.ustream[((size_t)S.misc[13] * P.ustream_steps + (size_t)ms) * (4 + (size_t)P.n) + 4 +
                      (size_t)j];
   uint32_t ph[4];
-  philox10((uint32_t)ms, chain, 1u, (uint32_t)j, P.k0, P.k1, ph);
+  philox10((uint32_t)ms, chain, 1u, (uint32_t)j, k0, k1, ph);
   return ph[0];
 }
 
@@ -131,7 +208,7 @@ static __device__ int beh_step(const DevProblem &P, const Slice &S, int i, uint3
   long long nb = 0, nh = 0, ne = 0, nl = 0;
   double zs = 0.0;
   for (int w = 0; w < W; ++w) {
-    uint32_t m = S.rowsT[w * n + i];
+    uint32_t m = S.rows[w * n + i];
     while (m) {
       const int j = (w << 5) + __ffs(m) - 1;
       m &= m - 1;
@@ -275,122 +352,31 @@ __device__ __forceinline__ void keytop_merge(KeyTop &a, const KeyTop &c) {
     a.ub2 = fmaxf(fmaxf(a.ub2, c.ub2), __fadd_rn(c.b1, c.e1));
   }
 }
-__device__ __forceinline__ KeyTop team_keytop(const Team &T, KeyTop x, double *red) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    KeyTop y;
-    y.b1 = __shfl_xor_sync(kFull, x.b1, o);
-    y.e1 = __shfl_xor_sync(kFull, x.e1, o);
-    y.ub2 = __shfl_xor_sync(kFull, x.ub2, o);
-    y.j1 = __shfl_xor_sync(kFull, x.j1, o);
-    keytop_merge(x, y);
-  }
-  if (T.G == 1) return x;
-  float *rb = (float *)red;          // 3 floats per warp
-  int *rj = (int *)(rb + 3 * T.G);   // 1 int per warp
-  T.sync();
-  if (T.lane == 0) {
-    rb[3 * T.warp] = x.b1;
-    rb[3 * T.warp + 1] = x.e1;
-    rb[3 * T.warp + 2] = x.ub2;
-    rj[T.warp] = x.j1;
-  }
-  T.sync();
-  KeyTop a{rb[0], rb[1], rb[2], rj[0]};
-  for (int w = 1; w < T.G; ++w) keytop_merge(a, KeyTop{rb[3 * w], rb[3 * w + 1], rb[3 * w + 2], rj[w]});
-  return a;
+// Order-preserving integer image of a float32 (no NaN), and back.
+__device__ __forceinline__ int fkey(float x) {
+  const int b = __float_as_int(x);
+  return b ^ ((b >> 31) & 0x7FFFFFFF);
+}
+__device__ __forceinline__ float funkey(int k) { return __int_as_float(k ^ ((k >> 31) & 0x7FFFFFFF)); }
+
+// The warp's KeyTop: two integer warp maxima. Every lane other than the best
+// one's contributes its own best key's upper bound; a second lane with an equal
+// key then has an upper bound above it, which sends the choice to float64.
+__device__ __forceinline__ KeyTop warp_keytop(const KeyTop &x, int lane) {
+  const int mine = fkey(x.b1), m = __reduce_max_sync(kFull, mine);
+  const int src = __ffs(__ballot_sync(kFull, mine == m)) - 1;
+  const float u = lane == src ? x.ub2 : fmaxf(x.ub2, __fadd_rn(x.b1, x.e1));
+  KeyTop t;
+  t.ub2 = funkey(__reduce_max_sync(kFull, fkey(u)));
+  t.b1 = funkey(m);
+  t.e1 = __shfl_sync(kFull, x.e1, src);
+  t.j1 = __shfl_sync(kFull, x.j1, src);
+  return t;
 }
 
 __device__ __forceinline__ bool is_nan64(double x) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
   return ((b >> 52) & 0x7FF) == 0x7FF && (b & 0xFFFFFFFFFFFFFull) != 0;
-}
-
-// The score sums are formed per alter group: the 32-alter blocks b (alter j
-// in block j >> 5, on lane j & 31) fall into nsb groups, block b into group
-// b mod nsb, with nsb fixed by n alone. A team of G warps takes groups g,
-// g+G, ...; each group costs one warp reduction, so networks of up to 16
-// blocks use at most four groups (up to four blocks each; teams of up to four
-// warps share them), and larger ones a multiple of 4 with up to two blocks per
-// group (shared evenly by teams of up to 16 warps). A lane adds its alters of a group in ascending
-// block order into double-float accumulators, one warp reduction per group
-// follows, and the group records are combined in group order: every sum's
-// order depends on n and j only, never on the team size.
-__host__ __device__ __forceinline__ int lse_groups(int nb) {
-  // up to 16 blocks: about four blocks per group, at least two groups (so a
-  // team of two warps shares the pass); beyond: about two blocks per group
-  if (nb <= 16) return nb < 4 ? nb : 4;
-  const int g = 4 * ((nb + 7) / 8);
-  return g < nb ? g : nb;
-}
-
-// Adds one alter's score quantities to the lane's accumulators, held as
-// packed pairs of quantities (quantities 2x and 2x+1 in H[x], L[x]):
-// quantity 0 the weight w = exp(f_j) relative to the "no change" alter
-// (whose predictor is 0), quantity 1+e the product w * d_e (not for the "no
-// change" alter). Every product is a Dekker product of the weight's pair with
-// d_e's pair, added with TwoSum, two quantities per instruction. LOMASK: bit
-// e set when d_e may have a double-float remainder (integer counts have none).
-// first (uniform over the warp): the accumulators are still zero, so the
-// products are stored as they are (what TwoSum onto zero would give, bit for
-// bit).
-template <int V, unsigned LOMASK>
-__device__ __forceinline__ void lse_accumulate(float2 (&H)[(V + 1) / 2], float2 (&L)[(V + 1) / 2],
-                                               float wh, float wl, const float *d32,
-                                               const float *d32lo, bool weighted, int k,
-                                               bool first) {
-  const float2 w2 = make_float2(wh, wh), wl2 = make_float2(wl, wl);
-#pragma unroll
-  for (int x = 0; x < (V + 1) / 2; ++x) {
-    const int qa = 2 * x, qb = 2 * x + 1;
-    // d of quantity q: 1 for the weight itself, d_{q-1} for a product, 0
-    // beyond the model's effects or for the "no change" alter
-    const bool ua = qa == 0 || (weighted && qa - 1 < k), ub = qb < V && weighted && qb - 1 < k;
-    const float da = qa == 0 ? 1.f : (ua ? d32[qa - 1] : 0.f);
-    const float db = ub ? d32[qb - 1] : 0.f;
-    const float2 d2 = make_float2(da, db);
-    const float2 p = __fmul2_rn(w2, d2);
-    float2 pl = __ffma2_rn(wl2, d2, __ffma2_rn(w2, d2, make_float2(-p.x, -p.y)));
-    const bool la = qa > 0 && ((LOMASK >> (qa - 1)) & 1u), lb = (LOMASK >> (qb - 1)) & 1u;
-    if (la || lb) {
-      const float2 dl2 =
-          make_float2(la && ua ? d32lo[qa - 1] : 0.f, lb && ub ? d32lo[qb - 1] : 0.f);
-      pl = __ffma2_rn(w2, dl2, pl);
-    }
-    if (first) {
-      H[x] = p;
-      L[x] = pl;
-    } else {
-      ff_add2(H[x], L[x], p, pl);
-    }
-  }
-}
-
-// The group sums of the warp's lanes reduced by the fixed recursive-halving
-// warp reduction; the lane holding quantity q stores it as the pair
-// rec[2q], rec[2q+1].
-template <int V>
-__device__ __forceinline__ void lse_store(float *rec, float (&h)[V], float (&l)[V], int k,
-                                          int lane) {
-  bool writer;
-  const int q = warp_multi_sum_ff<V>(h, l, lane, &writer);
-  if (writer && q <= k) {
-    rec[2 * q] = h[0];
-    rec[2 * q + 1] = l[0];
-  }
-}
-
-// The group records combined by one warp of the team: lane q adds quantity
-// q's records in group order (double-float). Quantity q lands in
-// S.red[32G + q] as a double, past the warp slots the team reductions use.
-__device__ __forceinline__ void combine_groups(const Team &T, const Slice &S, int nsb, int k) {
-  const int q = T.lane;
-  if (q > k) return;
-  const float *rec = S.blk + 2 * q;
-  const size_t stride = 2 * (size_t)(k + 1);
-  float h = rec[0], l = rec[1];
-  for (int g = 1; g < nsb; ++g) ff_add(h, l, rec[g * stride], rec[g * stride + 1]);
-  S.red[32 * T.G + q] = __dadd_rn((double)h, (double)l);
 }
 
 // The float64 predictor f_j of alter j (and its change statistics in d): the
@@ -400,7 +386,7 @@ template <bool MULTI>
 __device__ __forceinline__ double f64_of(const DevProblem &P, const Slice &S, const StepCtx &X,
                                          int j, double *d, int net) {
   const int n = P.n, i = X.i;
-  const int aij = bit_of(S.rowsT, n, i, j), aji = bit_of(S.colsT, n, i, j);
+  const int aij = bit_of(S.rows, n, i, j), aji = bit_of(S.cols, n, i, j);
   (void)net;
 #if defined(CUSNA_JIT_SPEC)
   return jit_change_stats<true>(P, S, X, j, aij, aji, d);
@@ -417,13 +403,12 @@ __device__ __forceinline__ double f64_of(const DevProblem &P, const Slice &S, co
 // exp(f_j - lmax) and wsum_e = sum of exp(f_j - lmax) d_je over permitted
 // alters, every f_j and d_je the reference's float64 value. The sums run per
 // 32-alter block (fixed warp reduction) and over blocks in order, so they do
-// not depend on the team size; results land in S.red[32G + q]. Used when a
-// predictor leaves the double-float exponential's range or is not finite,
+// not depend on the team size; quantity 0 (the weights) and 1 + e land in
+// S.red[32G + q]. Then score_e += d_{jstar,e} - wsum_e / sume. Used by chains whose parameters exceed the fixed-point range
 // and at every ministep under F_LSE64. Called by the whole team.
 template <bool MULTI, int VQ>
-static __device__ __noinline__ void lse_float64(const Team &T, const DevProblem &P,
-                                                const Slice &S, const StepCtx &X, double *d,
-                                                int net) {
+static __device__ __noinline__ void lse_float64(const Team T, const DevProblem &P, const Slice S,
+                                                const StepCtx X, double *d, int net, int jstar) {
   constexpr int V = VQ <= 8 ? 8 : (VQ <= 16 ? 16 : 32);  // warp_multi_sum's power of two
   const int n = P.n, k = P.k, L = T.L, i = X.i;
   long long mk = dkey(0.0);
@@ -436,7 +421,7 @@ static __device__ __noinline__ void lse_float64(const Team &T, const DevProblem 
     }
   }
   const double lmax = dunkey(team_max_ll(T, mk, S.red));
-  double *rec64 = (double *)S.blk;
+  double *rec64 = S.blk;
   for (int jb = 32 * T.warp; jb < n; jb += L) {
     const int j = jb + T.lane;
     double w = 0.0;
@@ -471,17 +456,185 @@ static __device__ __noinline__ void lse_float64(const Team &T, const DevProblem 
     const bool writer = (V >= 32) || ((T.lane & ((32 / V) - 1)) == 0);
     if (writer && q <= k) S.red[32 * T.G + q] = v[0];
   }
+  // the chosen alter's statistics and the score update
+  if (T.tl == 0) {
+    if (jstar == i)
+      for (int e = 0; e < k; ++e) d[e] = 0.0;
+    else
+      f64_of<MULTI>(P, S, X, jstar, d, net);
+    for (int e = 0; e < k; ++e) S.dstar[e] = d[e];
+  }
+  T.sync();
+  for (int e = T.tl; e < k; e += L)
+    S.sc[e] = __dadd_rn(S.sc[e], __dsub_rn(S.dstar[e], __ddiv_rn(S.red[32 * T.G + 1 + e], S.red[32 * T.G])));
 }
 
-// Compile-time width of the score sums (the k + 1 quantities in a specialised
-// build; the library build rounds k + 1 up to a power of two) and the mask of
-// effects whose change statistic can have a double-float remainder (LOMASK).
-#if defined(CUSNA_JIT_SPEC)
-#define CUSNA_LSE_V (CUSNA_JIT_K + 1)
-#define CUSNA_LSE_LOMASK CUSNA_JIT_LOMASK
-#else
-#define CUSNA_LSE_LOMASK 0xFFFFFFFFu
+// ---- score sums in fixed point ---------------------------------------------------
+// Quantities: 0 the weights w_j (every permitted alter, "no change" included), 1
+// delta_j w_j, 2 + e the weighted magnitude delta_j w_j |d_je| of an effect of
+// class FX_CNT or FX_REAL. Each lane adds its alters in 64-bit integers (scale
+// 2^-(44 - sh); real statistics as mulhi_fx(w 2^6, m)), the warp adds its lanes'
+// accumulators as three integer limbs, and the warps' sums are added as integers:
+// no order matters. kFxRoom bounds a lane's sums (see step_guard).
+// A specialised build fixes the number (CUSNA_FX_V) and the ones in use.
+#ifndef CUSNA_FX_MASK
+#define CUSNA_FX_MASK 0xFFFFFFFFu
 #endif
+
+// Adds alter j's weight W and magnitudes v to the lane's accumulators.
+template <int V>
+__device__ __forceinline__ void sums_add(const Slice &S, int k, int64_t (&acc)[V], uint64_t W,
+                                         int aij, const uint64_t *v) {
+  const int64_t wd = signed_fx(W, aij);
+  const uint64_t w6 = W << 6;
+  acc[0] += (int64_t)W;
+  acc[1] += wd;
+#pragma unroll
+  for (int e = 0; e < V - 2; ++e) {
+    if (e >= k) continue;
+    const int cls = S.ecls[e] & 0xFF;
+    if (cls == FX_CNT) {
+      acc[2 + e] += wd * (int64_t)v[e];
+    } else if (cls == FX_REAL) {
+      acc[2 + e] += signed_fx(mulhi_fx(w6, v[e]), aij);
+    }
+  }
+}
+
+// The warp's sums: afterwards lane q holds quantity q's total as lo + 2^48 hi.
+template <int V>
+__device__ __forceinline__ void sums_reduce(const int64_t (&acc)[V], int lane, int64_t &lo, int &hi) {
+  lo = 0;
+  hi = 0;
+#pragma unroll
+  for (int q = 0; q < V; ++q) {
+    if (!((CUSNA_FX_MASK >> q) & 1u)) continue;
+    const uint64_t a = (uint64_t)acc[q];
+    const unsigned s0 = __reduce_add_sync(kFull, (unsigned)a & 0xFFFFFFu);
+    const unsigned s1 = __reduce_add_sync(kFull, (unsigned)(a >> 24) & 0xFFFFFFu);
+    const int s2 = __reduce_add_sync(kFull, (int)(acc[q] >> 48));
+    if (lane == q) {
+      lo = (int64_t)s0 + ((int64_t)s1 << 24);
+      hi = s2;
+    }
+  }
+}
+
+// The ring: ministep slot's score sums as they left the pass (quantity q as lo +
+// 2^48 hi), the chosen alter's magnitudes (v of change_fixed; a FX_UNI effect's
+// float64 magnitude) and meta = 4 sh + 2 a_ij + ("no change" chosen). Divisions
+// and float64 arithmetic wait for scores_flush: on this chip a dependent FP64
+// operation is tens of cycles and a division hundreds, 2,700 of the 8,800 cycles
+// of a ministep of one warp (n = 50) when every ministep did its own; eight at
+// a time, one per lane group, they cost about a tenth of that.
+struct ScoreRing {
+  int64_t *lo, *dst;
+  int *hi, *meta;
+};
+__device__ __forceinline__ ScoreRing ring_of(const Slice &S, int k) {
+  ScoreRing R;
+  R.lo = reinterpret_cast<int64_t *>(S.blk);
+  R.dst = R.lo + kRing * (k + 2);
+  R.hi = reinterpret_cast<int *>(R.dst + kRing * k);
+  R.meta = R.hi + kRing * (k + 2);
+  return R;
+}
+
+// Adds the warps' sums into the ring (one warp, lane q).
+__device__ __forceinline__ void sums_combine(const Team &T, const Slice &S, const ScoreRing &R,
+                                             int k, int slot) {
+  const int64_t *lo = reinterpret_cast<const int64_t *>(S.red);
+  int64_t a = 0;
+  int h = 0;
+  for (int w = 0; w < T.G; ++w) {
+    a += lo[32 * w + T.lane];
+    h += S.redh[32 * w + T.lane];
+  }
+  if (T.lane < k + 2) {
+    R.lo[slot * (k + 2) + T.lane] = a;
+    R.hi[slot * (k + 2) + T.lane] = h;
+  }
+}
+
+// score_e += d_e - wsum_e / sume over the ring's first cnt ministeps (one warp):
+// lane = 8 (e mod 4) + slot, the slots' terms added in a fixed tree, so the scores
+// do not depend on the team size.
+static __device__ __noinline__ void scores_flush(const ScoreRing R, const int *ecls,
+                                                 const int *ety, const int *esd, double *sc,
+                                                 int k, int lane, int cnt) {
+  const int slot = lane & (kRing - 1);
+  const bool on = slot < cnt;
+  auto dbl = [&](int q) {
+    const int x = slot * (k + 2) + q;
+    return __dadd_rn((double)R.lo[x], __dmul_rn((double)R.hi[x], 281474976710656.0));
+  };
+  const int meta = on ? R.meta[slot] : 0;
+  const int sh = meta >> 2;
+  const double dl = (meta & 1) ? 0.0 : ((meta & 2) ? -1.0 : 1.0);
+  const double w = on ? dbl(0) : 1.0, dw = on ? dbl(1) : 0.0;
+  const double inv = __ddiv_rn(1.0, w);
+  // the "no change" alter's weight (exp_fx(0, sh)), and a factor that the compiler
+  // does not turn into a subtraction (see signed_fx)
+  const int64_t stay = sh <= kWBits ? 1LL << (kWBits - sh) : (sh == kWBits + 1 ? 1 : 0);
+  int64_t minus8;
+  asm volatile("mov.b64 %0, -8;" : "=l"(minus8));
+  auto term = [&](int e) -> double {
+    if (!on || e >= k) return 0.0;
+    const int cls = ecls[e] & 0xFF, ty = ety[e];
+    const int64_t m = R.dst[slot * k + e];
+    if (cls == FX_DELTA) return __dsub_rn(dl, __dmul_rn(dw, inv));
+    if (cls == FX_UNI)   // a_ij = 0: the magnitude itself
+      return __dmul_rn(__longlong_as_double(m), __dsub_rn(dl, __dmul_rn(dw, inv)));
+    if (cls == FX_CNT) return __dsub_rn(__dmul_rn(dl, (double)m), __dmul_rn(dbl(2 + e), inv));
+    if (cls != FX_REAL) return 0.0;
+    // the 2^62 of every magnitude added 16 w delta: over all alters, or over those
+    // that the creation (no tie) or endowment (tie) type leaves, which is half of
+    // w (1 + delta), or of w (delta - 1), without "no change". Taken off in
+    // integers, so that magnitudes of 0 leave 0.
+    const int x = slot * (k + 2);
+    const int64_t cd = ty == 0 ? 2 : 1, cw = ty == 1 ? 1 : (ty == 2 ? -1 : 0),
+                  cs = ty == 1 ? -1 : (ty == 2 ? 1 : 0);
+    int64_t lo = R.lo[x + 2 + e] + (R.lo[x + 1] * cd + R.lo[x] * cw + stay * cs) * minus8;
+    const int64_t hi = R.hi[x + 2 + e] + (R.hi[x + 1] * cd + R.hi[x] * cw) * minus8 + (lo >> 48);
+    lo &= (1LL << 48) - 1;
+    const double back = pow2(-esd[e]);
+    const double mean = __dmul_rn(
+        __dmul_rn(__dadd_rn((double)lo, __dmul_rn((double)hi, 281474976710656.0)), inv),
+        __dmul_rn(pow2(58), back));
+    // (a magnitude of 0 marks one that the type rules out)
+    const double ds = m ? __dmul_rn(__dmul_rn(dl, (double)(m - (1LL << 62))), back) : 0.0;
+    return __dsub_rn(ds, mean);
+  };
+  for (int e0 = 0; e0 < k; e0 += 8) {   // two effects at once: their chains overlap
+    const int e = e0 + (lane >> 3);
+    double c = term(e), c4 = term(e + 4);
+#pragma unroll
+    for (int o = 1; o < kRing; o <<= 1) {
+      c = __dadd_rn(c, __shfl_xor_sync(kFull, c, o));
+      c4 = __dadd_rn(c4, __shfl_xor_sync(kFull, c4, o));
+    }
+    if (slot == 0 && e < k) sc[e] = __dadd_rn(sc[e], c);
+    if (slot == 0 && e + 4 < k) sc[e + 4] = __dadd_rn(sc[e + 4], c4);
+  }
+}
+__device__ __forceinline__ void scores_flush(const Team &T, const Slice &S, int k, int cnt) {
+  // not the first warp, whose lanes toggle the tie meanwhile
+  if (T.warp == T.G - 1) scores_flush(ring_of(S, k), S.ecls, S.ety, S.esd, S.sc, k, T.lane, cnt);
+}
+
+// Largest f (scale 2^-14) for which no lane's sums can leave 63 bits: with nb
+// blocks of 32 alters a lane adds at most nb products w |d| at scale 2^44 (real
+// statistics: w 2^50 at most), so w mb nb <= 2^17 keeps them below 2^61, mb
+// being the largest count that the ministep can meet (at least 16).
+__device__ __forceinline__ int step_guard(const DevProblem &P, const Slice &S, const StepCtx &X) {
+  const int nb = (P.n + 31) >> 5;
+  int mb = max(16, max(2 * X.od_i + 2, X.id_i + 1));
+  mb = max(mb, S.misc[10] + 1);
+  // out-degrees of every network (cross effects count another network's ties)
+  for (int w = 0; w < X.net.D; ++w) mb = max(mb, X.net.misc[w * X.net.misc_stride + 11] + 1);
+  const int lg = 17 - (32 - __clz(mb * nb - 1));   // floor(log2(2^17 / (mb nb)))
+  return lg * 11356;                               // ln2 at 2^-14
+}
 
 // Per-thread scratch of one alter's change statistics in the pass over the
 // alters: the model's k in the specialised build, the capacity otherwise.
@@ -491,248 +644,300 @@ constexpr int kScratchK = CUSNA_JIT_K;
 constexpr int kScratchK = kMaxEff;
 #endif
 
-// The pass over the alters of one network ministep (see net_choice): per
-// alter the change statistics, the float32 Gumbel key with its error bound
-// (into *best and S.gbuf), the permitted-alter bits (S.okbits) and, when the
-// double-float score sums are wanted (fast_sums), the alter's score
-// quantities into its lane's group accumulators; each group's sums end in its
-// record in S.blk. Returns true on lanes that saw a predictor outside the
-// double-float exponential's range.
+// The pass over the alters of one network ministep (see net_choice): per alter
+// the magnitudes and the predictor, the float32 Gumbel key with its error bound
+// (into *best and S.gbuf), the permitted-alter bits (S.okbits) and, with sums,
+// the weight exp(f_j) 2^-sh and its products, whose warp sums end in S.red and
+// S.redh. Returns the lane's largest predictor (scale 2^-14). Block b of 32
+// alters belongs to warp b mod G.
 template <bool MULTI, bool VALID, int V>
-__device__ __forceinline__ bool alter_pass(const Team &T, const DevProblem &P, const Slice &S,
-                                           const StepCtx &X, long long ms, uint32_t chain,
-                                           KeyTop &best, bool fast_sums, int net) {
-  const int n = P.n, k = P.k, i = X.i;
+__device__ __forceinline__ int alter_pass(const Team &T, const DevProblem &P, const Slice &S,
+                                          const StepCtx &X, long long ms, uint32_t chain,
+                                          KeyTop &best, bool sums, int sh, int net) {
+  const int n = prob_n(P), k = prob_k(P), i = X.i;
   (void)net;
-  const float ecoef = (float)(k + 10) * 5.9604644775390625e-8f;
-  const int nb = (n + 31) >> 5, nsb = lse_groups(nb);
+  const int nb = (n + 31) >> 5;
 #ifdef CUSNA_JIT_K
   constexpr int KS = CUSNA_JIT_K;
 #else
   const int KS = k;
 #endif
-  bool wide = false;
-  // without score sums the blocks are simply dealt to the warps in turn
-  const int ng = fast_sums ? nsb : nb;
-  for (int g = T.warp; g < ng; g += T.G) {
-    float2 AH[(V + 1) / 2], AL[(V + 1) / 2];
+  int64_t acc[V];
 #pragma unroll
-    for (int x = 0; x < (V + 1) / 2; ++x) {
-      AH[x] = make_float2(0.f, 0.f);
-      AL[x] = make_float2(0.f, 0.f);
-    }
-    for (int b = g; b < nb; b += ng) {
-      const int j = (b << 5) + T.lane;
-      // the alter's float32 change statistics and their double-float
-      // remainders: in the specialised build every index is a constant, so
-      // these stay in registers
-      float d32[kScratchK], d32lo[kScratchK];
-      bool ok = false, stay = false;
-      float f = 0.f;
-      float2 fx = make_float2(0.f, 0.f);
-      if (j < n) {
-        const int aij = bit_of(S.rowsT, n, i, j);
-        float ub = -INFINITY;
-        stay = j == i;
-        ok = stay || (bit_of(P.permT, n, i, j) && !(P.maxdeg > 0 && aij == 0 && X.od_i >= P.maxdeg));
-        if (ok) {
-          float absf = 0.f;
+  for (int q = 0; q < V; ++q) acc[q] = 0;
+  int fmax = 0;
+  const bool full = P.maxdeg > 0 && X.od_i >= P.maxdeg;   // no new tie
+  const uint32_t *permr = P.permr;
+  const uint32_t k0 = P.k0, k1 = P.k1;
+#pragma unroll 1
+  for (int b = T.warp; b < nb; b += T.G) {
+    const int jl = (b << 5) + T.lane, j = jl < n ? jl : n - 1;
+    const int aij = bit_of(S.rows, n, i, j), aji = bit_of(S.cols, n, i, j);
+    const bool stay = j == i;
+    const bool ok = jl < n && (stay || (bit_of(permr, n, i, j) && !(full && aij == 0)));
+    const float gum = gumbel_est(alter_word<VALID>(P, S, ms, chain, j, k0, k1));
+    uint64_t v[kScratchK];
 #if defined(CUSNA_JIT_SPEC)
-          // the effect plan compiled in (saom_jit.cu): the same float32 values
-          if (!stay)
-            f = jit_change_stats32(P, S, X, j, aij, bit_of(S.colsT, n, i, j), d32, d32lo, &absf,
-                                   &fx);
+    int64_t f = jit_change_fixed(P, S, X, j, aij, aji, v);
 #elif defined(CUSNA_JIT_MULTI)
-          if (!stay)
-            f = jit_change_stats32(net, P, S, X, j, aij, bit_of(S.colsT, n, i, j), d32, d32lo,
-                                   &absf, &fx);
+    int64_t f = jit_change_fixed(net, P, S, X, j, aij, aji, v);
 #else
-          if (!stay)
-            f = change_stats32<MULTI>(P, S, X, j, aij, bit_of(S.colsT, n, i, j), d32, d32lo,
-                                      &absf, &fx);
+    int64_t f = change_fixed<MULTI>(P, S, X, j, aij, aji, v);
 #endif
-          const float gk = __fsub_rn(f, loglog_est(alter_word<VALID>(P, S, ms, chain, j)));
-          const float E = __fadd_rn(__fmul_rn(ecoef, absf), 6e-6f);
-          ub = __fadd_rn(gk, E);
-          keytop_add(best, gk, E, j);
-        }
-        S.gbuf[j] = ub;
-      }
-      const uint32_t okb = __ballot_sync(kFull, ok);
-      if (T.lane == 0) S.okbits[b] = okb;
-      // the group's first block initialises every lane's accumulators (a lane
-      // without a permitted alter there stores zeros); later blocks add the
-      // permitted alters
-      const bool first = b == g;
-      if (fast_sums && (ok || first)) {
-        float wh = ok ? 1.f : 0.f, wl = 0.f;  // the "no change" alter: exp(0)
-        if (ok && !stay) {
-          if (fabsf(f) <= kFFExpMax) {
-            exp_ff(fx.x, fx.y, S.etab, wh, wl);
-          } else {  // also NaN
-            wide = true;
-            wh = 0.f;
-          }
-        }
-        lse_accumulate<V, CUSNA_LSE_LOMASK>(AH, AL, wh, wl, d32, d32lo, ok && !stay, KS, first);
-      }
+    f = stay ? 0 : signed_fx((uint64_t)f, aij);
+    const int fh = (int)(f >> 32);
+    // float32 rounding of f 2^-46
+    const float f32 = fmaf((float)fh, 6.103515625e-5f, __fmul_rn((float)(uint32_t)f, 1.4210854715202004e-14f));
+    const float gk = __fsub_rn(f32, gum);
+    const float E = fmaf(fabsf(f32), 3.6e-7f, 3e-5f);
+    if (ok) {
+      fmax = max(fmax, fh);
+      keytop_add(best, gk, E, j);
     }
-    if (fast_sums) {
-      float ah[V], al[V];
-#pragma unroll
-      for (int q = 0; q < V; ++q) {
-        ah[q] = (q & 1) ? AH[q >> 1].y : AH[q >> 1].x;
-        al[q] = (q & 1) ? AL[q >> 1].y : AL[q >> 1].x;
+    if (jl < n) S.gbuf[j] = ok ? __fadd_rn(gk, E) : -INFINITY;
+    const uint32_t okb = __ballot_sync(kFull, ok);
+    if (T.lane == 0) S.okbits[b] = okb;
+    if (sums) {
+      uint64_t W = exp_fx(f, sh, S.etab);
+      if (!ok) W = 0;
+      if (stay) {
+        acc[0] += (int64_t)W;
+      } else {
+#if defined(CUSNA_JIT_SPEC)
+        jit_sums_add(acc, W, aij, v);
+#elif defined(CUSNA_JIT_MULTI)
+        jit_sums_add(net, acc, W, aij, v);
+#else
+        sums_add<V>(S, KS, acc, W, aij, v);
+#endif
       }
-      lse_store<V>(S.blk + (size_t)g * 2 * (k + 1), ah, al, KS, T.lane);
     }
   }
-  return wide;
+  if (sums) {
+    int64_t lo;
+    int hi;
+    sums_reduce<V>(acc, T.lane, lo, hi);
+    reinterpret_cast<int64_t *>(S.red)[32 * T.warp + T.lane] = lo;
+    S.redh[32 * T.warp + T.lane] = hi;
+  }
+  return fmax;
+}
+
+// Every permitted alter a candidate for the float64 keys: a ministep of a chain
+// outside the fixed-point range. (The functions of the rare paths take the slice
+// by value: a reference would keep it in memory, and the hot path's shared-memory
+// pointers with it.)
+static __device__ __noinline__ void mark_all(const Team T, const DevProblem &P, const Slice S,
+                                             const StepCtx X) {
+  const int n = P.n, i = X.i;
+  const bool full = P.maxdeg > 0 && X.od_i >= P.maxdeg;
+  for (int b = T.warp; b < ((n + 31) >> 5); b += T.G) {
+    const int j = (b << 5) + T.lane;
+    const bool ok = j < n && (j == i || (bit_of(P.permr, n, i, j) &&
+                                         !(full && bit_of(S.rows, n, i, j) == 0)));
+    if (j < n) S.gbuf[j] = ok ? INFINITY : -INFINITY;
+    const uint32_t okb = __ballot_sync(kFull, ok);
+    if (T.lane == 0) S.okbits[b] = okb;
+  }
+  T.sync();
+}
+
+// The choice by exact float64 keys among the permitted alters whose upper bound
+// is not below lb (the reference's f_j - log(-log u_j), ties to the smaller j).
+template <bool MULTI, bool VALID>
+static __device__ __noinline__ int choice_float64(const Team T, const DevProblem &P, const Slice S,
+                                                  const StepCtx X, long long ms, uint32_t chain,
+                                                  float lb, double *d, int net) {
+  const int n = P.n, i = X.i;
+  long long bk = dkey(-1e300);
+  int bj = 0x7FFFFFFF;
+  for (int j = T.tl; j < n; j += T.L) {
+    const bool okj = (S.okbits[j >> 5] >> (j & 31)) & 1u;
+    if (okj && !(S.gbuf[j] < lb)) {
+      const double f = j != i ? f64_of<MULTI>(P, S, X, j, d, net) : 0.0;
+      const double g = __dsub_rn(f, log(-log(unif01(alter_word<VALID>(P, S, ms, chain, j, P.k0, P.k1)))));
+      if (is_nan64(g)) continue;
+      const long long kg = dkey(g);
+      if (kg > bk || (kg == bk && j < bj)) { bk = kg; bj = j; }
+    }
+  }
+  return team_argmax(T, bk, bj, S.red + 32 * T.G + 32);
+}
+
+// The chain's scores go through the ring.
+__device__ __forceinline__ bool ring_scores(const DevProblem &P, const Slice &S) {
+  return (P.flags & (F_NO_SCORES | F_LSE64)) == 0 && S.fx[1] != 0;
+}
+// After ministep slot's choice and a team barrier: a full ring into the scores.
+__device__ __forceinline__ void score_slot(const Team &T, const DevProblem &P, const Slice &S,
+                                           int slot) {
+  if (slot == kRing - 1 && ring_scores(P, S)) scores_flush(T, S, prob_k(P), kRing);
 }
 
 // One network ministep of focal actor i on the network of slice S, up to the
-// choice: change statistics, float32 keys and the double-float score sums, the
-// certified or exact float64 choice, and the chosen alter's float64 change
-// statistics in S.dstar. Returns j*. The score sums are left in S.red[32G + q]
-// (float64) for the score update. d (float64) is per-thread scratch of k
-// values.
-// MULTI: the network is one of a multi-network problem's, whose network w has
-// its rows at rows0 + w*net_stride words (cross effects read them).
+// choice: the pass over the alters and the certified or exact float64 choice.
+// Returns j*. The score sums and the chosen alter's magnitudes go to slot of the
+// ring, which the caller flushes after a team barrier (score_slot). d (float64)
+// is per-thread scratch of k values.
+// MULTI: the network is one of a multi-network problem's. nb0 locates the state
+// of every network (of the one network).
 // VALID: validation mode (caller-supplied words in place of Philox).
 template <bool MULTI, bool VALID = false>
 __device__ __forceinline__ int net_choice(const Team &T, const DevProblem &P, const Slice &S,
                                           int i, long long ms, uint32_t chain, double *d,
-                                          const uint32_t *rows0 = nullptr,
-                                          size_t net_stride = 0, int net = 0) {
-  const int n = P.n, W = P.W, k = P.k, L = T.L;
+                                          const NetBase *nb0, int slot, int net = 0) {
+  const int n = prob_n(P), W = prob_w(P), k = prob_k(P), L = T.L, fl = P.flags;
   (void)net;
-  step_helpers(T, P, S, i);
   StepCtx X;
   X.i = i;
   X.od_i = S.outdeg[i];
   X.id_i = S.indeg[i];
   X.rdeg_i = 0;
-  if (P.flags & F_NEED_RDEG)
-    for (int w = 0; w < W; ++w) X.rdeg_i += __popc(S.rowsT[w * n + i] & S.colsT[w * n + i]);
-  X.zvi = (P.flags & F_HAS_Z) ? __dsub_rn((double)S.z[i], P.zbar) : 0.0;
-  X.rows0 = rows0;
-  X.net_stride = net_stride;
-  if (P.flags & F_HAS_STEP) {
+  if (fl & F_NEED_RDEG)
+    for (int w = 0; w < W; ++w) X.rdeg_i += __popc(S.rows[w * n + i] & S.cols[w * n + i]);
+  X.zvi = (fl & F_HAS_Z) ? __dsub_rn((double)S.z[i], P.zbar) : 0.0;
+  X.net = *nb0;
+  X.tabq = P.tabq;
+  step_helpers(T, P, S, X);
+  X.f0 = S.fx[0];
+  const bool ranged = S.fx[1] != 0;
+  if (fl & F_HAS_STEP) {
     step_values(T, P, S, X);
     T.sync();
+    if (ranged)
+      for (int e = 0; e < k; ++e)
+        if ((S.ecls[e] & 0xFF) == FX_UNI)
+          X.f0 += term_fx(S.thq[e], S.ecls[e], S.stepq[4 * e]);
   }
 
   // ---- one pass over the alters (alter_pass) -------------------------------
-  // Lane by lane: integer change statistics, the
-  // float32 predictor f32_j (change_stats32) and the float32 Gumbel key
-  // g_j = f32_j - loglog_est(u_j) with u_j from the reference's counters
-  // (msteps, chain, 1, j). The key is within
-  //   E_j = (k + 10) 2^-24 absf_j + 6e-6
-  // of the float64 key f_j - log(-log u_j): (k + 8) u absf_j for f32_j, 4e-6
-  // for loglog_est and u (absf_j + 23) for the subtraction (|f32_j| <= absf_j,
-  // |log(-log u)| < 23). gbuf[j] keeps the upper bound g_j + E_j.
-  // The score sums are formed per group of alters (lse_groups; the grouping
-  // and every order of addition depend on n and j only) in double-float
-  // arithmetic: the predictor as a double-float pair (within ~2^-47 absf_j of
-  // the reference's float64 f_j), its exponential relative to the "no change"
-  // alter (exp_ff, relative error ~2e-14), and the weighted change
-  // statistics; the groups are combined after the choice in group order
-  // (combine_groups), so the scores do not depend on the launch shape. A
-  // predictor outside [-60, 60] (or not finite) sends the ministep's sums to
-  // the float64 path (lse_float64), as does F_LSE64. Without requested scores
-  // (F_NO_SCORES) no sums are formed.
-  KeyTop best{-INFINITY, 0.f, -INFINITY, 0x7FFFFFFF};
-  const bool want_sums = (P.flags & F_NO_SCORES) == 0;
-  const bool fast_sums = want_sums && (P.flags & F_LSE64) == 0;
-#ifdef CUSNA_LSE_V
-  const bool wide = alter_pass<MULTI, VALID, CUSNA_LSE_V>(T, P, S, X, ms, chain, best,
-                                                          fast_sums, net);
+  // The key's error: f32 is within 2 2^-24 |f32| of the fixed-point predictor,
+  // itself within 3k 2^-46 + 2^-50 (the tables) of the float64 f_j; gumbel_est
+  // is within kGumbelErr; the subtraction rounds by 2^-24 (|f32| + 23). All of
+  // it is below E_j = 3.6e-7 |f32| + 3e-5 (kGumbelErr + 1.4e-6 + the rest, twice).
+  // gbuf[j] keeps the upper bound g_j + E_j. When a predictor exceeds the room
+  // that the sums have (step_guard), the pass is repeated with every weight
+  // scaled by 2^-sh, sh from the largest predictor (so from the alters alone).
+  // Without requested scores (F_NO_SCORES) no sums are formed.
+  const bool want_sums = (fl & F_NO_SCORES) == 0;
+  const bool fast_sums = want_sums && (fl & F_LSE64) == 0 && ranged;
+  KeyTop top{-INFINITY, 0.f, INFINITY, 0x7FFFFFFF};
+  float lb = -INFINITY;
+  int sh = 0;
+  if (ranged) {
+    const int room = fast_sums ? step_guard(P, S, X) : 0x7FFFFFFF;
+    for (;;) {
+      KeyTop best{-INFINITY, 0.f, -INFINITY, 0x7FFFFFFF};
+      int fm;
+#ifdef CUSNA_FX_V
+      fm = alter_pass<MULTI, VALID, CUSNA_FX_V>(T, P, S, X, ms, chain, best, fast_sums, sh, net);
 #else
-  bool wide;
-  if (k + 1 <= 8)
-    wide = alter_pass<MULTI, VALID, 8>(T, P, S, X, ms, chain, best, fast_sums, net);
-  else if (k + 1 <= 16)
-    wide = alter_pass<MULTI, VALID, 16>(T, P, S, X, ms, chain, best, fast_sums, net);
-  else
-    wide = alter_pass<MULTI, VALID, 32>(T, P, S, X, ms, chain, best, fast_sums, net);
+      if (k + 2 <= 8)
+        fm = alter_pass<MULTI, VALID, 8>(T, P, S, X, ms, chain, best, fast_sums, sh, net);
+      else if (k + 2 <= 16)
+        fm = alter_pass<MULTI, VALID, 16>(T, P, S, X, ms, chain, best, fast_sums, sh, net);
+      else
+        fm = alter_pass<MULTI, VALID, 26>(T, P, S, X, ms, chain, best, fast_sums, sh, net);
 #endif
-  if (__any_sync(kFull, wide) && T.lane == 0) S.misc[12] = (int)ms;
-  T.sync();
-  const KeyTop top = team_keytop(T, best, S.red + 26 * T.G);
+      top = warp_keytop(best, T.lane);
+      fm = __reduce_max_sync(kFull, fm);
+      if (T.G > 1) {
+        float *rb = reinterpret_cast<float *>(S.red + 32 * T.G + 32);   // 4 words per warp
+        int *ri = reinterpret_cast<int *>(rb);
+        if (T.lane == 0) {
+          rb[4 * T.warp] = top.b1;
+          rb[4 * T.warp + 1] = top.e1;
+          rb[4 * T.warp + 2] = top.ub2;
+          ri[4 * T.warp + 3] = top.j1;
+          S.rfm[T.warp] = fm;
+        }
+        T.sync();
+        top = KeyTop{rb[0], rb[1], rb[2], ri[3]};
+        fm = S.rfm[0];
+        for (int w = 1; w < T.G; ++w) {
+          keytop_merge(top, KeyTop{rb[4 * w], rb[4 * w + 1], rb[4 * w + 2], ri[4 * w + 3]});
+          fm = max(fm, S.rfm[w]);
+        }
+      } else {
+        __syncwarp();
+      }
+      if (fm <= room) break;
+      // the smallest scaling for which the largest predictor fits (ln2 at 2^-14)
+      const int need = (fm - room + 11355) / 11356;
+      if (need <= sh) break;
+      sh = need;
+      T.sync();   // every warp has read the first pass's scratch
+    }
+    lb = __fsub_rn(top.b1, top.e1);
+  } else {
+    mark_all(T, P, S, X);
+  }
 
   // ---- the chosen alter ---------------------------------------------------
   // The float32 keys decide when the best key's lower bound exceeds every
-  // other alter's upper bound. Otherwise every permitted alter whose upper
-  // bound is not below that lower bound (a NaN on either side counts as
-  // reaching it) gets its exact float64 key (the reference's
-  // f_j - log(-log u_j)) and those decide, ties to the smaller j. The "no
-  // change" alter always has a finite key, so a choice always exists.
-  int jstar;
-  const float lb = __fsub_rn(top.b1, top.e1);
-  if (lb > top.ub2) {
-    jstar = top.j1;
-  } else {
-    long long bk = dkey(-1e300);
-    int bj = 0x7FFFFFFF;
-    for (int j = T.tl; j < n; j += L) {
-      const bool okj = (S.okbits[j >> 5] >> (j & 31)) & 1u;
-      if (okj && !(S.gbuf[j] < lb)) {
-        const double f = j != i ? f64_of<MULTI>(P, S, X, j, d, net) : 0.0;
-        const double g = __dsub_rn(f, log(-log(unif01(alter_word<VALID>(P, S, ms, chain, j)))));
-        if (is_nan64(g)) continue;
-        const long long kg = dkey(g);
-        if (kg > bk || (kg == bk && j < bj)) { bk = kg; bj = j; }
-      }
-    }
-    jstar = team_argmax(T, bk, bj, S.red + 29 * T.G);
-  }
+  // other alter's upper bound; otherwise the exact float64 keys of the permitted
+  // alters that reach it decide. The "no change" alter always has a finite key,
+  // so a choice always exists.
+  int jstar = lb > top.ub2 ? top.j1
+                           : choice_float64<MULTI, VALID>(T, P, S, X, ms, chain, lb, d, net);
   // never an index outside the network, whatever the inputs
   if ((unsigned)jstar >= (unsigned)n) jstar = i;
 
-  // the score sums: normally the block records combined into quantity q (0:
-  // sum of weights, 1+e: weighted sum of d_e), by a warp other than the
-  // chosen alter's owner, which meanwhile forms the chosen alter's float64
-  // statistics; on the float64 path, the whole team
-  const bool sums64 = want_sums && (!fast_sums || S.misc[12] == (int)ms);
-  if (sums64) {
-#ifdef CUSNA_LSE_V
-    lse_float64<MULTI, CUSNA_LSE_V>(T, P, S, X, d, net);
+  // the score sums into the ring by a warp other than the chosen alter's owner,
+  // which meanwhile forms the chosen alter's magnitudes; on the float64 path, the
+  // scores by the whole team
+  if (want_sums && !fast_sums) {
+#ifdef CUSNA_JIT_K
+    lse_float64<MULTI, CUSNA_JIT_K + 1>(T, P, S, X, d, net, jstar);
 #else
-    if (k + 1 <= 8) lse_float64<MULTI, 8>(T, P, S, X, d, net);
-    else if (k + 1 <= 16) lse_float64<MULTI, 16>(T, P, S, X, d, net);
-    else lse_float64<MULTI, 32>(T, P, S, X, d, net);
+    if (k + 1 <= 8) lse_float64<MULTI, 8>(T, P, S, X, d, net, jstar);
+    else if (k + 1 <= 16) lse_float64<MULTI, 16>(T, P, S, X, d, net, jstar);
+    else lse_float64<MULTI, 32>(T, P, S, X, d, net, jstar);
 #endif
   } else if (fast_sums) {
-    const int owner_warp = (jstar % L) >> 5;
-    if (T.warp == (T.G > 1 ? (owner_warp + 1) % T.G : 0)) {
-      const int nsb = lse_groups((n + 31) >> 5);
-#ifdef CUSNA_JIT_K
-      combine_groups(T, S, nsb, CUSNA_JIT_K);
-#else
-      combine_groups(T, S, nsb, k);
-#endif
-    }
-  }
-
-  // ---- the chosen alter's change statistics, in float64 as the reference
-  // adds them (for the score update only)
-  if (want_sums && T.tl == jstar % L) {
-    if (jstar == i) {
-      for (int e = 0; e < k; ++e) S.dstar[e] = 0.0;
-    } else {
-      const int aij = bit_of(S.rowsT, n, i, jstar);
-      const int aji = bit_of(S.colsT, n, i, jstar);
+    const ScoreRing R = ring_of(S, k);
+    const int owner = jstar & (L - 1);   // L and G are powers of two
+    if (T.warp == (((owner >> 5) + 1) & (T.G - 1))) sums_combine(T, S, R, k, slot);
+    if (T.tl == owner) {
+      const int aij = bit_of(S.rows, n, i, jstar), aji = bit_of(S.cols, n, i, jstar);
+      uint64_t *v = reinterpret_cast<uint64_t *>(R.dst) + slot * k;
+      R.meta[slot] = 4 * sh + 2 * aij + (jstar == i ? 1 : 0);
+      if (jstar == i) {
+        for (int e = 0; e < k; ++e) v[e] = 0;
+      } else {
 #if defined(CUSNA_JIT_SPEC)
-      jit_change_stats<false>(P, S, X, jstar, aij, aji, d);
+        jit_change_fixed(P, S, X, jstar, aij, aji, v);
 #elif defined(CUSNA_JIT_MULTI)
-      jit_change_stats<false>(net, P, S, X, jstar, aij, aji, d);
+        jit_change_fixed(net, P, S, X, jstar, aij, aji, v);
 #else
-      change_stats<false, MULTI>(P, S, X, jstar, aij, aji, d);
+        change_fixed<MULTI>(P, S, X, jstar, aij, aji, v);
 #endif
-      for (int e = 0; e < k; ++e) S.dstar[e] = d[e];
+      }
+      if (fl & F_HAS_STEP)
+        for (int e = 0; e < k; ++e)
+          if ((S.ecls[e] & 0xFF) == FX_UNI) v[e] = (uint64_t)__double_as_longlong(S.stepd[4 * e]);
     }
   }
   return jstar;
+}
+
+// Toggles the tie i -> j (dl = +-1; and j -> i, symmetric): the bits by lanes 0
+// and 1, the degrees and their largest values by lanes 2 and 3 (4..7: the other
+// direction), each access of all of them at once. The two directions write
+// different words, except the largest degrees.
+__device__ __forceinline__ void toggle_tie(const Team &T, const Slice &S, int n, int i, int j,
+                                           int dl, int symflag) {
+  if (T.tl >= (symflag ? 8 : 4)) return;
+  const int u = T.tl & 4 ? j : i, v = T.tl & 4 ? i : j;
+  if ((T.tl & 2) == 0) {
+    uint32_t *w = T.tl & 1 ? S.cols + (u >> 5) * n + v : S.rows + (v >> 5) * n + u;
+    *w ^= 1u << ((T.tl & 1 ? u : v) & 31);
+  } else {
+    short *d = T.tl & 1 ? S.outdeg + u : S.indeg + v;
+    const int x = *d + dl;
+    *d = (short)x;
+    atomicMax(S.misc + 10 + (T.tl & 1), x);
+  }
 }
 
 // Validation trace record of ministep ms (validation mode only): (step,
@@ -752,7 +957,7 @@ __device__ __forceinline__ void trace_put(const DevProblem &P, int c, long long 
 // One chain: the ministep loop and the chain's outputs.
 template <bool VALID>
 static __device__ void run_chain(const Team &T, const DevProblem &P, const Slice &S, int c) {
-  const int n = P.n, k = P.k;
+  const int n = prob_n(P), k = prob_k(P);
   const uint32_t chain = P.chain_offset + (uint32_t)c;
   chain_init(T, P, S, c);
 
@@ -762,8 +967,10 @@ static __device__ void run_chain(const Team &T, const DevProblem &P, const Slice
   const double den = __dmul_rn((double)P.nact, __dadd_rn(lam, lamb));
   const double pnet = __ddiv_rn(lam, __dadd_rn(lam, lamb));
   long long dist = 0, bdist = 0, ms = 0, msb = 0;
-  double t = 0.0, rho = 0.0;
+  double t = 0.0, rho = 0.0, tnext = 0.0;
+  bool over = false;   // tnext ends an unconditional period
   double d[kMaxEff];
+  const NetBase nb{S.rows, S.cols, S.cm, 0, 0, 0, S.misc, 0, 1};
 
   for (;;) {
     int i;
@@ -793,9 +1000,16 @@ static __device__ void run_chain(const Team &T, const DevProblem &P, const Slice
           S.rr3[T.lane] = rr[3];
         }
         T.sync();
+        tnext = __dadd_rn(t, S.rtau[0]);
+        over = !P.cond && tnext > 1.0;
       }
-      t = __dadd_rn(t, S.rtau[slot]);
-      if (!P.cond && t > 1.0) break;
+      // the time after the following ministep is formed while this one runs
+      t = tnext;
+      if (over) break;
+      if (slot < 31) {
+        tnext = __dadd_rn(t, S.rtau[slot + 1]);
+        over = !P.cond && tnext > 1.0;
+      }
       is_net = S.rnet[slot] != 0;
       i = S.rfocal[slot];
       r3 = S.rr3[slot];
@@ -815,34 +1029,23 @@ static __device__ void run_chain(const Team &T, const DevProblem &P, const Slice
       continue;
     }
 
-    const int jstar = net_choice<false, VALID>(T, P, S, i, ms, chain, d);
-    const int aij_star = bit_of(S.rowsT, n, i, jstar);
+    const int rslot = (int)(ms - msb) & (kRing - 1);
+    const int jstar = net_choice<false, VALID>(T, P, S, i, ms, chain, d, &nb, rslot);
+    const int aij_star = bit_of(S.rows, n, i, jstar);
     T.sync();
-    if (!(P.flags & F_NO_SCORES) && T.tl < k) {
-      const int e = T.tl;
-      const double s0 = S.red[32 * T.G], se = S.red[32 * T.G + 1 + e];
-      S.sc[e] = __dadd_rn(S.sc[e], __dsub_rn(S.dstar[e], __ddiv_rn(se, s0)));
-    }
+    score_slot(T, P, S, rslot);
     const long long dist0 = dist;
     ++ms;
     if (jstar != i) {
       const int j = jstar;
       const long long chg = P.symflag ? 2 : 1;
-      if (bit_of(P.kdistT, n, i, j))
-        dist += (aij_star == bit_of(P.x0T, n, i, j)) ? chg : -chg;
-      if (T.tl == 0) {
-        const int dl = 1 - 2 * aij_star;
-        S.rowsT[(j >> 5) * n + i] ^= 1u << (j & 31);
-        S.colsT[(i >> 5) * n + j] ^= 1u << (i & 31);
-        S.indeg[j] += dl;
-        S.outdeg[i] += dl;
-        if (P.symflag) {
-          S.rowsT[(i >> 5) * n + j] ^= 1u << (i & 31);
-          S.colsT[(j >> 5) * n + i] ^= 1u << (j & 31);
-          S.indeg[i] += dl;
-          S.outdeg[j] += dl;
-        }
-      }
+      // (the distance's words are used after the toggle, off its path)
+      const uint32_t kd = P.kdistr[(j >> 5) * n + i], x0 = P.x0r[(j >> 5) * n + i];
+      if (P.cnt.mask)
+        counts_toggle(T, P, nb, i, j, 1 - 2 * aij_star);
+      toggle_tie(T, S, n, i, j, 1 - 2 * aij_star, P.symflag);
+      if ((kd >> (j & 31)) & 1u)
+        dist += (uint32_t)aij_star == ((x0 >> (j & 31)) & 1u) ? chg : -chg;
     }
     if (T.tl == 0) trace_put<VALID>(P, c, ms - 1, i, jstar, dist - dist0);
     if (P.nrate > 0 && T.tl == 0) {
@@ -858,6 +1061,9 @@ static __device__ void run_chain(const Team &T, const DevProblem &P, const Slice
     if (ms >= kMaxSteps) break;
   }
 
+  T.sync();
+  if (((ms - msb) & (kRing - 1)) && ring_scores(P, S))
+    scores_flush(T, S, k, (int)(ms - msb) & (kRing - 1));
   chain_finish(T, P, S, c, dist, bdist, ms, msb, t, rho, lam, lamb);
 }
 

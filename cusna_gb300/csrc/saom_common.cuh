@@ -12,6 +12,7 @@ typedef unsigned short uint16_t;
 typedef unsigned long long uintptr_t;
 #define INFINITY __int_as_float(0x7f800000)
 #else
+#include <cmath>
 #include <cstdint>
 #include <cuda_runtime.h>
 #endif
@@ -25,19 +26,12 @@ constexpr unsigned kFull = 0xFFFFFFFFu;
 
 // Problem flags (DevProblem::flags).
 enum : int {
-  F_NEED_TP = 1 << 0,      // transTies: two-path counts tp[h] = |out_i & in_h|
+  F_NEED_TP = 1 << 0,      // transTies: masks of the h with 0 / 1 two-paths i -> h
   F_NEED_RDEG = 1 << 1,    // reciAct: reciprocated degree of i
   F_NEED_GW29 = 1 << 2,    // gwdspFF: per-h weight differences over tp
   F_NEED_GW30 = 1 << 3,    // gwdspFB: per-h weight differences over |out_i & out_h|
   F_WANT_ENDS = 1 << 4,    // dense end networks requested
   F_HAS_INTER = 1 << 5,    // interaction effects present
-  F_PC_RI_CJ = 1 << 6,     // popcount needs of the change statistics
-  F_PC_RI_RJ = 1 << 7,
-  F_PC_RJ_CI = 1 << 8,
-  F_PC_CI_CJ = 1 << 9,
-  F_PC_CI_RJ = 1 << 10,
-  F_PC_RICIRJ = 1 << 11,
-  F_COLS_GLOBAL = 1 << 12, // the chain's in-rows live in global scratch
   F_THETA_TAB = 1 << 13,   // term tables hold theta_e * d for every chain
   F_HAS_STEP = 1 << 14,    // some effect is constant within a ministep
   F_HAS_Z = 1 << 15,       // behaviour values are read (behaviour or dynamic covariates)
@@ -75,6 +69,48 @@ struct MultiDev {
   uint8_t *a_ends;
 };
 
+// Two-path counters. The change statistics of a ministep need, for every alter
+// j, the number of h in some set of actors that depends on the focal actor i
+// alone (its out- or in-neighbours, ...) with a tie between h and j. Counter c
+// is one such set and one relation of h and j (with m2, the sum over two).
+//   set:      CL_OUT out_i, CL_IN in_i, CL_MUTUAL out_i & in_i, CL_TP0 / CL_TP1
+//             the h of out_i with 0 / 1 two-paths i -> h (by counter tp),
+//             CL_NET + w out_i in network w
+//   relation: CM_ROWS a tie h -> j, CM_COLS a tie j -> h, CM_NCOLS + w a tie
+//             j -> h in network w
+// Those of CL_OUT, CL_IN and CL_NET are matrix products of the networks; a chain
+// may hold them (mask) as n x n matrices of counts that every toggle updates
+// (saom_kernel.cuh, counts_toggle), so that the pass over the alters reads row i.
+enum : int { CL_OUT = 0, CL_IN = 1, CL_MUTUAL = 2, CL_TP0 = 3, CL_TP1 = 4, CL_NET = 5 };
+enum : int { CM_ROWS = 0, CM_COLS = 1, CM_NCOLS = 2, CM_NONE = 255 };
+constexpr int kMaxCnt = 16, kMaxTask = 32;
+// One update of a count matrix when the network's tie u -> v toggles: every
+// member x of a set of u's or v's neighbours (in network set_net, its out- or
+// in-neighbours) changes the cell (fix, x), or by column (x, fix), fix being u or
+// v, of matrix `rank` of network `net`.
+constexpr unsigned task_pack(bool set_in, bool set_of_v, bool fix_v, bool by_col, int rank,
+                             int set_net, int net) {
+  return (unsigned)set_in | (unsigned)set_of_v << 1 | (unsigned)fix_v << 2 |
+         (unsigned)by_col << 3 | (unsigned)rank << 4 | (unsigned)set_net << 8 | (unsigned)net << 12;
+}
+struct CounterSet {
+  int n;
+  int tp, tq;     // the counter of |out_i & in_h| and |out_i & out_h|, where read by h
+  unsigned mask;  // counters held as matrices
+  unsigned char list[kMaxCnt], m1[kMaxCnt], m2[kMaxCnt];
+  int ntask;      // updates of a toggle in this network
+  unsigned task[kMaxTask];
+};
+// Counts per matrix: n*n padded so that every matrix starts on 16 bytes (they
+// are copied 16 bytes and updated 4 bytes at a time).
+__host__ __device__ constexpr size_t cm_size(int n) {
+  return ((size_t)n * n + 7) & ~(size_t)7;
+}
+// An effect's count function packed with its counters a, b, c (0xFF: none).
+constexpr int cfn_pack(int fn, int a = 0xFF, int b = 0xFF, int c = 0xFF) {
+  return fn | (a << 8) | (b << 16) | (int)((unsigned)c << 24);
+}
+
 // Canonical device form of one cusna_saom_problem. Every network is stored
 // word-major: element (w, j) of an n-actor bit matrix is word w of actor j's
 // row, at index w*n + j. Word w of row i, bit b, is the tie i -> 32*w + b.
@@ -103,9 +139,9 @@ struct DevProblem {
   const uint32_t *inact;                                    // W bits
   const int *z0, *bkdist;                                   // n
 
-  // networks, word-major W*n
-  const uint32_t *x0T, *x0cT, *simT, *simcT, *kdistT, *permT;
-  const uint32_t *keepT, *forceT, *keepcT, *forcecT;       // statistic masks
+  // networks, word-major W*n (rows and, with suffix c, in-rows)
+  const uint32_t *x0r, *x0c, *simr, *simc, *kdistr, *permr;
+  const uint32_t *keepr, *forcer, *keepc, *forcec;       // statistic masks
 
   // per-chain parameters: chain c reads row c * prow (prow 1: one row per
   // chain, as the ABI lays them out; 0: one row shared by every chain)
@@ -114,11 +150,13 @@ struct DevProblem {
 
   // effect plan (k each) and its table pool
   const int *ekind, *ecfn, *eoffd, *eofft;
+  CounterSet cnt;
+  const uint16_t *c0;  // start values of the counters held as matrices, cm_size(n) each
   const double *tab;
-  // tab's lookup values as double-float pairs: .x the float32 rounding (the
-  // float32 pass), .y the float32 rounding of the remainder (x + y is tab's
-  // value to ~2^-48, for the score sums); one 8-byte load per lookup
-  const float2 *tab2;
+  // tab's lookup values in fixed point (see the scales below); entries 0..255 of
+  // both pools are exp_fx's table
+  const uint64_t *tabq;
+  const double *ebound;  // k  bound on |d_e|
 
   // outputs (chain-major), any may be null
   double *stats, *ntim;
@@ -195,112 +233,131 @@ __device__ __forceinline__ float loglog_est(uint32_t x) {
   return logf(L);
 }
 
-// ---- double-float arithmetic ------------------------------------------------
-// An unevaluated pair (h, l) of float32 values stands for h + l, with |l| at
-// most about 2^-24 |h|: 48 significant bits on the float32 pipes, which on
-// this GPU run 64 times as many operations per cycle as the float64 pipe.
-// The error-free transformations are Knuth's TwoSum and Dekker's product
-// through a fused multiply-add (T. J. Dekker, "A floating-point technique for
-// extending the available precision", Numer. Math. 18, 1971). Every sum uses
-// the _rn intrinsics, so no compiler contraction or reassociation can change
-// the result.
-
-// s + e = a + b exactly, s = fl(a + b).
-__device__ __forceinline__ void two_sum(float a, float b, float &s, float &e) {
-  s = __fadd_rn(a, b);
-  const float bb = __fsub_rn(s, a);
-  e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+// Faster estimate of log(-log u) for the Gumbel keys, 14 instructions without a
+// branch (loglog_est above: about 80, both branches of every warp). With the
+// documented errors of lg2.approx.f32 (2^-22 absolute on (0.5, 2), 2^-22
+// relative elsewhere):
+//   L = -log u: below v = 1 - u = 1/16 the series v + v^2/2 + v^3/3 + v^4/4
+//   (omitted terms under v^4/5 = 3.1e-6 relative), else -ln2 lg2(u), relative
+//   error under (1.7e-7 + 3e-8) / L = 3.1e-6 at L = 1/16; log L then adds
+//   2^-22 ln2 |lg2 L| <= 5.5e-6 for L in [1e-10, 23]: 1e-5 in all, kGumbelErr.
+constexpr float kGumbelErr = 1.5e-5f;
+__device__ __forceinline__ float lg2_approx(float x) {
+  float r;
+  asm("lg2.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float gumbel_est(uint32_t x) {
+  const float u = fmaf((float)x, 2.3283064365386962890625e-10f, 1.16415321826934814453125e-10f);
+  const float v = fmaf((float)~x, 2.3283064365386962890625e-10f, 1.16415321826934814453125e-10f);
+  const float a = __fmul_rn(lg2_approx(u), -0.693147180559945f);
+  const float b = __fmul_rn(v, fmaf(v, fmaf(v, fmaf(v, 0.25f, 0.33333333f), 0.5f), 1.f));
+  return __fmul_rn(lg2_approx(v < 0.0625f ? b : a), 0.693147180559945f);
 }
 
-// (ah, al) += (bh, bl), keeping the pair unnormalised: the rounding error of
-// the high sum joins the low parts, whose own rounding is ~2^-24 of them.
-__device__ __forceinline__ void ff_add(float &ah, float &al, float bh, float bl) {
-  float s, e;
-  two_sum(ah, bh, s, e);
-  ah = s;
-  al = __fadd_rn(__fadd_rn(al, bl), e);
+// ---- fixed-point arithmetic of the pass over the alters ------------------------
+// A ministep's predictors and score sums are 64-bit integers: their sums are
+// exact whatever the order, so any split of the alters over warps gives the
+// same bits, and a count's term is one 64-bit multiply-add.
+//   predictor f_j          scale 2^-46 (kFBits)
+//   weight exp(f_j)        scale 2^-44 (kWBits), "no change" weighs 1
+//   real statistic d_e     |d_e| 2^sd + 2^62 as an unsigned number, sd_e from
+//                          the effect's largest |d_e| (fx_scale)
+constexpr int kFBits = 46, kWBits = 44;
+
+// Largest sd with |d| 2^sd < 2^62 for every |d| <= bound (0: a bound of 1).
+__host__ __device__ inline int fx_scale(double bound) {
+  int p = 0;
+  if (!(bound > 0.0)) bound = 1.0;
+#ifdef __CUDA_ARCH__
+  p = (int)((__double_as_longlong(bound) >> 52) & 0x7FF) - 1022;   // bound < 2^p
+#else
+  std::frexp(bound, &p);
+#endif
+  return 62 - p;
 }
 
-// The same on two independent pairs at once with the packed float32x2
-// instructions of this architecture (__fadd2_rn, __ffma2_rn: each component
-// rounded as __fadd_rn / __fmaf_rn), which issue one instruction for two
-// operations. a - b is fma(b, -1, a), one rounding of the exact difference.
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
-  return __ffma2_rn(b, make_float2(-1.f, -1.f), a);
-}
-__device__ __forceinline__ void ff_add2(float2 &ah, float2 &al, float2 bh, float2 bl) {
-  const float2 s = __fadd2_rn(ah, bh);
-  const float2 bb = sub2(s, ah);
-  const float2 e = __fadd2_rn(sub2(ah, sub2(s, bb)), sub2(bh, bb));
-  ah = s;
-  al = __fadd2_rn(__fadd2_rn(al, bl), e);
+// High 64 bits of a * b without the product of the low halves (at most 3 below
+// the exact ones).
+__host__ __device__ __forceinline__ uint64_t mulhi_fx(uint64_t a, uint64_t b) {
+  const uint32_t ah = (uint32_t)(a >> 32), al = (uint32_t)a;
+  const uint32_t bh = (uint32_t)(b >> 32), bl = (uint32_t)b;
+#ifdef __CUDA_ARCH__
+  return (uint64_t)ah * bh + __umulhi(ah, bl) + __umulhi(al, bh);
+#else
+  return (uint64_t)ah * bh + (((uint64_t)ah * bl) >> 32) + (((uint64_t)al * bh) >> 32);
+#endif
 }
 
-// Largest |x| the double-float exponential accepts; the score sums fall back
-// to float64 when a predictor leaves this range (or is not finite).
-constexpr float kFFExpMax = 60.f;
+// x, or -x for neg = 1. Written with the bits' complement: subtractions and
+// negations of 64-bit values inside a chain of additions lost a borrow in code
+// compiled for sm_103a (nvcc 13.0) when the subtracted value's low word was 0, so
+// the fixed-point code adds only.
+__host__ __device__ __forceinline__ int64_t signed_fx(uint64_t x, int neg) {
+  const uint32_t s = 0u - (uint32_t)neg;
+  return (int64_t)((x ^ ((uint64_t)s << 32 | s)) + (uint32_t)neg);
+}
 
-// ln(2)/64 split as C1 + C2 + C3: C1 has 11 significant bits, so N*C1 is exact
-// for |N| < 2^13 (|x| <= 60 gives |N| <= 5540); C2 and C3 are the next two
-// float32 roundings of the remainder (the split leaves 1.8e-22).
-constexpr float kLn2o64C1 = 0x1.63p-7f;
-constexpr float kLn2o64C2 = -0x1.bd0106p-19f;
-constexpr float kLn2o64C3 = 0x1.cf79acp-46f;
-constexpr float k64oLn2 = 0x1.715476p+6f;   // 64/ln(2), only to choose N
+// exp(f 2^-46) 2^(44 - sh) rounded, for |f| < 2^61 and a result below 2^63, by
+// Tang's table-driven method (P. T. P. Tang, "Table-driven implementation of the
+// exponential function in IEEE floating-point arithmetic", ACM TOMS 15(2), 1989)
+// in integers: f = N ln2/256 + r with |r| <= 0.53 ln2/256 = 0.00143 at scale
+// 2^-62; e^r - 1 = r + r^2/2 (from r at 2^-40: error 1.3e-15) + r^3/6 + r^4/24
+// (float32; the omitted r^5/120 is 5e-17); tab[N & 255] = 2^((N & 255)/256) at
+// 2^-62, as (high, signed low) words; then the power of two. Relative error
+// below 3e-15 + the rounding to 2^-(44-sh).
+__host__ __device__ __forceinline__ uint64_t exp_fx(int64_t f, int sh, const int2 *tab) {
+  const int fh = (int)(f >> 32);   // scale 2^-14
+  // N = round(f 256/ln2): 256/ln2 = 369.3299304675746 at 2^-20
+  const int N = (int)(((int64_t)fh * 387270501 + ((int64_t)1 << 33)) >> 34);
+  // ln2/256 at 2^-62
+  const int64_t r = (int64_t)((uint64_t)f << 16) + (int64_t)N * -12486629536330718LL;
+  const int s = (int)(r >> 22);    // scale 2^-40
+  const float rf = (float)s * 9.094947017729282e-13f;
+  const int c3 = (int)(rf * rf * rf * (rf * 0.041666668f + 0.16666667f) * 1.152921504606847e18f);
+  const int64_t e = r + (((int64_t)s * s) >> 19) + ((int64_t)c3 << 2);   // c3 at 2^-60
+  const int2 t = tab[N & 255];
+  const int64_t T = ((int64_t)t.x << 32) + t.y;
+  const int eh = (int)(e >> 32);
+  const uint32_t el = (uint32_t)e;
+  const int64_t lowp = (int64_t)t.x * el + (int64_t)t.y * eh;
+  const uint64_t m = (uint64_t)(T + (((int64_t)t.x * eh) << 2) + (lowp >> 30));
+  int k = 17 - (N >> 8) + sh;      // one less than the shift, for the rounding
+  if (k > 62) return 0;
+  if (k < 0) k = 0;                // out of range: the caller repeats with a larger sh
+  return ((m >> k) + 1) >> 1;
+}
 
-// The table 2^(j/64), j = 0..63, as double-float pairs (h, l): computed from
-// the float64 exp2, whose error is far below the pair's 2^-48.
-__device__ __forceinline__ void fill_exp_table(float2 *tab, int tl, int L) {
-  for (int j = tl; j < 64; j += L) {
-    const double v = exp2((double)j * 0.015625);
-    const float h = (float)v;
-    tab[j] = make_float2(h, (float)__dsub_rn(v, (double)h));
+// 2^(j/256) at scale 2^-62 as exp_fx's table entry.
+__host__ __device__ __forceinline__ int2 exp_fx_entry(double v) {   // v = 2^(j/256)
+  const int64_t T = (int64_t)(v * 4611686018427387904.0);
+  const int lo = (int)(uint32_t)T;
+  int2 t;
+  t.x = (int)((T - lo) >> 32);
+  t.y = lo;
+  return t;
+}
+
+// Bound on |d_e| of effect type t for the fixed-point scale and range check
+// (vmax, wmax: the largest |covariate| and |weight|; dmax: of a table).
+__host__ __device__ inline double effect_bound(int t, int n, double vmax, double wmax, double p1,
+                                               double p2) {
+  const double N = n, a1 = p1 < 0 ? -p1 : p1, a2 = p2 < 0 ? -p2 : p2;
+  switch (t) {
+    case 0: case 1: case 13: case 20: case 31: case 33: case 34: case 35: return 1.0;
+    case 2: case 6: case 16: case 19: return 2.0 * N + 1.0;
+    case 3: case 23: case 4: case 5: case 8: case 14: case 36: case 37: return N + 1.0;
+    case 7: case 9: case 15: return N + 1.0;
+    case 17: return 2.0 * N + 2.0;    // 1.5 sqrt(n + 1) at most
+    case 18: return N + 1.0 + a1;
+    case 10: case 11: return vmax;
+    case 12: return 1.0 + 2.0 * vmax * a1 + a2;
+    case 21: return vmax * vmax;
+    case 25: return 2.0 * vmax;
+    case 24: case 26: case 27: case 28: return wmax;
+    case 29: case 30: return 2.0 * N * wmax;
+    default: return 1.0;
   }
-}
-
-// exp(xh + xl) as a double-float pair (wh, wl) for |xh| <= kFFExpMax, relative
-// error below about 2e-14. Tang's table-driven method (P. T. P. Tang, "Table-
-// driven implementation of the exponential function in IEEE floating-point
-// arithmetic", ACM TOMS 15(2), 1989) in double-float arithmetic:
-//   x = N ln2/64 + r, |r| <= ln2/128 (Cody-Waite reduction with the three-part
-//   constant above, the first product exact, the second through Dekker's
-//   product, so r is known to ~1e-18);
-//   exp(r) - 1 = r + r^2/2 + r^3/6 + r^4/24 + r^5/120 (the omitted terms are
-//   below 4e-17): the first two terms in double-float, the rest in float32
-//   (their sum is below 2.7e-8, so its rounding is below 2e-15);
-//   exp(x) = 2^(N>>6) * 2^((N&63)/64) * exp(r), the table entry multiplied in
-//   double-float and the power of two applied exactly to both halves.
-__device__ __forceinline__ void exp_ff(float xh, float xl, const float2 *tab, float &wh,
-                                       float &wl) {
-  const float Nf = rintf(__fmul_rn(xh, k64oLn2));
-  const int N = (int)Nf;
-  const float t1 = fmaf(-Nf, kLn2o64C1, xh);  // exact
-  const float p = __fmul_rn(Nf, kLn2o64C2);
-  const float pe = fmaf(Nf, kLn2o64C2, -p);  // p + pe = N C2 exactly
-  float rh, e;
-  two_sum(t1, -p, rh, e);
-  const float rl = __fadd_rn(__fsub_rn(__fsub_rn(e, pe), __fmul_rn(Nf, kLn2o64C3)), xl);
-  // r^2 = sqh + sql (dropping rl^2 < 1e-19)
-  const float sqh = __fmul_rn(rh, rh);
-  const float sql = fmaf(__fmul_rn(2.f, rh), rl, fmaf(rh, rh, -sqh));
-  // r^3/6 + r^4/24 + r^5/120, plus the r^2 rl / 2 part of the cubic term
-  const float q = fmaf(__fmul_rn(sqh, rh),
-                       fmaf(rh, fmaf(rh, 8.3333333333e-3f, 4.1666666667e-2f), 1.6666666667e-1f),
-                       __fmul_rn(__fmul_rn(0.5f, sqh), rl));
-  float sh, e1;
-  two_sum(rh, __fmul_rn(0.5f, sqh), sh, e1);
-  const float sl = __fadd_rn(__fadd_rn(__fadd_rn(rl, __fmul_rn(0.5f, sql)), q), e1);
-  // T (1 + sh + sl), T = 2^((N & 63)/64) in [1, 2) as (T.x, T.y)
-  const float2 T = tab[N & 63];
-  const float ph = __fmul_rn(T.x, sh);
-  const float pl = fmaf(T.x, sh, -ph);
-  const float h = __fadd_rn(T.x, ph);  // |T.x| >= 1 > |ph|: Fast2Sum
-  float l = __fsub_rn(ph, __fsub_rn(h, T.x));
-  l = __fadd_rn(l, __fadd_rn(pl, fmaf(T.x, sl, fmaf(T.y, sh, T.y))));
-  // 2^(N >> 6), N >> 6 in [-87, 86]: a normal float32
-  const float s = __int_as_float(((N >> 6) + 127) << 23);
-  wh = __fmul_rn(h, s);
-  wl = __fmul_rn(l, s);
 }
 
 }  // namespace cusna

@@ -8,6 +8,7 @@
 #include <nvrtc.h>
 #include <nvtx3/nvToolsExt.h>
 
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <condition_variable>
@@ -46,52 +47,29 @@ struct Gen {
   }
 };
 
-const int kPcAll = F_PC_RI_CJ | F_PC_RI_RJ | F_PC_RJ_CI | F_PC_CI_CJ | F_PC_CI_RJ | F_PC_RICIRJ;
-
-void gen_pair_counts(Gen &g, int fl) {
-  g.s += "  int ri_cj = 0, ri_rj = 0, rj_ci = 0, ci_cj = 0, ci_rj = 0, ricirj = 0;\n"
-         "  (void)ri_cj; (void)ri_rj; (void)rj_ci; (void)ci_cj; (void)ci_rj; (void)ricirj;\n";
-  if (!(fl & kPcAll)) return;
-  g.s += "  for (int w = 0; w < W; ++w) {\n"
-         "    const uint32_t ri = S.rowsT[w * n + i], rj = S.rowsT[w * n + j];\n"
-         "    const uint32_t ci = S.colsT[w * n + i], cj = S.colsT[w * n + j];\n"
-         "    (void)ri; (void)rj; (void)ci; (void)cj;\n";
-  if (fl & F_PC_RI_CJ) g.s += "    ri_cj += __popc(ri & cj);\n";
-  if (fl & F_PC_RI_RJ) g.s += "    ri_rj += __popc(ri & rj);\n";
-  if (fl & F_PC_RJ_CI) g.s += "    rj_ci += __popc(rj & ci);\n";
-  if (fl & F_PC_CI_CJ) g.s += "    ci_cj += __popc(ci & cj);\n";
-  if (fl & F_PC_CI_RJ) g.s += "    ci_rj += __popc(ci & rj);\n";
-  if (fl & F_PC_RICIRJ) g.s += "    ricirj += __popc(ri & ci & rj);\n";
-  g.s += "  }\n";
-}
-
 // the integer magnitude c of a K_CNT effect, or the table index of a K_LOOK one
-void gen_count(Gen &g, int cfn) {
-  switch (cfn) {
+void gen_count(Gen &g, int pk) {
+  const int ca = (pk >> 8) & 0xFF, cb = (pk >> 16) & 0xFF, cc = (pk >> 24) & 0xFF;
+  switch (pk & 0xFF) {
     case 0: g.s += "    const int c = 1;\n"; break;
     case 1: g.s += "    const int c = aji;\n"; break;
-    case 2: g.s += "    const int c = ri_cj + ri_rj;\n"; break;
-    case 3: g.s += "    const int c = rj_ci;\n"; break;
+    case 2: case 3: g.put("    const int c = q%d;\n", ca); break;
     case 4: g.s += "    const int c = S.indeg[j] + 1 - aij;\n"; break;
     case 5:
-      g.s += "    int c = 0;\n"
-             "    const uint32_t *eq = S.tpeq + (aij ? W : 0);\n"
-             "    for (int w = 0; w < W; ++w)\n"
-             "      c += __popc(S.rowsT[w * n + i] & S.rowsT[w * n + j] & eq[w]);\n"
-             "    if (S.tp[j] > 0) ++c;\n";
+      // counter ca holds the one of the two that a_ij selects (gen_popcounts)
+      g.put("    const int c = q%d + (q%d > 0 ? 1 : 0);\n", ca, cc);
       break;
-    case 6: g.s += "    const int c = (aji ? ri_cj : 0) + ricirj;\n"; break;
+    case 6:
+      g.put("    const int c = (aji ? q%d : 0) + q%d;\n", ca, cb);
+      break;
     default: g.s += "    const int c = S.outdeg[j];\n"; break;
   }
 }
-void gen_index(Gen &g, int cfn) {
-  switch (cfn) {
+void gen_index(Gen &g, int pk) {
+  switch (pk & 0xFF) {
     case 4: g.s += "    const int idx = S.indeg[j] + 1 - aij;\n"; break;
     case 7: g.s += "    const int idx = S.outdeg[j];\n"; break;
-    case 8: g.s += "    const int idx = ri_cj;\n"; break;
-    case 9: g.s += "    const int idx = ri_rj;\n"; break;
-    case 10: g.s += "    const int idx = ci_cj;\n"; break;
-    case 11: g.s += "    const int idx = ci_rj;\n"; break;
+    case 8: g.put("    const int idx = q%d;\n", (pk >> 8) & 0xFF); break;
     case 12: g.s += "    const int idx = j;\n"; break;
     case 13: g.s += "    const int idx = S.z[j] - P.zlo;\n"; break;
     case 14: g.s += "    const int idx = i * n + j;\n"; break;
@@ -105,109 +83,194 @@ void gen_shape(Gen &g, const JitPlan &J) {
   else g.s += "  const int n = P.n, W = P.W;\n";
 }
 
+// The plan's two-path counts of alter j as constants-indexed variables q0, q1, ...:
+// row i of the matrices the chain keeps (mask), popcounts of the rest in one
+// loop over the words. With n read at run time the matrices are the problem's
+// choice.
+const char *set_word(int list) {
+  switch (list) {
+    case CL_OUT: return "ri";
+    case CL_IN: return "ci";
+    case CL_MUTUAL: return "(ri & ci)";
+    case CL_TP0: return "(ri & S.tpeq[aij ? W + w : w])";  // the one that a_ij selects
+    default: return nullptr;
+  }
+}
+void gen_popcounts(Gen &g, const CounterSet &C, unsigned which, const char *ind) {
+  if (!which) return;
+  bool ri = false, ci = false, rj = false, cj = false;
+  std::string nets;
+  for (int c = 0; c < C.n; ++c) {
+    if (!((which >> c) & 1u)) continue;
+    const int l = C.list[c];
+    ri |= l == CL_OUT || l == CL_MUTUAL || l == CL_TP0 || l == CL_TP1;
+    ci |= l == CL_IN || l == CL_MUTUAL;
+    for (int m : {(int)C.m1[c], (int)C.m2[c]}) {
+      cj |= m == CM_ROWS;
+      rj |= m == CM_COLS;
+    }
+  }
+  g.put("%sfor (int w = 0; w < W; ++w) {\n", ind);
+  if (ri) g.put("%s  const uint32_t ri = S.rows[w * n + i];\n", ind);
+  if (ci) g.put("%s  const uint32_t ci = S.cols[w * n + i];\n", ind);
+  if (rj) g.put("%s  const uint32_t rj = S.rows[w * n + j];\n", ind);
+  if (cj) g.put("%s  const uint32_t cj = S.cols[w * n + j];\n", ind);
+  for (int c = 0; c < C.n; ++c) {
+    if (!((which >> c) & 1u) || C.list[c] == CL_TP1) continue;
+    const int l = C.list[c];
+    std::string a = l >= CL_NET ? "X.net.rows[" + std::to_string(l - CL_NET) + " * X.net.row_stride + w * n + i]"
+                                : std::string(set_word(l));
+    for (int m : {(int)C.m1[c], (int)C.m2[c]}) {
+      if (m == CM_NONE) continue;
+      const std::string r = m == CM_ROWS ? "cj" : (m == CM_COLS ? "rj" : "X.net.rows[" +
+                            std::to_string(m - CM_NCOLS) + " * X.net.row_stride + w * n + j]");
+      g.put("%s  q%d += __popc(%s & %s);\n", ind, c, a.c_str(), r.c_str());
+    }
+  }
+  g.put("%s}\n", ind);
+}
+// The counts of alter j as variables q0, q1, ...: row i of the matrices that the
+// chain keeps, popcounts of the rest in one loop over the words. With n read at
+// run time the matrices are the problem's choice.
+void gen_counts(Gen &g, const JitPlan &J) {
+  const CounterSet &C = J.cnt;
+  unsigned all = 0, can = 0;
+  for (int c = 0; c < C.n; ++c) {
+    all |= 1u << c;
+    if (C.list[c] == CL_OUT || C.list[c] == CL_IN || C.list[c] >= CL_NET) can |= 1u << c;
+    g.put("  int q%d = 0;\n  (void)q%d;\n", c, c);
+  }
+  auto reads = [&](const char *ind) {
+    for (int c = 0, r = 0; c < C.n; ++c)
+      if ((can >> c) & 1u)
+        g.put("%sq%d = S.cm[%d * cm_size(n) + (size_t)i * n + j];\n", ind, c, r++);
+  };
+  if (J.n > 0) {
+    if (C.mask) reads("  ");
+    gen_popcounts(g, C, all & ~C.mask, "  ");
+  } else {
+    if (can) {
+      g.s += "  if (P.cnt.mask) {\n";
+      reads("    ");
+      g.s += "  } else {\n";
+      gen_popcounts(g, C, can, "    ");
+      g.s += "  }\n";
+    }
+    gen_popcounts(g, C, all & ~can, "  ");
+  }
+}
+
+// a generic effect's two-path count argument
+std::string gen_cnt_arg(int ca) {
+  return ca == 0xFF ? "0" : "q" + std::to_string(ca);
+}
+
+// a cross effect's magnitude
+void gen_cross(Gen &g, int e, int cfn, int ca) {
+  if (cfn >= 36) g.put("    const int c = q%d;\n", ca);
+  else g.put("    const int c = cross_count(P, S, X, n, %d, S.eoffd[%d], 255, i, j);\n", cfn, e);
+}
+
 // jit_change_stats32<sfx> and jit_change_stats<sfx><TERMS> of one effect plan
 void gen_functions(Gen &g, const JitPlan &J, const std::string &sfx, bool multi) {
   const int k = (int)J.kind.size();
-  const int fl = J.pc_flags;
   const char *x = sfx.c_str();
-  // float32 pass (change_stats32), with the double-float remainders of the
-  // change statistics and of the predictor for the score sums
-  g.put("__device__ __forceinline__ float jit_change_stats32%s(const DevProblem &P, const Slice &S,\n"
-        "    const StepCtx &X, int j, int aij, int aji, float *d32, float *d32lo, float *absf,\n"
-        "    float2 *fx) {\n", x);
+  // the fixed-point pass (change_fixed)
+  g.put("__device__ __forceinline__ int64_t jit_change_fixed%s(const DevProblem &P, const Slice &S,\n"
+        "    const StepCtx &X, int j, int aij, int aji, uint64_t *v) {\n", x);
   g.s += "  const int i = X.i;\n";
   gen_shape(g, J);
-  g.s += "  (void)n; (void)W; (void)i; (void)aji; (void)d32lo;\n";
-  gen_pair_counts(g, fl);
-  g.put("  const uint32_t sg = aij ? 0x80000000u : 0u;\n"
-        "  float f = 0.f, a = 0.f, tt[%d], tl[%d];\n", k, k);
+  g.s += "  (void)n; (void)W; (void)i; (void)aji; (void)v;\n";
+  gen_counts(g, J);
+  g.s += "  int64_t f = X.f0;\n";
   for (int e = 0; e < k; ++e) {
-    const int kind = J.kind[e], cfn = J.cfn[e], t = J.tid[e];
+    const int kind = J.kind[e], pk = J.cfn[e], cfn = pk & 0xFF, ca = (pk >> 8) & 0xFF, t = J.tid[e];
+    const int cls = fx_class(kind, cfn, t, J.ety[e]);
+    if (cls < FX_CNT) continue;
     g.put("  {  // effect %d: type %d, kind %d, function %d\n", e, t, kind, cfn);
-    g.put("    const float th = S.th32[%d];\n", e);
-    g.s += "    float v, vlo = 0.f, term = 0.f, tlo = 0.f;\n    bool has_term = true;\n"
-           "    (void)th; (void)vlo;\n";
-    if (kind == K_CNT) {
-      gen_count(g, cfn);
-      g.s += "    v = __uint_as_float(__float_as_uint((float)c) ^ sg);\n"
-             "    term = __fmul_rn(th, v);\n";
-      // c in {0, 1} (density, reciprocity): theta * v is exact
-      if (cfn != 0 && cfn != 1) g.s += "    tlo = fmaf(th, v, -term);\n";
-    } else if (kind == K_LOOK) {
-      gen_index(g, cfn);
-      g.put("    const float2 t2 = P.tab2[S.eoffd[%d] + idx];\n"
-            "    v = __uint_as_float(__float_as_uint(t2.x) ^ sg);\n"
-            "    vlo = __uint_as_float(__float_as_uint(t2.y) ^ sg);\n"
-            "    term = __fmul_rn(th, v);\n"
-            "    tlo = fmaf(th, vlo, fmaf(th, v, -term));\n", e);
-    } else if (kind == K_STEP) {
-      g.put("    const int q = 2 * aij + aji;\n"
-            "    v = S.stepd32[%d + q];\n    vlo = S.stepdlo32[%d + q];\n"
-            "    term = S.stept32[%d + q];\n    tlo = S.steptlo32[%d + q];\n",
-            4 * e, 4 * e, 4 * e, 4 * e);
-    } else if (kind == K_ZERO) {
-      g.s += "    v = 0.f;\n    has_term = false;\n";
-    } else if (multi && kind == K_CROSS) {
-      g.put("    const int c = cross_count(S, X, n, W, %d, S.eoffd[%d], i, j);\n"
-            "    const bool rt = %d == 36 && S.p1[%d] >= 2.0;\n"
-            "    const float m = rt ? sqrtf((float)c) : (float)c;\n"
-            "    const float mlo = (rt && c > 0) ? __fdiv_rn(fmaf(-m, m, (float)c), __fmul_rn(2.f, m)) : 0.f;\n"
-            "    v = __uint_as_float(__float_as_uint(m) ^ sg);\n"
-            "    vlo = __uint_as_float(__float_as_uint(mlo) ^ sg);\n"
-            "    term = __fmul_rn(th, v);\n"
-            "    tlo = fmaf(th, vlo, fmaf(th, v, -term));\n", cfn, e, cfn, e);
-    } else if (t == 32) {
-      const int c0 = J.i0[e], c1 = J.i1[e], c2 = J.i2[e];
-      g.put("    v = __fmul_rn(d32[%d], d32[%d]);\n"
-            "    vlo = __fadd_rn(fmaf(d32[%d], d32[%d], -v),\n"
-            "                    fmaf(d32[%d], d32lo[%d], __fmul_rn(d32lo[%d], d32[%d])));\n",
-            c0, c1, c0, c1, c0, c1, c0, c1);
-      if (c2 >= 0)
-        g.put("    {\n      const float v2 = __fmul_rn(v, d32[%d]);\n"
-              "      vlo = __fadd_rn(fmaf(v, d32[%d], -v2), fmaf(v, d32lo[%d], __fmul_rn(vlo, d32[%d])));\n"
-              "      v = v2;\n    }\n", c2, c2, c2, c2);
-      else g.s += "    if (aij) { v = -v; vlo = -vlo; }\n";
-      g.s += "    term = __fmul_rn(th, v);\n"
-             "    tlo = fmaf(th, vlo, fmaf(th, v, -term));\n";
-    } else {
-      g.put("    {\n      const double v64 = gen_stat(P, S, X, %d, j, aij, aji, ri_cj, ri_rj, rj_ci,\n"
-            "                                  ci_cj, ci_rj, nullptr);\n"
-            "      v = (float)v64;\n      vlo = (float)__dsub_rn(v64, (double)v);\n    }\n"
-            "    term = __fmul_rn(th, v);\n"
-            "    tlo = fmaf(th, vlo, fmaf(th, v, -term));\n", e);
+    const char *off = J.ety[e] == 1 ? "aij" : (J.ety[e] == 2 ? "!aij" : nullptr);
+    if (cls == FX_CNT) {
+      if (multi && kind == K_CROSS) gen_cross(g, e, cfn, ca);
+      else gen_count(g, pk);
+      if (off) g.put("    const int m = %s ? 0 : c;\n", off);
+      else g.s += "    const int m = c;\n";
+      g.put("    v[%d] = (uint64_t)m;\n", e);
+      if (kind == K_CNT && cfn == 1) g.put("    f += m ? (int64_t)S.thq[%d] : 0;\n  }\n", e);
+      else g.put("    f += (int64_t)S.thq[%d] * m;\n  }\n", e);
+      continue;
     }
-    if (J.ety[e] == 1) g.s += "    if (aij) { v = 0.f; vlo = 0.f; has_term = false; }\n";
-    else if (J.ety[e] == 2) g.s += "    if (!aij) { v = 0.f; vlo = 0.f; has_term = false; }\n";
-    g.put("    d32[%d] = v;\n    d32lo[%d] = vlo;\n", e, e);
-    g.put("    tt[%d] = has_term ? term : 0.f;\n    tl[%d] = has_term ? tlo : 0.f;\n", e, e);
-    g.s += "    if (has_term) {\n      f = __fadd_rn(f, term);\n"
-           "      a = __fadd_rn(a, fabsf(term));\n    }\n  }\n";
+    if (kind == K_LOOK) {
+      gen_index(g, pk);
+      g.put("    const uint64_t m = X.tabq[S.eoffd[%d] + idx];\n", e);
+    } else if (kind == K_STEP) {
+      g.put("    const uint64_t m = S.stepq[%d + 2 * aij + aji];\n", 4 * e);
+    } else if (t == 32) {
+      auto mag = [&](int q) {
+        const int cl = fx_class(J.kind[q], J.cfn[q] & 0xFF, J.tid[q], J.ety[q]);
+        char b[128];
+        if (cl == FX_DELTA) std::snprintf(b, sizeof b, "((int64_t)1 << S.esd[%d])", q);
+        else if (cl == FX_CNT) std::snprintf(b, sizeof b, "((int64_t)v[%d] << S.esd[%d])", q, q);
+        else if (cl == FX_UNI) std::snprintf(b, sizeof b, "(int64_t)(S.stepq[%d] - (1ull << 62))", 4 * q);
+        else if (cl == FX_REAL) std::snprintf(b, sizeof b, "(v[%d] ? (int64_t)(v[%d] - (1ull << 62)) : 0)", q, q);
+        else std::snprintf(b, sizeof b, "(int64_t)0");
+        return std::string(b);
+      };
+      g.put("    int64_t p = __mul64hi(%s, %s);\n", mag(J.i0[e]).c_str(), mag(J.i1[e]).c_str());
+      if (J.i2[e] >= 0) g.put("    p = __mul64hi(p, %s);\n", mag(J.i2[e]).c_str());
+      g.s += "    const uint64_t m = (uint64_t)(p + (1LL << 62));\n";
+    } else if (cfn == 16) {
+      g.put("    const uint64_t m = gw_fixed(S, X, n, W, %d, %d, j, aij);\n", e, t);
+    } else {
+      g.put("    const double d = gen_stat(P, S, X, %d, j, aij, aji, %s, nullptr);\n"
+            "    const uint64_t m = real_fx(aij ? -d : d, S.esd[%d]);\n", e, gen_cnt_arg(ca).c_str(), e);
+    }
+    char tb[96];
+    std::snprintf(tb, sizeof tb, "term_fx(S.thq[%d], S.ecls[%d], m)", e, e);
+    if (off) {
+      g.put("    v[%d] = %s ? 0 : m;\n    if (!(%s)) f += %s + base_fx(S.thq[%d], S.ecls[%d]);\n  }\n", e,
+            off, off, tb, e, e);
+    } else {
+      g.put("    v[%d] = m;\n    f += %s;\n  }\n", e, tb);
+    }
   }
-  // the predictor as a double-float pair: the terms' pairs added in a fixed
-  // packed tree (f, the float32 sum in effect order, keys the choice)
-  g.put("  *absf = a;\n  *fx = ff_tree_sum<%d>(tt, tl);\n  return f;\n}\n", k);
+  g.s += "  return f;\n}\n";
+  // the score sums (sums_add)
+  g.put("template <int V>\n__device__ __forceinline__ void jit_sums_add%s(int64_t (&acc)[V], uint64_t W, int aij,\n"
+        "    const uint64_t *v) {\n"
+        "  const int64_t wd = signed_fx(W, aij);\n  const uint64_t w6 = W << 6;\n"
+        "  (void)v; (void)w6;\n  acc[0] += (int64_t)W;\n  acc[1] += wd;\n", x);
+  for (int e = 0; e < k; ++e) {
+    const int cfn = J.cfn[e] & 0xFF, cls = fx_class(J.kind[e], cfn, J.tid[e], J.ety[e]);
+    if (cls == FX_CNT && J.kind[e] == K_CNT && cfn == 1)
+      g.put("  acc[%d] += v[%d] ? wd : 0;\n", 2 + e, e);
+    else if (cls == FX_CNT)
+      g.put("  acc[%d] += wd * (int64_t)(uint32_t)v[%d];\n", 2 + e, e);
+    else if (cls == FX_REAL)
+      g.put("  acc[%d] += signed_fx(mulhi_fx(w6, v[%d]), aij);\n", 2 + e, e);
+  }
+  g.s += "}\n";
   // float64 evaluation (change_stats): the chosen alter and uncertified choices
   g.put("template <bool TERMS>\n"
         "__device__ __forceinline__ double jit_change_stats%s(const DevProblem &P, const Slice &S,\n"
         "    const StepCtx &X, int j, int aij, int aji, double *d) {\n", x);
   g.s += "  const int i = X.i;\n";
   gen_shape(g, J);
-  g.s += "  (void)n; (void)W; (void)i; (void)aji;\n"
-         "  const unsigned long long sg = aij ? 0x8000000000000000ull : 0ull;\n"
+  g.s += "  (void)n; (void)W; (void)i; (void)aji;\n";
+  gen_counts(g, J);
+  g.s += "  const unsigned long long sg = aij ? 0x8000000000000000ull : 0ull;\n"
          "  const bool ttab = (P.flags & F_THETA_TAB) != 0;\n  (void)ttab;\n";
-  gen_pair_counts(g, fl);
   g.s += "  double f = 0.0;\n";
   for (int e = 0; e < k; ++e) {
-    const int kind = J.kind[e], cfn = J.cfn[e];
+    const int kind = J.kind[e], pk = J.cfn[e], cfn = pk & 0xFF, ca = (pk >> 8) & 0xFF;
     g.put("  {  // effect %d\n", e);
     g.s += "    double v, term = 0.0;\n    bool has_term = TERMS;\n";
     if (kind == K_CNT) {
-      gen_count(g, cfn);
+      gen_count(g, pk);
       g.put("    v = flip(i2d(c), sg);\n"
             "    if (TERMS) term = ttab ? flip(P.tab[S.eofft[%d] + c], sg) : __dmul_rn(S.th[%d], v);\n",
             e, e);
     } else if (kind == K_LOOK) {
-      gen_index(g, cfn);
+      gen_index(g, pk);
       g.put("    v = flip(P.tab[S.eoffd[%d] + idx], sg);\n"
             "    if (TERMS) term = ttab ? flip(P.tab[S.eofft[%d] + idx], sg) : __dmul_rn(S.th[%d], v);\n",
             e, e, e);
@@ -217,12 +280,12 @@ void gen_functions(Gen &g, const JitPlan &J, const std::string &sfx, bool multi)
     } else if (kind == K_ZERO) {
       g.s += "    v = 0.0;\n    has_term = false;\n";
     } else if (multi && kind == K_CROSS) {
-      g.put("    const int c = cross_count(S, X, n, W, %d, S.eoffd[%d], i, j);\n"
-            "    v = flip((%d == 36 && S.p1[%d] >= 2.0) ? sqrt(i2d(c)) : i2d(c), sg);\n"
-            "    if (TERMS) term = __dmul_rn(S.th[%d], v);\n", cfn, e, cfn, e, e);
+      gen_cross(g, e, cfn, ca);
+      g.put("    v = flip((%d == 36 && S.p1[%d] >= 2.0) ? sqrt(i2d(c)) : i2d(c), sg);\n"
+            "    if (TERMS) term = __dmul_rn(S.th[%d], v);\n", cfn, e, e);
     } else {
-      g.put("    v = gen_stat(P, S, X, %d, j, aij, aji, ri_cj, ri_rj, rj_ci, ci_cj, ci_rj, d);\n"
-            "    if (TERMS) term = __dmul_rn(S.th[%d], v);\n", e, e);
+      g.put("    v = gen_stat(P, S, X, %d, j, aij, aji, %s, d);\n"
+            "    if (TERMS) term = __dmul_rn(S.th[%d], v);\n", e, gen_cnt_arg(ca).c_str(), e);
     }
     if (J.ety[e] == 1) g.s += "    if (aij) { v = 0.0; has_term = false; }\n";
     else if (J.ety[e] == 2) g.s += "    if (!aij) { v = 0.0; has_term = false; }\n";
@@ -234,19 +297,20 @@ void gen_functions(Gen &g, const JitPlan &J, const std::string &sfx, bool multi)
 
 }  // namespace
 
-// Effects whose change statistic can have a double-float remainder: every
-// kind but the integer counts (and the zero dyadic covariate).
-unsigned lo_mask(const JitPlan &J) {
-  unsigned m = 0;
+// The score-sum quantities that a plan uses (saom_chain.cuh).
+unsigned quantity_mask(const JitPlan &J) {
+  unsigned m = 3;
   for (size_t e = 0; e < J.kind.size(); ++e)
-    if (J.kind[e] != K_CNT && J.kind[e] != K_ZERO) m |= 1u << e;
+    if (fx_class(J.kind[e], J.cfn[e] & 0xFF, J.tid[e], J.ety[e]) >= FX_CNT) m |= 4u << e;
   return m;
 }
 
 std::string jit_spec_source(const JitPlan &J) {
   Gen g;
-  g.put("#define CUSNA_JIT_SPEC 1\n#define CUSNA_JIT_K %d\n#define CUSNA_JIT_LOMASK 0x%xu\n"
-        "namespace cusna {\n", (int)J.kind.size(), lo_mask(J));
+  g.put("#define CUSNA_JIT_SPEC 1\n#define CUSNA_JIT_K %d\n#define CUSNA_FX_V %d\n"
+        "#define CUSNA_FX_MASK 0x%xu\nnamespace cusna {\n", (int)J.kind.size(),
+        (int)J.kind.size() + 2, quantity_mask(J));
+  if (J.n > 0) g.put("#define CUSNA_JIT_N %d\n", J.n);
   gen_functions(g, J, "", false);
   g.s += "}  // namespace cusna\n";
   return g.s;
@@ -254,25 +318,35 @@ std::string jit_spec_source(const JitPlan &J) {
 
 std::string jit_multi_spec_source(const std::vector<JitPlan> &nets) {
   Gen g;
-  g.s += std::string(kJitMultiTag) + "\n#define CUSNA_JIT_MULTI 1\nnamespace cusna {\n";
+  unsigned mask = 0;
+  size_t kmax = 0;
+  for (const JitPlan &J : nets) {
+    mask |= quantity_mask(J);
+    kmax = std::max(kmax, J.kind.size());
+  }
+  g.s += std::string(kJitMultiTag) + "\n#define CUSNA_JIT_MULTI 1\n";
+  g.put("#define CUSNA_FX_V %d\n#define CUSNA_FX_MASK 0x%xu\nnamespace cusna {\n", (int)kmax + 2, mask);
   const int D = (int)nets.size();
   for (int d = 0; d < D; ++d) gen_functions(g, nets[d], "_n" + std::to_string(d), true);
   // the chosen network's plan (warp-uniform per ministep)
-  g.s += "__device__ __forceinline__ float jit_change_stats32(int net, const DevProblem &P,\n"
-         "    const Slice &S, const StepCtx &X, int j, int aij, int aji, float *d32, float *d32lo,\n"
-         "    float *absf, float2 *fx) {\n"
+  g.s += "__device__ __forceinline__ int64_t jit_change_fixed(int net, const DevProblem &P,\n"
+         "    const Slice &S, const StepCtx &X, int j, int aij, int aji, uint64_t *v) {\n"
          "  switch (net) {\n";
   for (int d = 0; d < D; ++d)
-    g.put("    case %d: return jit_change_stats32_n%d(P, S, X, j, aij, aji, d32, d32lo, absf, fx);\n",
-          d, d);
-  g.s += "    default: *absf = 0.f; *fx = make_float2(0.f, 0.f); return 0.f;\n  }\n}\n";
+    g.put("    case %d: return jit_change_fixed_n%d(P, S, X, j, aij, aji, v);\n", d, d);
+  g.s += "    default: return 0;\n  }\n}\n";
+  g.s += "template <int V>\n__device__ __forceinline__ void jit_sums_add(int net, int64_t (&acc)[V],\n"
+         "    uint64_t W, int aij, const uint64_t *v) {\n  switch (net) {\n";
+  for (int d = 0; d < D; ++d) g.put("    case %d: jit_sums_add_n%d(acc, W, aij, v); break;\n", d, d);
+  g.s += "    default: break;\n  }\n}\n";
   g.s += "template <bool TERMS>\n"
          "__device__ __forceinline__ double jit_change_stats(int net, const DevProblem &P,\n"
          "    const Slice &S, const StepCtx &X, int j, int aij, int aji, double *d) {\n"
          "  switch (net) {\n";
   for (int d = 0; d < D; ++d)
     g.put("    case %d: return jit_change_stats_n%d<TERMS>(P, S, X, j, aij, aji, d);\n", d, d);
-  g.s += "    default: return 0.0;\n  }\n}\n}  // namespace cusna\n";
+  g.s += "    default: return 0.0;\n  }\n}\n";
+  g.s += "}  // namespace cusna\n";
   return g.s;
 }
 
@@ -807,8 +881,7 @@ int jit_blocks_per_sm(const JitKernel &K, int threads, size_t dyn_smem) {
 
 cudaError_t launch_period_jit(const JitKernel &K, const LaunchShape &sh, const DevProblem *probs,
                               const long long *unit_start, int nprob, long long total,
-                              unsigned long long *counter, uint32_t *cols_scratch,
-                              uint32_t *rows_scratch, size_t cols_words, cudaStream_t st) {
+                              unsigned long long *counter, const Scratch &sc, cudaStream_t st) {
   const Driver &D = driver();
   const int threads = 32 * sh.G * sh.teams_per_cta;
   const size_t dyn = sh.lay.bytes * sh.teams_per_cta;
@@ -817,8 +890,9 @@ cudaError_t launch_period_jit(const JitKernel &K, const LaunchShape &sh, const D
   if (!raise_jit_dyn_smem(f, dyn)) return cudaErrorInvalidValue;
   SliceLayout lay = sh.lay;
   int G = sh.G;
-  void *args[] = {&probs, &unit_start, &nprob, &total, &counter, &lay, &G, &cols_scratch,
-                  &rows_scratch, &cols_words};
+  Scratch s = sc;
+  void *args[] = {&probs, &unit_start, &nprob, &total, &counter, &lay, &G, &s.cols, &s.rows,
+                  &s.cols_words, &s.counts, &s.counts_stride};
   const CUresult r = D.launch(f, (unsigned)sh.ctas, 1, 1, (unsigned)threads, 1, 1, (unsigned)dyn,
                               (CUstream)st, args, nullptr);
   if (r != CUDA_SUCCESS) return cudaErrorLaunchFailure;
@@ -828,8 +902,7 @@ cudaError_t launch_period_jit(const JitKernel &K, const LaunchShape &sh, const D
 
 cudaError_t launch_multi_jit(const JitKernel &K, const LaunchShape &sh, const DevProblem *nets,
                              const MultiDev &md, int M, unsigned long long *counter,
-                             uint32_t *cols_scratch, uint32_t *rows_scratch, size_t cols_words,
-                             cudaStream_t st) {
+                             const Scratch &sc, cudaStream_t st) {
   const Driver &D = driver();
   const int threads = 32 * sh.G * sh.teams_per_cta;
   const size_t dyn = sh.lay.bytes * md.D * sh.teams_per_cta;
@@ -839,7 +912,9 @@ cudaError_t launch_multi_jit(const JitKernel &K, const LaunchShape &sh, const De
   MultiDev mdv = md;
   SliceLayout lay = sh.lay;
   int G = sh.G, Mv = M;
-  void *args[] = {&nets, &mdv, &Mv, &counter, &lay, &G, &cols_scratch, &rows_scratch, &cols_words};
+  Scratch s = sc;
+  void *args[] = {&nets, &mdv, &Mv, &counter, &lay, &G, &s.cols, &s.rows, &s.cols_words,
+                  &s.counts, &s.counts_stride};
   const CUresult r = D.launch(f, (unsigned)sh.ctas, 1, 1, (unsigned)threads, 1, 1, (unsigned)dyn,
                               (CUstream)st, args, nullptr);
   if (r != CUDA_SUCCESS) return cudaErrorLaunchFailure;

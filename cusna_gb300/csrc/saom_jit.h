@@ -20,11 +20,11 @@ namespace cusna {
 
 // The effect plan the specialised code is generated from.
 struct JitPlan {
-  int pc_flags = 0;  // F_PC_* popcount needs
+  CounterSet cnt{};  // two-path counters
   int n = 0;         // actors when every problem of the launch has the same
-                     // number (compiled in with W: the popcount loops unroll
-                     // and the strides are constants), else 0
-  std::vector<int> kind, cfn, tid, ety, i0, i1, i2;
+                     // number (compiled in with W: the strides are constants),
+                     // else 0
+  std::vector<int> kind, cfn, tid, ety, i0, i1, i2;  // cfn packed (cfn_pack)
 };
 
 // Source text of the specialised effect evaluation (the key of the compiled
@@ -55,12 +55,10 @@ bool jit_get(const std::string &spec, JitKernel *out, bool now = false);
 int jit_blocks_per_sm(const JitKernel &K, int threads, size_t dyn_smem);
 cudaError_t launch_period_jit(const JitKernel &K, const LaunchShape &sh, const DevProblem *probs,
                               const long long *unit_start, int nprob, long long total,
-                              unsigned long long *counter, uint32_t *cols_scratch,
-                              uint32_t *rows_scratch, size_t cols_words, cudaStream_t st);
+                              unsigned long long *counter, const Scratch &sc, cudaStream_t st);
 cudaError_t launch_multi_jit(const JitKernel &K, const LaunchShape &sh, const DevProblem *nets,
                              const MultiDev &md, int M, unsigned long long *counter,
-                             uint32_t *cols_scratch, uint32_t *rows_scratch, size_t cols_words,
-                             cudaStream_t st);
+                             const Scratch &sc, cudaStream_t st);
 // NVRTC compile of spec without loading it (no device needed): 0 on success,
 // else the NVRTC log in *log.
 int jit_compile_only(const std::string &spec, std::string *log, double *seconds);

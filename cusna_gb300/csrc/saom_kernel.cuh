@@ -4,19 +4,20 @@
 // take chains from a global work counter, so a launch holds one team per
 // resident slot and runs until the queue is empty (a persistent kernel). Each
 // team owns a slice of dynamic shared memory: the chain's out-rows and in-rows
-// as word-major bitsets, degrees, behaviour values and per-alter scratch.
+// as word-major bitsets (or pointers to them in global scratch), degrees, behaviour values and per-alter scratch.
 //
 // A network ministep (src/libcusna_saom_cpu.cpp:229-287) is one pass over the
 // alters j, which the team's lanes split in strides of 32*G: change statistics
-// d_je from popcounts of the bitsets, the linear predictor f_j = sum_e theta_e
-// d_je in float32 with a rigorous error bound, the float32 Gumbel key
-// g_j = f_j - log(-log u_j) with its bound, and an online log-sum-exp of the
-// score sums. The keys decide the chosen alter when the best key's lower bound
-// beats every other key's upper bound; otherwise the exact float64 keys of the
-// alters still in range decide, ties to the smaller j, as the reference
-// chooses. u_j comes from the reference's Philox counters (msteps, chain, 1,
-// j), so the chosen alter, and therefore the whole trajectory, equals the CPU
-// engine's.
+// d_je from degrees and two-path counts (popcounts of the bitsets, or for larger
+// networks a row of count matrices that the chain keeps up to date), the linear
+// predictor f_j = sum_e theta_e d_je in 64-bit fixed point, the float32 Gumbel
+// key g_j = f_j - log(-log u_j) with its error bound, and the score sums of
+// exp(f_j) and exp(f_j) d_je, in fixed point as well. The keys decide the chosen
+// alter when the best key's lower bound beats every other key's upper bound;
+// otherwise the exact float64 keys of the alters still in range decide, ties to
+// the smaller j, as the reference chooses. u_j comes from the reference's Philox
+// counters (msteps, chain, 1, j), so the chosen alter, and therefore the whole
+// trajectory, equals the CPU engine's.
 #pragma once
 #include "saom_common.cuh"
 
@@ -33,21 +34,26 @@ struct Team {
 
 // Per-team shared-memory slice. Sizes depend on the launch's largest problem.
 struct Slice {
-  uint32_t *rowsT;   // W*n
-  uint32_t *colsT;   // W*n (shared or global scratch)
+  uint32_t *rows;    // W*n (shared or global scratch)
+  uint32_t *cols;    // W*n (shared or global scratch)
   short *indeg, *outdeg;  // n each (degrees < 2^15 as n <= 8192)
   int *z;
   float *gbuf;       // n   upper bounds of the float32 Gumbel keys
-  float *blk;        // ceil(n/32)*2*(k+1)  per 32-alter block: the score sums as
-                     //   double-float pairs (or k+1 doubles on the float64 path)
+  double *blk;       // ceil(n/32)*(k+1)  per 32-alter block: the score sums of the
+                     //   float64 path; the same bytes hold the ring (ScoreRing)
   uint32_t *okbits;  // W
-  int *tp;           // n   (transTies / gwdsp)
+  int *tp;           // n   (gwdspFF)
   int *tq;           // n   (gwdspFB)
   uint32_t *tpeq;    // 2W  (transTies masks tp==0, tp==1)
+  uint16_t *cm;      // the counters held as matrices, cm_size(n) each (global scratch)
   double *crate;     // n   (non-basic rates)
-  double *red;       // 32*G + 32 reduction scratch
+  double *red;       // 32*G + 64 reduction scratch
+  int *redh;         // 32*G  high parts of the warps' score sums
+  int *rfm;          // G    the warps' largest predictors
   double *th;        // k  parameters of the current chain
-  float *th32;       // k  the same parameters (they are float32 inputs)
+  uint64_t *thq;     // k  the same in fixed point (theta_fx)
+  int *esd, *ecls;   // k  scale of a real statistic, class (FX_*) of an effect
+  int64_t *fx;       // 2  constant part of the predictor; chain in range (0/1)
   double *sc;        // k  scores
   double *dstar;     // k  change statistics of the chosen alter
   double *thb, *bsc; // kb
@@ -60,19 +66,24 @@ struct Slice {
   uint32_t *rr3;     //   behaviour uniform
   int *ekind, *ecfn, *eoffd, *eofft;  // k  effect plan
   double *stepd, *stept;  // 4k  per-ministep K_STEP magnitudes and terms
-  float *stepd32, *stept32;  // 4k  their float32 roundings
-  float *stepdlo32, *steptlo32;  // 4k  and the remainders (double-float pairs)
-  float2 *etab;      // 64   2^(j/64) as double-float pairs (the score exponential)
+  uint64_t *stepq;   // 4k  their magnitudes in fixed point
+  const int2 *etab;  // exp_fx's table (the CTA's)
 };
 
 struct SliceLayout {
   size_t bytes;  // per team
   size_t o_rows, o_cols, o_indeg, o_outdeg, o_z, o_g, o_blk, o_ok, o_tp, o_tq, o_tpeq, o_crate, o_red, o_th, o_sc, o_dstar, o_thb, o_bsc, o_rsc, o_p1, o_p2, o_tid,
       o_ety, o_dyn, o_i0, o_i1, o_i2, o_bty, o_rkind, o_misc, o_rtau, o_rnet, o_rfocal, o_rr3, o_ekind, o_ecfn, o_eoffd, o_eofft,
-      o_stepd, o_stept, o_th32, o_stepd32, o_stept32, o_stepdlo32, o_steptlo32, o_etab;
+      o_stepd, o_stept, o_stepq, o_thq, o_esd, o_ecls, o_fx, o_redh, o_rfm;
 };
 
 __host__ __device__ inline size_t al16(size_t x) { return (x + 15) & ~(size_t)15; }
+
+// Ministeps whose score sums wait for one flush (scores_flush).
+constexpr int kRing = 8;
+__host__ __device__ inline size_t ring_bytes(int k) {
+  return (size_t)kRing * ((k + 2) * 12 + k * 8 + 4);
+}
 
 // Layout of one team slice for maxima (n, k, ...) over the launch.
 __host__ __device__ inline SliceLayout make_layout(int n, int W, int k, int kb, int nrate, int G,
@@ -87,13 +98,15 @@ __host__ __device__ inline SliceLayout make_layout(int n, int W, int k, int kb, 
   put(s.o_outdeg, (size_t)n * 2);
   put(s.o_z, (size_t)n * 4);
   put(s.o_g, (size_t)n * 4);
-  put(s.o_blk, (size_t)((n + 31) / 32) * 2 * (k + 1) * 4);
+  // the score sums of the float64 path, or the ring of the fixed-point one
+  const size_t blk = (size_t)((n + 31) / 32) * (k + 1) * 8, ring = ring_bytes(k);
+  put(s.o_blk, blk > ring ? blk : ring);
   put(s.o_ok, (size_t)W * 4);
-  put(s.o_tp, need_tp || need_gw ? (size_t)n * 4 : 0);
+  put(s.o_tp, need_gw ? (size_t)n * 4 : 0);
   put(s.o_tq, need_tq ? (size_t)n * 4 : 0);
   put(s.o_tpeq, need_tp ? (size_t)W * 8 : 0);
   put(s.o_crate, nrate > 0 ? (size_t)n * 8 : 0);
-  put(s.o_red, (size_t)32 * G * 8 + 32 * 8);   // 32 slots per warp, then 32 team values
+  put(s.o_red, (size_t)32 * G * 8 + 64 * 8);   // 32 slots per warp, 32 results, 32 scratch
   put(s.o_th, (size_t)k * 8);
   put(s.o_sc, (size_t)k * 8);
   put(s.o_dstar, (size_t)k * 8);
@@ -121,30 +134,34 @@ __host__ __device__ inline SliceLayout make_layout(int n, int W, int k, int kb, 
   put(s.o_eofft, (size_t)k * 4);
   put(s.o_stepd, (size_t)k * 4 * 8);
   put(s.o_stept, (size_t)k * 4 * 8);
-  put(s.o_th32, (size_t)k * 4);
-  put(s.o_stepd32, (size_t)k * 4 * 4);
-  put(s.o_stept32, (size_t)k * 4 * 4);
-  put(s.o_stepdlo32, (size_t)k * 4 * 4);
-  put(s.o_steptlo32, (size_t)k * 4 * 4);
-  put(s.o_etab, (size_t)64 * 8);
+  put(s.o_stepq, (size_t)k * 4 * 8);
+  put(s.o_thq, (size_t)k * 8);
+  put(s.o_esd, (size_t)k * 4);
+  put(s.o_ecls, (size_t)k * 4);
+  put(s.o_fx, 16);
+  put(s.o_redh, (size_t)32 * G * 4);
+  put(s.o_rfm, (size_t)G * 4);
   s.bytes = al16(o);
   return s;
 }
 
+// A null rows or in-rows pointer: that part of the chain's state is in the slice.
 __device__ __forceinline__ Slice carve(unsigned char *base, const SliceLayout &L,
-                                       uint32_t *cols_global, uint32_t *rows_global) {
+                                       uint32_t *cols_global, uint32_t *rows_global,
+                                       uint16_t *counts_global, const int2 *etab) {
   Slice s;
-  s.rowsT = rows_global ? rows_global : (uint32_t *)(base + L.o_rows);
-  s.colsT = cols_global ? cols_global : (uint32_t *)(base + L.o_cols);
+  s.rows = rows_global ? rows_global : (uint32_t *)(base + L.o_rows);
+  s.cols = cols_global ? cols_global : (uint32_t *)(base + L.o_cols);
   s.indeg = (short *)(base + L.o_indeg);
   s.outdeg = (short *)(base + L.o_outdeg);
   s.z = (int *)(base + L.o_z);
   s.gbuf = (float *)(base + L.o_g);
-  s.blk = (float *)(base + L.o_blk);
+  s.blk = (double *)(base + L.o_blk);
   s.okbits = (uint32_t *)(base + L.o_ok);
   s.tp = (int *)(base + L.o_tp);
   s.tq = (int *)(base + L.o_tq);
   s.tpeq = (uint32_t *)(base + L.o_tpeq);
+  s.cm = counts_global;
   s.crate = (double *)(base + L.o_crate);
   s.red = (double *)(base + L.o_red);
   s.th = (double *)(base + L.o_th);
@@ -174,12 +191,14 @@ __device__ __forceinline__ Slice carve(unsigned char *base, const SliceLayout &L
   s.eofft = (int *)(base + L.o_eofft);
   s.stepd = (double *)(base + L.o_stepd);
   s.stept = (double *)(base + L.o_stept);
-  s.th32 = (float *)(base + L.o_th32);
-  s.stepd32 = (float *)(base + L.o_stepd32);
-  s.stept32 = (float *)(base + L.o_stept32);
-  s.stepdlo32 = (float *)(base + L.o_stepdlo32);
-  s.steptlo32 = (float *)(base + L.o_steptlo32);
-  s.etab = (float2 *)(base + L.o_etab);
+  s.stepq = (uint64_t *)(base + L.o_stepq);
+  s.thq = (uint64_t *)(base + L.o_thq);
+  s.esd = (int *)(base + L.o_esd);
+  s.ecls = (int *)(base + L.o_ecls);
+  s.fx = (int64_t *)(base + L.o_fx);
+  s.redh = (int *)(base + L.o_redh);
+  s.rfm = (int *)(base + L.o_rfm);
+  s.etab = etab;
   return s;
 }
 
@@ -192,11 +211,8 @@ __device__ __forceinline__ int bit_of(const uint32_t *T, int n, int row, int col
 // exchanges half of the remaining values with the lane 16>>s away, so a lane
 // does V-1 + (5 - log2 V) additions instead of 5V. Afterwards the lane holds the
 // warp total of quantity q(lane) in v[0]; lanes with bit 0 clear report it.
-__device__ __forceinline__ double radd(double a, double b) { return __dadd_rn(a, b); }
-__device__ __forceinline__ float radd(float a, float b) { return __fadd_rn(a, b); }
-
-template <int V, class R>
-__device__ __forceinline__ int warp_multi_sum(R (&v)[V], int lane) {
+template <int V>
+__device__ __forceinline__ int warp_multi_sum(double (&v)[V], int lane) {
   int q = 0;
   int cnt = V;
 #pragma unroll
@@ -206,10 +222,10 @@ __device__ __forceinline__ int warp_multi_sum(R (&v)[V], int lane) {
     const bool up = (lane & o) != 0;
 #pragma unroll
     for (int x = 0; x < half; ++x) {
-      const R send = up ? v[x] : v[x + half];
-      const R keep = up ? v[x + half] : v[x];
-      const R got = __shfl_xor_sync(kFull, send, o);
-      v[x] = radd(keep, got);
+      const double send = up ? v[x] : v[x + half];
+      const double keep = up ? v[x + half] : v[x];
+      const double got = __shfl_xor_sync(kFull, send, o);
+      v[x] = __dadd_rn(keep, got);
     }
     if (up) q += half;
     cnt = half;
@@ -219,76 +235,9 @@ __device__ __forceinline__ int warp_multi_sum(R (&v)[V], int lane) {
 #pragma unroll
   for (int s = 0; s < 5; ++s) {
     const int o = 16 >> s;
-    if ((1 << s) >= V) v[0] = radd(v[0], __shfl_xor_sync(kFull, v[0], o));
+    if ((1 << s) >= V) v[0] = __dadd_rn(v[0], __shfl_xor_sync(kFull, v[0], o));
   }
   return q;
-}
-
-// Recursive halving over V double-float pairs (h[q], l[q]), any V <= 32: at
-// stage s (partner lane^(16>>s)) a lane holding c values keeps the lower
-// m = ceil(c/2) (bit clear) or the upper c - m, shifted down (bit set; an odd
-// c pads the upper half with a zero), and adds its partner's copies, so every
-// stage takes ceil(c/2) additions and V values need about V + 3 in all.
-// Afterwards the lane's h[0], l[0] is the warp total of quantity q (returned)
-// when *real is set; each quantity has exactly one such lane. ff_add is
-// symmetric in its operands (TwoSum's error term is exact).
-template <int V>
-__device__ __forceinline__ int warp_multi_sum_ff(float (&h)[V], float (&l)[V], int lane,
-                                                 bool *real) {
-  int q = 0, r = V;  // r: how many of the lane's values are real
-  int c = V;
-#pragma unroll
-  for (int s = 0; s < 5; ++s) {
-    const int o = 16 >> s;
-    const int m = (c + 1) >> 1;
-    const bool up = (lane & o) != 0;
-#pragma unroll
-    for (int x = 0; x < m; ++x) {
-      const bool pair = m + x < c;
-      const float vh = pair ? h[pair ? m + x : 0] : 0.f, vl = pair ? l[pair ? m + x : 0] : 0.f;
-      const float sh = up ? h[x] : vh, sl = up ? l[x] : vl;
-      float kh = up ? vh : h[x], kl = up ? vl : l[x];
-      const float gh = __shfl_xor_sync(kFull, sh, o), gl = __shfl_xor_sync(kFull, sl, o);
-      ff_add(kh, kl, gh, gl);
-      h[x] = kh;
-      l[x] = kl;
-    }
-    if (up) {
-      q += m;
-      r = r > m ? r - m : 0;
-    } else {
-      r = r < m ? r : m;
-    }
-    c = m;
-  }
-  *real = r > 0;
-  return q;
-}
-
-// Sum of K double-float pairs (h[e], l[e]) in a fixed pairwise tree, two
-// additions per packed instruction: h[x] += h[x + m] for the upper half at
-// each level (an odd count leaves its middle element for the next level).
-template <int K>
-__device__ __forceinline__ float2 ff_tree_sum(float (&h)[K], float (&l)[K]) {
-  int c = K;
-#pragma unroll
-  for (int s = 0; s < 5; ++s) {
-    if (c > 1) {
-      const int m = (c + 1) >> 1, na = c - m;
-#pragma unroll
-      for (int x = 0; x + 1 < na; x += 2) {
-        float2 ah = make_float2(h[x], h[x + 1]), al = make_float2(l[x], l[x + 1]);
-        ff_add2(ah, al, make_float2(h[x + m], h[x + 1 + m]), make_float2(l[x + m], l[x + 1 + m]));
-        h[x] = ah.x;
-        h[x + 1] = ah.y;
-        l[x] = al.x;
-        l[x + 1] = al.y;
-      }
-      if (na & 1) ff_add(h[na - 1], l[na - 1], h[na - 1 + m], l[na - 1 + m]);
-      c = m;
-    }
-  }
-  return make_float2(h[0], l[0]);
 }
 
 __device__ __forceinline__ long long warp_max_ll(long long x) {
@@ -297,12 +246,6 @@ __device__ __forceinline__ long long warp_max_ll(long long x) {
     long long y = __shfl_xor_sync(kFull, x, o);
     x = y > x ? y : x;
   }
-  return x;
-}
-
-__device__ __forceinline__ float warp_max_f(float x) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) x = fmaxf(x, __shfl_xor_sync(kFull, x, o));
   return x;
 }
 
@@ -322,18 +265,6 @@ __device__ __forceinline__ long long team_max_ll(const Team &T, long long x, dou
   T.sync();
   long long m = r[0];
   for (int w = 1; w < T.G; ++w) m = r[w] > m ? r[w] : m;
-  return m;
-}
-
-__device__ __forceinline__ float team_max_f(const Team &T, float x, double *red) {
-  x = warp_max_f(x);
-  if (T.G == 1) return x;
-  float *r = (float *)red;
-  T.sync();
-  if (T.lane == 0) r[T.warp] = x;
-  T.sync();
-  float m = r[0];
-  for (int w = 1; w < T.G; ++w) m = fmaxf(m, r[w]);
   return m;
 }
 
@@ -371,13 +302,25 @@ __device__ __forceinline__ int team_argmax(const Team &T, long long key, int j, 
 }
 
 // ------------------------------------------------------- change statistics
+// Multi-network teams: network w's rows are rows + w*row_stride words, its
+// in-rows cols + w*col_stride words, its count matrices cm + w*cm_stride.
+struct NetBase {
+  const uint32_t *rows, *cols;
+  uint16_t *cm;
+  size_t row_stride, col_stride, cm_stride;
+  // the networks' slices' misc words (largest degrees), misc_stride apart
+  const int *misc;
+  size_t misc_stride;
+  int D;
+};
+
 // Per-ministep context shared by all alters (uniform over the team).
 struct StepCtx {
   int i, od_i, id_i, rdeg_i;
   double zvi;
-  // multi-network teams: network w's rows are rows0 + w*net_stride words
-  const uint32_t *rows0;
-  size_t net_stride;
+  int64_t f0;   // part of the fixed-point predictor that no alter changes
+  const uint64_t *tabq;
+  NetBase net;
 };
 
 // Popcount of (A_word(a) & B_word(b)) summed over the W words.
@@ -385,6 +328,118 @@ __device__ __forceinline__ int pc2(const uint32_t *A, int a, const uint32_t *B, 
   int c = 0;
   for (int w = 0; w < W; ++w) c += __popc(A[w * n + a] & B[w * n + b]);
   return c;
+}
+
+// ------------------------------------------------------- two-path counters
+// Position of counter c among the counters held as matrices.
+__device__ __forceinline__ int cm_rank(unsigned mask, int c) {
+  return __popc(mask & ((1u << c) - 1u));
+}
+
+// Row words of a relation's transpose (for alter j, the h with the relation).
+__device__ __forceinline__ const uint32_t *rel_rows(const Slice &S, const NetBase &N, int m) {
+  return m == CM_ROWS ? S.cols
+                      : (m == CM_COLS ? S.rows : N.rows + (size_t)(m - CM_NCOLS) * N.row_stride);
+}
+
+// Where focal actor i's counts of one counter come from: row i of its matrix (cm),
+// or popcounts of the set A (and B, bs words apart) with the alters' rows in M1
+// (and M2). Resolved once for a loop over the alters.
+struct CountRow {
+  const uint16_t *cm;
+  const uint32_t *A, *B, *M1, *M2;
+  int bs;
+};
+__device__ __forceinline__ CountRow count_row(const DevProblem &P, const Slice &S,
+                                              const StepCtx &X, int n, int W, int c) {
+  CountRow R{nullptr, S.rows + X.i, nullptr, nullptr, nullptr, n};
+  const unsigned mask = P.cnt.mask;
+  if ((mask >> c) & 1u) {
+    R.cm = S.cm + cm_rank(mask, c) * cm_size(n) + (size_t)X.i * n;
+    return R;
+  }
+  const int list = P.cnt.list[c], m1 = P.cnt.m1[c], m2 = P.cnt.m2[c];
+  if (list == CL_IN) R.A = S.cols + X.i;
+  else if (list == CL_MUTUAL) R.B = S.cols + X.i;
+  else if (list == CL_TP0 || list == CL_TP1) {   // the transTies masks are W words
+    R.B = S.tpeq + (list == CL_TP1 ? W : 0);
+    R.bs = 1;
+  } else if (list >= CL_NET) R.A = X.net.rows + (size_t)(list - CL_NET) * X.net.row_stride + X.i;
+  R.M1 = rel_rows(S, X.net, m1);
+  if (m2 != CM_NONE) R.M2 = rel_rows(S, X.net, m2);
+  return R;
+}
+// Alter j's count.
+__device__ __forceinline__ int count_of(const CountRow &R, int n, int W, int j) {
+  if (R.cm) return R.cm[j];
+  int c = 0;
+  if (!R.B && !R.M2) {
+#pragma unroll 4
+    for (int w = 0; w < W; ++w) c += __popc(R.A[w * n] & R.M1[w * n + j]);
+    return c;
+  }
+  for (int w = 0; w < W; ++w) {
+    uint32_t a = R.A[w * n];
+    if (R.B) a &= R.B[w * R.bs];
+    c += __popc(a & R.M1[w * n + j]);
+    if (R.M2) c += __popc(a & R.M2[w * n + j]);
+  }
+  return c;
+}
+__device__ __forceinline__ int count_at(const DevProblem &P, const Slice &S, const StepCtx &X,
+                                        int c, int j) {
+  return count_of(count_row(P, S, X, P.n, P.W, c), P.n, P.W, j);
+}
+
+// transTies: masks {h : tp_h == 0} and {h : tp_h == 1} of the two-path counts
+// tp_h = |out_i & in_h| (counter c), word-parallel via ballots.
+__device__ __forceinline__ void tp_masks(const Team &T, const DevProblem &P, const Slice &S,
+                                         const StepCtx &X, int n, int W, int c) {
+  const CountRow R = count_row(P, S, X, n, W, c);
+  for (int hb = 32 * T.warp; hb < W * 32; hb += T.L) {
+    const int h = hb + T.lane;
+    const int v = h < n ? count_of(R, n, W, h) : -1;
+    const uint32_t z0 = __ballot_sync(kFull, v == 0), z1 = __ballot_sync(kFull, v == 1);
+    if (T.lane == 0) { S.tpeq[hb >> 5] = z0; S.tpeq[W + (hb >> 5)] = z1; }
+  }
+}
+
+// Updates the team's count matrices for the toggle u -> v (dl = +-1) in network
+// net of problem P, and for v -> u in a symmetric one: the tasks of P.cnt
+// (saom_launch.h, counter_tasks), each one word of its set per lane, as many
+// tasks at once as the lanes hold. The sets are read while the tie toggles: they
+// hold it at most at the diagonal cell, which is left out (and never read), so
+// this needs no order with the toggle. Two 16-bit counts share a word; the
+// reductions need no answer, so the warp does not wait for memory, and no count
+// leaves 0..2n, so no half borrows from or carries into the other.
+static __device__ __noinline__ void counts_toggle(const Team &T, const DevProblem &P,
+                                                  const NetBase &N, int u, int v, int dl) {
+  const int n = P.n, W = P.W;
+  const int lg = W > 16 ? 5 : 32 - __clz(W - 1);   // lanes per task: 2^lg
+  const int per = 32 >> lg;                        // tasks per warp at a time
+  for (int s = 0; s <= (P.symflag ? 1 : 0); ++s) {
+    for (int t = T.warp * per + (T.lane >> lg); t < P.cnt.ntask; t += T.G * per) {
+      const unsigned k = P.cnt.task[t];
+      const int a = (k & 2) ? v : u, fix = (k & 4) ? v : u;
+      const size_t sn = (k >> 8) & 15;
+      const uint32_t *set = ((k & 1) ? N.cols + sn * N.col_stride : N.rows + sn * N.row_stride) +
+                            a;
+      uint16_t *M = N.cm + (size_t)(k >> 12) * N.cm_stride + ((k >> 4) & 15) * cm_size(n);
+      const size_t base = (k & 8) ? fix : (size_t)fix * n, stride = (k & 8) ? n : 1;
+      for (int w = T.lane & ((1 << lg) - 1); w < W; w += 32) {
+        uint32_t m = set[w * n];
+        if (w == (fix >> 5)) m &= ~(1u << (fix & 31));
+        while (m) {
+          const size_t cell = base + stride * ((w << 5) + __ffs(m) - 1);
+          m &= m - 1;
+          atomicAdd(reinterpret_cast<unsigned *>(M) + (cell >> 1), (unsigned)dl << (16 * (cell & 1)));
+        }
+      }
+    }
+    const int x = u;
+    u = v;
+    v = x;
+  }
 }
 
 // Exact (double)c for 0 <= c < 2^31 built on the integer pipes.
@@ -399,12 +454,22 @@ __device__ __forceinline__ double flip(double x, unsigned long long sgn) {
   return __longlong_as_double(__double_as_longlong(x) ^ (long long)sgn);
 }
 
+// 2^e as a double, -1022 <= e <= 1023.
+__device__ __forceinline__ double pow2(int e) {
+  return __longlong_as_double((long long)(1023 + e) << 52);
+}
+// A real magnitude in fixed point: d 2^sd + 2^62.
+__device__ __forceinline__ uint64_t real_fx(double d, int sd) {
+  return (uint64_t)(__double2ll_rn(__dmul_rn(d, pow2(sd))) + (1LL << 62));
+}
+
 // Generic change statistic of one effect (src/libcusna_saom_cpu.cpp:49-101 and
 // :246-251): the reference formula evaluated per alter. Used for the kinds no
-// table covers (gwdsp, interactions, dyadic covariates of very large n).
+// table covers (gwdsp, interactions, dyadic covariates of very large n); cnt is
+// the effect's two-path count of j (types 24, 26-28).
 static __device__ __noinline__ double gen_stat(const DevProblem &P, const Slice &S, const StepCtx &X,
-                                        int e, int j, int aij, int aji, int ri_cj, int ri_rj,
-                                        int rj_ci, int ci_cj, int ci_rj, const double *d) {
+                                        int e, int j, int aij, int aji, int cnt,
+                                        const double *d) {
   const int n = P.n, W = P.W, i = X.i, t = S.tid[e];
   const unsigned long long sg = aij ? 0x8000000000000000ull : 0ull;
   const double dl = aij ? -1.0 : 1.0;
@@ -424,10 +489,7 @@ static __device__ __noinline__ double gen_stat(const DevProblem &P, const Slice 
   switch (t) {
     case 7: return flip(sqrt(i2d(S.indeg[j] + 1 - aij)), sg);
     case 9: return flip(sqrt(i2d(S.outdeg[j])), sg);
-    case 24: return flip(P.wtab[(size_t)e * (n + 1) + ri_cj], sg);
-    case 26: return flip(P.wtab[(size_t)e * (n + 1) + ri_rj], sg);
-    case 27: return flip(P.wtab[(size_t)e * (n + 1) + ci_cj], sg);
-    case 28: return flip(P.wtab[(size_t)e * (n + 1) + ci_rj], sg);
+    case 24: case 26: case 27: case 28: return flip(P.wtab[(size_t)e * (n + 1) + cnt], sg);
     case 11: return flip(vj, sg);
     case 12: return flip(__dsub_rn(__dsub_rn(1.0, __dmul_rn(fabs(__dsub_rn(vi, vj)), S.p1[e])), S.p2[e]), sg);
     case 13: return flip(fabs(__dsub_rn(vi, vj)) < 1e-9 ? 1.0 : 0.0, sg);
@@ -443,7 +505,7 @@ static __device__ __noinline__ double gen_stat(const DevProblem &P, const Slice 
       // adds: the gw weight difference at p_h = |out_i & in_h| (29) or
       // |out_i & out_h| (30), both precomputed for this ministep
       const double *wr = P.wtab + (size_t)e * (n + 1);
-      const uint32_t *B = (t == 29) ? S.rowsT : S.colsT;
+      const uint32_t *B = (t == 29) ? S.rows : S.cols;
       const int *pc = (t == 29) ? S.tp : S.tq;
       double acc = 0.0;
       for (int w = 0; w < W; ++w) {
@@ -462,9 +524,30 @@ static __device__ __noinline__ double gen_stat(const DevProblem &P, const Slice 
   }
 }
 
+// gwdsp's magnitude at 2^sd + 2^62 (type 29, or 30) from the fixed-point weight
+// differences w[p + 1] - w[p]: whole-number sums over the set bits of alter j's
+// row. Float64 differences put two dependent FP64 additions on each set bit.
+__device__ __forceinline__ uint64_t gw_fixed(const Slice &S, const StepCtx &X, int n, int W, int e,
+                                             int t, int j, int aij) {
+  const uint64_t *dq = X.tabq + S.eoffd[e] - aij;   // a tie's alter is in every p_h
+  const uint32_t *B = (t == 29 ? S.rows : S.cols) + j;
+  const int *pc = t == 29 ? S.tp : S.tq;
+  uint64_t acc = 1ull << 62;
+  for (int w = 0; w < W; ++w) {
+    uint32_t m = B[w * n];
+    if ((X.i >> 5) == w) m &= ~(1u << (X.i & 31));
+    while (m) {
+      const int h = (w << 5) + __ffs(m) - 1;
+      m &= m - 1;
+      acc += dq[pc[h]];
+    }
+  }
+  return acc;
+}
+
 // Per-ministep magnitudes of the K_STEP effects (types 10, 14-19): for each
 // (a_ij, a_ji) the reference's d and theta * d, into stepd/stept[e*4 + q],
-// q = 2*a_ij + a_ji. Lanes take (e, q) pairs.
+// q = 2*a_ij + a_ji, and the magnitude in fixed point. Lanes take (e, q) pairs.
 __device__ __forceinline__ void step_values(const Team &T, const DevProblem &P, const Slice &S,
                                             const StepCtx &X) {
   for (int x = T.tl; x < 4 * P.k; x += T.L) {
@@ -494,26 +577,21 @@ __device__ __forceinline__ void step_values(const Team &T, const DevProblem &P, 
         break;
       default: v = 0.0; break;
     }
-    const double tv = __dmul_rn(S.th[e], v);
-    const float v32 = (float)v, t32 = (float)tv;
     S.stepd[x] = v;
-    S.stept[x] = tv;
-    S.stepd32[x] = v32;
-    S.stept32[x] = t32;
-    S.stepdlo32[x] = (float)__dsub_rn(v, (double)v32);
-    S.steptlo32[x] = (float)__dsub_rn(tv, (double)t32);
+    S.stept[x] = __dmul_rn(S.th[e], v);
+    S.stepq[x] = real_fx(flip(v, sg), S.esd[e]);
   }
 }
 
 // Change statistics of toggling i -> j for all k effects into d[0..k-1]
 // (src/libcusna_saom_cpu.cpp:49-101 per effect type, :243-261 for the loop with
 // interactions and creation/endowment zeroing), and with TERMS the linear
-// predictor f = sum_e theta_e d_e in the reference's e-order. Popcounts of the
-// word-major bitsets replace the reference's O(n) dense loops; they count the
-// same sets:
-//   |out_i & in_j| = #{h: a_ih a_hj}      |out_i & out_j| = #{h: a_ih a_jh}
-//   |out_j & in_i| = #{h: a_jh a_hi}      |in_i & in_j|   = #{h: a_hi a_hj}
-//   |in_i & out_j| = #{h: a_hi a_jh}
+// predictor f = sum_e theta_e d_e in the reference's e-order. The two-path
+// counters replace the reference's O(n) dense loops; they count the same sets:
+//   |out_i & in_j| = #{h: a_ih a_hj}: set out_i, ties h -> j
+//   |out_i & out_j| = #{h: a_ih a_jh}: set out_i, ties j -> h
+//   |out_j & in_i| = #{h: a_jh a_hi}: set in_i, ties j -> h
+//   |in_i & in_j| = #{h: a_hi a_hj}: set in_i, ties h -> j
 // Every d and every term equals the reference's float64 value: delta * x is a
 // sign flip, table entries are the reference's expressions evaluated once, and
 // f adds the terms in e-order (terms of zeroed effects are +-0 and change
@@ -521,25 +599,15 @@ __device__ __forceinline__ void step_values(const Team &T, const DevProblem &P, 
 // Cross-network change statistic magnitude (before the sign of the toggle) of
 // toggling i -> j in the own network for cross effect type t, reading network
 // w's current rows (src/libcusna_saom_cpu.cpp:431-444): 33 a_w[i][j], 34
-// a_w[j][i], 35 both, 36 |out_w(i) & out_w(j)|, 37 |out_w(i) & in_own(j)|.
-__device__ __forceinline__ int cross_count(const Slice &S, const StepCtx &X, int n, int W, int t,
-                                           int w, int i, int j) {
-  const uint32_t *Rw = X.rows0 + (size_t)w * X.net_stride;
-  switch (t) {
-    case 33: return bit_of(Rw, n, i, j);
-    case 34: return bit_of(Rw, n, j, i);
-    case 35: return bit_of(Rw, n, i, j) & bit_of(Rw, n, j, i);
-    case 36: {
-      int c = 0;
-      for (int x = 0; x < W; ++x) c += __popc(Rw[x * n + i] & Rw[x * n + j]);
-      return c;
-    }
-    default: {  // 37
-      int c = 0;
-      for (int x = 0; x < W; ++x) c += __popc(Rw[x * n + i] & S.colsT[x * n + j]);
-      return c;
-    }
-  }
+// a_w[j][i], 35 both, 36 |out_w(i) & out_w(j)| and 37 |out_w(i) & in_own(j)|
+// (counter c).
+__device__ __forceinline__ int cross_count(const DevProblem &P, const Slice &S, const StepCtx &X,
+                                           int n, int t, int w, int c, int i, int j) {
+  if (t >= 36) return count_at(P, S, X, c, j);
+  int v = 1;
+  if (t != 34) v = bit_of(X.net.rows + (size_t)w * X.net.row_stride, n, i, j);
+  if (t != 33) v &= bit_of(X.net.cols + (size_t)w * X.net.col_stride, n, i, j);
+  return v;
 }
 
 // MULTI: the kernel serves multi-network problems (cross effects K_CROSS);
@@ -548,28 +616,16 @@ template <bool TERMS, bool MULTI>
 __device__ __forceinline__ double change_stats(const DevProblem &P, const Slice &S,
                                                const StepCtx &X, int j, int aij, int aji,
                                                double *d) {
-  const int n = P.n, W = P.W, k = P.k, i = X.i;
+  const int n = P.n, k = P.k, i = X.i;
   const unsigned long long sg = aij ? 0x8000000000000000ull : 0ull;
-  const int fl = P.flags;
-  int ri_cj = 0, ri_rj = 0, rj_ci = 0, ci_cj = 0, ci_rj = 0, ricirj = 0;
-  if (fl & (F_PC_RI_CJ | F_PC_RI_RJ | F_PC_RJ_CI | F_PC_CI_CJ | F_PC_CI_RJ | F_PC_RICIRJ)) {
-    const uint32_t *R = S.rowsT, *Cc = S.colsT;
-    for (int w = 0; w < W; ++w) {
-      const uint32_t ri = R[w * n + i], rj = R[w * n + j];
-      const uint32_t ci = Cc[w * n + i], cj = Cc[w * n + j];
-      if (fl & F_PC_RI_CJ) ri_cj += __popc(ri & cj);
-      if (fl & F_PC_RI_RJ) ri_rj += __popc(ri & rj);
-      if (fl & F_PC_RJ_CI) rj_ci += __popc(rj & ci);
-      if (fl & F_PC_CI_CJ) ci_cj += __popc(ci & cj);
-      if (fl & F_PC_CI_RJ) ci_rj += __popc(ci & rj);
-      if (fl & F_PC_RICIRJ) ricirj += __popc(ri & ci & rj);
-    }
-  }
-  const bool ttab = (fl & F_THETA_TAB) != 0;
+  const bool ttab = (P.flags & F_THETA_TAB) != 0;
   double f = 0.0;
 #pragma unroll 1
   for (int e = 0; e < k; ++e) {
-    const int kind = S.ekind[e], cfn = S.ecfn[e];
+    const int kind = S.ekind[e], pk = S.ecfn[e], cfn = pk & 0xFF;
+    const int ca = (pk >> 8) & 0xFF, cb = (pk >> 16) & 0xFF, cc = (pk >> 24) & 0xFF;
+    auto cnt = [&](int c) { return count_at(P, S, X, c, j); };
+    (void)cb; (void)cc;
     double v, term = 0.0;
     bool has_term = TERMS;
     if (kind == K_CNT) {
@@ -577,18 +633,10 @@ __device__ __forceinline__ double change_stats(const DevProblem &P, const Slice 
       switch (cfn) {
         case 0: c = 1; break;
         case 1: c = aji; break;
-        case 2: c = ri_cj + ri_rj; break;
-        case 3: c = rj_ci; break;
+        case 2: case 3: c = cnt(ca); break;
         case 4: c = S.indeg[j] + 1 - aij; break;
-        case 5: {
-          c = 0;
-          const uint32_t *eq = S.tpeq + (aij ? W : 0);
-          for (int w = 0; w < W; ++w)
-            c += __popc(S.rowsT[w * n + i] & S.rowsT[w * n + j] & eq[w]);
-          if (S.tp[j] > 0) ++c;
-          break;
-        }
-        case 6: c = (aji ? ri_cj : 0) + ricirj; break;
+        case 5: c = cnt(aij ? cb : ca) + (cnt(cc) > 0 ? 1 : 0); break;
+        case 6: c = (aji ? cnt(ca) : 0) + cnt(cb); break;
         default: c = S.outdeg[j]; break;  // 7
       }
       v = flip(i2d(c), sg);
@@ -598,10 +646,7 @@ __device__ __forceinline__ double change_stats(const DevProblem &P, const Slice 
       switch (cfn) {
         case 4: idx = S.indeg[j] + 1 - aij; break;
         case 7: idx = S.outdeg[j]; break;
-        case 8: idx = ri_cj; break;
-        case 9: idx = ri_rj; break;
-        case 10: idx = ci_cj; break;
-        case 11: idx = ci_rj; break;
+        case 8: idx = cnt(ca); break;
         case 12: idx = j; break;
         case 13: idx = S.z[j] - P.zlo; break;
         case 14: idx = i * n + j; break;
@@ -617,11 +662,11 @@ __device__ __forceinline__ double change_stats(const DevProblem &P, const Slice 
       v = 0.0;
       has_term = false;
     } else if (MULTI && kind == K_CROSS) {
-      const int c = cross_count(S, X, n, W, cfn, S.eoffd[e], i, j);
+      const int c = cross_count(P, S, X, n, cfn, S.eoffd[e], ca, i, j);
       v = flip((cfn == 36 && S.p1[e] >= 2.0) ? sqrt(i2d(c)) : i2d(c), sg);
       if (TERMS) term = __dmul_rn(S.th[e], v);
     } else {
-      v = gen_stat(P, S, X, e, j, aij, aji, ri_cj, ri_rj, rj_ci, ci_cj, ci_rj, d);
+      v = gen_stat(P, S, X, e, j, aij, aji, ca != 0xFF ? cnt(ca) : 0, d);
       if (TERMS) term = __dmul_rn(S.th[e], v);
     }
     if ((S.ety[e] == 1 && aij) || (S.ety[e] == 2 && !aij)) {
@@ -634,150 +679,116 @@ __device__ __forceinline__ double change_stats(const DevProblem &P, const Slice 
   return f;
 }
 
-// float32 image of change_stats<true> for the shortlist pass: d32[e] is the
-// float32 rounding of the change statistic d_e (exact for the integer counts;
-// an interaction is the float32 product of its components), and the return
-// value is f32 = sum_e fl32(theta_e * d32[e]), added in the reference's e-order
-// in float32; *absf = sum_e |fl32(theta_e * d32[e])|. With u = 2^-24 each term
-// differs from theta_e d_e by at most 7u|term| (at most five roundings in an
-// interaction product, one in the product with theta) and the k additions add
-// at most (k-1)u absf, so |f32 - f| <= (k + 8) u absf for the float64 predictor
-// f of change_stats<true> (itself within 2^-50 absf of the exact sum).
-//
-// The same pass carries the double-float images the score sums use:
-// d32lo[e] with d32[e] + d32lo[e] = d_e to about 2^-48 (0 for the integer
-// counts), and the predictor as a double-float pair *fx, within about
-// 2^-47 absf of f: each term's remainder (an exact Dekker product for integer
-// counts; theta times the table's float32 remainder for looked-up values)
-// plus the exact TwoSum error of each float32 addition (fx->x = f32 here; the
-// specialised build adds the term pairs in a packed tree instead).
+// ---- the fixed-point pass -----------------------------------------------------
+// How an effect enters the pass (Slice::ecls; bit 8: theta < 0):
+enum : int {
+  FX_ZERO = 0,   // d = 0
+  FX_DELTA = 1,  // d = delta (density): part of f0, its score sum is that of delta w
+  FX_UNI = 2,    // magnitude the same for every alter (egoX, in-degree effects): as above
+  FX_CNT = 3,    // integer magnitude
+  FX_REAL = 4,   // real magnitude
+};
+__host__ __device__ __forceinline__ int fx_class(int kind, int cfn, int tid, int ety) {
+  if (kind == K_ZERO) return FX_ZERO;
+  if (kind == K_CNT && cfn == 0 && ety == 0) return FX_DELTA;
+  if (kind == K_STEP && (tid == 10 || tid == 14 || tid == 15) && ety == 0) return FX_UNI;
+  return (kind == K_CNT || kind == K_CROSS) ? FX_CNT : FX_REAL;
+}
+// theta of a count at scale 2^-46 (a float32 of at least 2^-23 is exact), of a
+// real statistic |theta| 2^(110 - sd), so that mulhi_fx with a magnitude at 2^sd
+// has scale 2^-46.
+__device__ __forceinline__ uint64_t theta_fx(double th, int cls, int sd) {
+  if (cls == FX_UNI || cls == FX_REAL) return (uint64_t)__double2ull_rn(__dmul_rn(fabs(th), pow2(110 - sd)));
+  return (uint64_t)__double2ll_rn(__dmul_rn(th, pow2(kFBits)));
+}
+// theta times the real magnitude m = |d| 2^sd + 2^62, but for the 2^62's part,
+// which is -base_fx and enters the predictor's constant part where it can.
+__device__ __forceinline__ int64_t term_fx(uint64_t thr, int cls, uint64_t m) {
+  return signed_fx(mulhi_fx(thr, m), cls >> 8);
+}
+__device__ __forceinline__ int64_t base_fx(uint64_t thr, int cls) {
+  return signed_fx(thr >> 2, (cls >> 8) ^ 1);
+}
+
+// Magnitudes of toggling i -> j for the effects of classes FX_CNT (the count) and
+// FX_REAL (|d| 2^sd + 2^62) into v, 0 for an effect that its creation or
+// endowment type rules out, and the predictor without its sign (f_j = delta
+// times it) at scale 2^-46. The terms' errors are at most 3 2^-46 each (mulhi_fx
+// and the rounding of theta and d), 0 for counts.
 template <bool MULTI>
-__device__ __forceinline__ float change_stats32(const DevProblem &P, const Slice &S,
+__device__ __forceinline__ int64_t change_fixed(const DevProblem &P, const Slice &S,
                                                 const StepCtx &X, int j, int aij, int aji,
-                                                float *d32, float *d32lo, float *absf,
-                                                float2 *fx) {
-  const int n = P.n, W = P.W, k = P.k, i = X.i;
-  const int fl = P.flags;
-  int ri_cj = 0, ri_rj = 0, rj_ci = 0, ci_cj = 0, ci_rj = 0, ricirj = 0;
-  if (fl & (F_PC_RI_CJ | F_PC_RI_RJ | F_PC_RJ_CI | F_PC_CI_CJ | F_PC_CI_RJ | F_PC_RICIRJ)) {
-    const uint32_t *R = S.rowsT, *Cc = S.colsT;
-    for (int w = 0; w < W; ++w) {
-      const uint32_t ri = R[w * n + i], rj = R[w * n + j];
-      const uint32_t ci = Cc[w * n + i], cj = Cc[w * n + j];
-      if (fl & F_PC_RI_CJ) ri_cj += __popc(ri & cj);
-      if (fl & F_PC_RI_RJ) ri_rj += __popc(ri & rj);
-      if (fl & F_PC_RJ_CI) rj_ci += __popc(rj & ci);
-      if (fl & F_PC_CI_CJ) ci_cj += __popc(ci & cj);
-      if (fl & F_PC_CI_RJ) ci_rj += __popc(ci & rj);
-      if (fl & F_PC_RICIRJ) ricirj += __popc(ri & ci & rj);
-    }
-  }
-  const uint32_t sg = aij ? 0x80000000u : 0u;
-  float f = 0.f, a = 0.f, fo = 0.f;
+                                                uint64_t *v) {
+  const int n = P.n, k = P.k, i = X.i;
+  int64_t f = X.f0;
 #pragma unroll 1
   for (int e = 0; e < k; ++e) {
-    const int kind = S.ekind[e], cfn = S.ecfn[e];
-    const float th = S.th32[e];
-    float v, vlo = 0.f, term = 0.f, tlo = 0.f;
-    bool has_term = true;
-    if (kind == K_CNT) {
+    const int cls = S.ecls[e] & 0xFF;
+    if (cls < FX_CNT) continue;
+    const int kind = S.ekind[e], pk = S.ecfn[e], cfn = pk & 0xFF;
+    const int ca = (pk >> 8) & 0xFF, cb = (pk >> 16) & 0xFF, cc = (pk >> 24) & 0xFF;
+    auto cnt = [&](int c) { return count_at(P, S, X, c, j); };
+    const int ety = S.ety[e];
+    if ((ety == 1 && aij) || (ety == 2 && !aij)) {
+      v[e] = 0;
+      continue;
+    }
+    if (cls == FX_CNT) {
       int c;
-      switch (cfn) {
-        case 0: c = 1; break;
-        case 1: c = aji; break;
-        case 2: c = ri_cj + ri_rj; break;
-        case 3: c = rj_ci; break;
-        case 4: c = S.indeg[j] + 1 - aij; break;
-        case 5: {
-          c = 0;
-          const uint32_t *eq = S.tpeq + (aij ? W : 0);
-          for (int w = 0; w < W; ++w)
-            c += __popc(S.rowsT[w * n + i] & S.rowsT[w * n + j] & eq[w]);
-          if (S.tp[j] > 0) ++c;
-          break;
+      if (MULTI && kind == K_CROSS) {
+        c = cross_count(P, S, X, n, cfn, S.eoffd[e], ca, i, j);
+      } else {
+        switch (cfn) {
+          case 0: c = 1; break;
+          case 1: c = aji; break;
+          case 2: case 3: c = cnt(ca); break;
+          case 4: c = S.indeg[j] + 1 - aij; break;
+          case 5: c = cnt(aij ? cb : ca) + (cnt(cc) > 0 ? 1 : 0); break;
+          case 6: c = (aji ? cnt(ca) : 0) + cnt(cb); break;
+          default: c = S.outdeg[j]; break;  // 7
         }
-        case 6: c = (aji ? ri_cj : 0) + ricirj; break;
-        default: c = S.outdeg[j]; break;  // 7
       }
-      v = __uint_as_float(__float_as_uint((float)c) ^ sg);
-      term = __fmul_rn(th, v);
-      tlo = fmaf(th, v, -term);
-    } else if (kind == K_LOOK) {
+      v[e] = (uint64_t)c;
+      f += (int64_t)S.thq[e] * c;
+      continue;
+    }
+    uint64_t m;
+    if (kind == K_LOOK) {
       int idx;
       switch (cfn) {
         case 4: idx = S.indeg[j] + 1 - aij; break;
         case 7: idx = S.outdeg[j]; break;
-        case 8: idx = ri_cj; break;
-        case 9: idx = ri_rj; break;
-        case 10: idx = ci_cj; break;
-        case 11: idx = ci_rj; break;
+        case 8: idx = cnt(ca); break;
         case 12: idx = j; break;
         case 13: idx = S.z[j] - P.zlo; break;
         case 14: idx = i * n + j; break;
         default: idx = (S.z[i] - P.zlo) * P.zR + (S.z[j] - P.zlo); break;  // 15
       }
-      const float2 t2 = P.tab2[S.eoffd[e] + idx];
-      v = __uint_as_float(__float_as_uint(t2.x) ^ sg);
-      vlo = __uint_as_float(__float_as_uint(t2.y) ^ sg);
-      term = __fmul_rn(th, v);
-      tlo = fmaf(th, vlo, fmaf(th, v, -term));
+      m = X.tabq[S.eoffd[e] + idx];
     } else if (kind == K_STEP) {
-      const int q = 2 * aij + aji;
-      v = S.stepd32[4 * e + q];
-      vlo = S.stepdlo32[4 * e + q];
-      term = S.stept32[4 * e + q];
-      tlo = S.steptlo32[4 * e + q];
-    } else if (kind == K_ZERO) {
-      v = 0.f;
-      has_term = false;
-    } else if (MULTI && kind == K_CROSS) {
-      const int c = cross_count(S, X, n, W, cfn, S.eoffd[e], i, j);
-      const bool rt = cfn == 36 && S.p1[e] >= 2.0;
-      const float m = rt ? sqrtf((float)c) : (float)c;
-      // sqrt(c) = m + (c - m^2) / (2m) to ~2^-48 (one Newton step; the residual is exact)
-      const float mlo = (rt && c > 0) ? __fdiv_rn(fmaf(-m, m, (float)c), __fmul_rn(2.f, m)) : 0.f;
-      v = __uint_as_float(__float_as_uint(m) ^ sg);
-      vlo = __uint_as_float(__float_as_uint(mlo) ^ sg);
-      term = __fmul_rn(th, v);
-      tlo = fmaf(th, vlo, fmaf(th, v, -term));
+      m = S.stepq[4 * e + 2 * aij + aji];
     } else if (S.tid[e] == 32) {
-      const int c0 = S.i0[e], c1 = S.i1[e], c2 = S.i2[e];
-      v = __fmul_rn(d32[c0], d32[c1]);
-      vlo = __fadd_rn(fmaf(d32[c0], d32[c1], -v),
-                      fmaf(d32[c0], d32lo[c1], __fmul_rn(d32lo[c0], d32[c1])));
-      if (c2 >= 0) {
-        const float v2 = __fmul_rn(v, d32[c2]);
-        vlo = __fadd_rn(fmaf(v, d32[c2], -v2), fmaf(v, d32lo[c2], __fmul_rn(vlo, d32[c2])));
-        v = v2;
-      } else if (aij) {
-        v = -v;
-        vlo = -vlo;
-      }
-      term = __fmul_rn(th, v);
-      tlo = fmaf(th, vlo, fmaf(th, v, -term));
+      // product of the components' magnitudes (each at its scale)
+      auto mag = [&](int q) -> int64_t {
+        const int cl = S.ecls[q] & 0xFF;
+        if (cl == FX_DELTA) return (int64_t)1 << S.esd[q];
+        if (cl == FX_CNT) return (int64_t)v[q] << S.esd[q];
+        if (cl == FX_UNI) return (int64_t)(S.stepq[4 * q] - (1ull << 62));
+        return cl == FX_REAL && v[q] ? (int64_t)(v[q] - (1ull << 62)) : 0;
+      };
+      int64_t p = __mul64hi(mag(S.i0[e]), mag(S.i1[e]));
+      if (S.i2[e] >= 0) p = __mul64hi(p, mag(S.i2[e]));
+      m = (uint64_t)(p + (1LL << 62));
+    } else if (cfn == 16) {
+      m = gw_fixed(S, X, n, P.W, e, S.tid[e], j, aij);
     } else {
-      const double v64 = gen_stat(P, S, X, e, j, aij, aji, ri_cj, ri_rj, rj_ci, ci_cj, ci_rj, nullptr);
-      v = (float)v64;
-      vlo = (float)__dsub_rn(v64, (double)v);
-      term = __fmul_rn(th, v);
-      tlo = fmaf(th, vlo, fmaf(th, v, -term));
+      const double g = gen_stat(P, S, X, e, j, aij, aji, ca != 0xFF ? cnt(ca) : 0, nullptr);
+      m = real_fx(aij ? -g : g, S.esd[e]);
     }
-    if ((S.ety[e] == 1 && aij) || (S.ety[e] == 2 && !aij)) {
-      v = 0.f;
-      vlo = 0.f;
-      has_term = false;
-    }
-    d32[e] = v;
-    d32lo[e] = vlo;
-    if (has_term) {
-      float err;
-      two_sum(f, term, f, err);
-      fo = __fadd_rn(fo, __fadd_rn(err, tlo));
-      a = __fadd_rn(a, fabsf(term));
-    }
+    v[e] = m;
+    f += term_fx(S.thq[e], S.ecls[e], m);
+    if (ety) f += base_fx(S.thq[e], S.ecls[e]);
   }
-  *absf = a;
-  *fx = make_float2(f, fo);
   return f;
 }
 

@@ -22,10 +22,96 @@ struct LaunchShape {
   SliceLayout lay;
 };
 
+// Global scratch of a launch, one piece per team (and network): the chain's
+// in-rows and out-rows (cols_words each; null where the slice holds them) and
+// its count matrices (counts_stride counts; null without).
+struct Scratch {
+  uint32_t *cols = nullptr, *rows = nullptr;
+  uint16_t *counts = nullptr;
+  size_t cols_words = 0, counts_stride = 0;
+};
+
+// The two-path counters of a model's effects and each effect's packed count
+// function (cfn_pack): fn[e] and the counters it reads. multi: cross effects
+// (types 36, 37) read network cross_src[e].
+inline void plan_counters(const int *tid, int k, bool multi, const int *cross_src, CounterSet &C,
+                          int *packed) {
+  C.n = 0;
+  C.mask = 0;
+  C.ntask = 0;
+  C.tp = C.tq = -1;
+  auto add = [&](int list, int m1, int m2 = CM_NONE) -> int {
+    for (int c = 0; c < C.n; ++c)
+      if (C.list[c] == list && C.m1[c] == m1 && C.m2[c] == m2) return c;
+    C.list[C.n] = (unsigned char)list;
+    C.m1[C.n] = (unsigned char)m1;
+    C.m2[C.n] = (unsigned char)m2;
+    return C.n++;
+  };
+  for (int e = 0; e < k; ++e) {
+    int &p = packed[e];
+    p = cfn_pack(0);
+    switch (tid[e]) {
+      case 2: p = cfn_pack(2, add(CL_OUT, CM_ROWS, CM_COLS)); break;
+      case 3: case 23: p = cfn_pack(3, add(CL_IN, CM_COLS)); break;
+      case 5: {
+        C.tp = add(CL_OUT, CM_ROWS);
+        const int a = add(CL_TP0, CM_COLS), b = add(CL_TP1, CM_COLS);
+        p = cfn_pack(5, a, b, C.tp);
+        break;
+      }
+      case 6: {
+        const int a = add(CL_OUT, CM_ROWS), b = add(CL_MUTUAL, CM_COLS);
+        p = cfn_pack(6, a, b);
+        break;
+      }
+      case 24: p = cfn_pack(8, add(CL_OUT, CM_ROWS)); break;
+      case 26: p = cfn_pack(8, add(CL_OUT, CM_COLS)); break;
+      case 27: p = cfn_pack(8, add(CL_IN, CM_ROWS)); break;
+      case 28: p = cfn_pack(8, add(CL_IN, CM_COLS)); break;
+      case 29: C.tp = add(CL_OUT, CM_ROWS); break;
+      case 30: C.tq = add(CL_OUT, CM_COLS); break;
+      case 36:
+        if (multi) p = cfn_pack(36, add(CL_NET + cross_src[e], CM_NCOLS + cross_src[e]));
+        break;
+      case 37:
+        if (multi) p = cfn_pack(37, add(CL_NET + cross_src[e], CM_ROWS));
+        break;
+      default: break;
+    }
+  }
+}
+
+// The updates of the count matrices when a tie toggles in network x: for the
+// counters (masked) of network d = 0..D-1 that read x. A counter is the product
+// C = L M of its set's relation L (i to h) and its relation M (h to j), so
+// toggling L's tie (i, h) adds row h of M to row i of C, and toggling M's tie
+// (h, j) adds column h of L to column j of C; both cannot meet off the diagonal.
+inline void counter_tasks(const CounterSet *const *nets, int D, int x, CounterSet &out) {
+  out.ntask = 0;
+  for (int d = 0; d < D; ++d) {
+    const CounterSet &C = *nets[d];
+    for (int c = 0, rank = 0; c < C.n; ++c) {
+      if (!((C.mask >> c) & 1u)) continue;
+      const bool lin = C.list[c] == CL_IN;
+      const int netL = C.list[c] >= CL_NET ? C.list[c] - CL_NET : d;
+      for (int m : {(int)C.m1[c], (int)C.m2[c]}) {
+        if (m == CM_NONE) continue;
+        const bool mrows = m == CM_ROWS;
+        const int netM = m >= CM_NCOLS ? m - CM_NCOLS : d;
+        // L's tie: i = u, h = v (CL_IN: i = v, h = u); row h of M into row i
+        if (netL == x) out.task[out.ntask++] = task_pack(!mrows, !lin, lin, false, rank, netM, d);
+        // M's tie: h = u, j = v (its transpose: h = v, j = u); column h of L into column j
+        if (netM == x) out.task[out.ntask++] = task_pack(!lin, !mrows, mrows, true, rank, netL, d);
+      }
+      ++rank;
+    }
+  }
+}
+
 cudaError_t launch_period(const LaunchShape &sh, const DevProblem *probs, const long long *unit_start,
                           int nprob, long long total, unsigned long long *counter,
-                          uint32_t *cols_scratch, uint32_t *rows_scratch, size_t cols_words,
-                          cudaStream_t st, bool valid = false);
+                          const Scratch &sc, cudaStream_t st, bool valid = false);
 // valid: the validation build of the period kernel (trace, supplied words;
 // CTAs of at most 256 threads)
 int period_blocks_per_sm(int threads, size_t dyn_smem, bool valid = false);
@@ -34,8 +120,7 @@ static_assert(kMaxNet == CUSNA_MAXNET, "network capacity of the kernels and the 
 static_assert(kMaxEff == CUSNA_MAXEFF, "effect capacity of the kernels and the ABI");
 int multi_blocks_per_sm(int threads, size_t dyn_smem);
 cudaError_t launch_multi(const LaunchShape &sh, const DevProblem *nets, const MultiDev &md, int M,
-                         unsigned long long *counter, uint32_t *cols_scratch,
-                         uint32_t *rows_scratch, size_t cols_words, cudaStream_t st);
+                         unsigned long long *counter, const Scratch &sc, cudaStream_t st);
 // Cross-network statistic of M dense own networks a against the dense source
 // predictor wp; ar (M*n*W words, type 37) and wr (n*W words, type 36) are
 // scratch for packed rows.
@@ -69,6 +154,9 @@ struct PlanTable {
 cudaError_t launch_plan_prologue(DevProblem *probs, const unsigned long long *base_seed, int count,
                                  unsigned long long *epoch, const PlanTable *tabs, int n_tabs,
                                  cudaStream_t st);
+// Start values of the count matrices of a launch's problems (their c0).
+cudaError_t launch_counts_init(const DevProblem *probs, int nprob, int nmax, bool multi,
+                               cudaStream_t st);
 long long kernel_launches();  // kernels launched so far by the calling thread
 void note_launch();           // counts a launch made outside the wrappers here
 // Raises a kernel's dynamic shared memory limit on the current device to at
@@ -89,7 +177,7 @@ cudaError_t launch_netstats(const uint8_t *a, int M, const StatDesc &D, double *
 cudaError_t launch_behstats(const int *z, int n, int M, int kb, const int *bty, const uint8_t *xnet,
                             const int *bkdist, double zbar, double brange, double bsimmean,
                             double *out, int sms, cudaStream_t st);
-cudaError_t launch_prep_bits(const uint32_t *src, int n, int W, uint32_t *dstT, uint32_t *dstcT,
+cudaError_t launch_prep_bits(const uint32_t *src, int n, int W, uint32_t *dst, uint32_t *dstc,
                              int def_mode, cudaStream_t st);
 cudaError_t launch_prep_desc(const double *d64, const float *d32, size_t cnt, double *dst,
                              cudaStream_t st);

@@ -21,15 +21,14 @@ int multi_blocks_per_sm(int threads, size_t dyn_smem) {
 }
 
 cudaError_t launch_multi(const LaunchShape &sh, const DevProblem *nets, const MultiDev &md, int M,
-                         unsigned long long *counter, uint32_t *cols_scratch,
-                         uint32_t *rows_scratch, size_t cols_words, cudaStream_t st) {
+                         unsigned long long *counter, const Scratch &sc, cudaStream_t st) {
   const int threads = 32 * sh.G * sh.teams_per_cta;
   const size_t dyn = sh.lay.bytes * md.D * sh.teams_per_cta;
   auto kern = threads <= 256 ? multi_kernel<256> : multi_kernel<512>;
   cudaError_t e = raise_dyn_smem((const void *)kern, dyn);
   if (e != cudaSuccess) return e;
-  kern<<<sh.ctas, threads, dyn, st>>>(nets, md, M, counter, sh.lay, sh.G, cols_scratch,
-                                      rows_scratch, cols_words);
+  kern<<<sh.ctas, threads, dyn, st>>>(nets, md, M, counter, sh.lay, sh.G, sc.cols, sc.rows,
+                                      sc.cols_words, sc.counts, sc.counts_stride);
   return cudaGetLastError();
 }
 

@@ -18,18 +18,21 @@ namespace cusna {
 
 __device__ __forceinline__ Slice multi_slice(unsigned char *base, const SliceLayout &lay, int d,
                                              uint32_t *cols_g, uint32_t *rows_g,
-                                             size_t cols_words) {
+                                             uint16_t *counts_g, size_t cols_words,
+                                             size_t counts_stride, const int2 *etab) {
   return carve(base + (size_t)d * lay.bytes, lay, cols_g ? cols_g + (size_t)d * cols_words : nullptr,
-               rows_g ? rows_g + (size_t)d * cols_words : nullptr);
+               rows_g ? rows_g + (size_t)d * cols_words : nullptr,
+               counts_g ? counts_g + (size_t)d * counts_stride : nullptr, etab);
 }
 
 static __device__ void run_chain_multi(const Team &T, const DevProblem *nets, const MultiDev &md,
                                 unsigned char *base, const SliceLayout &lay, uint32_t *cols_g,
-                                uint32_t *rows_g, size_t cols_words, int c) {
+                                uint32_t *rows_g, uint16_t *counts_g, size_t cols_words,
+                                size_t counts_stride, const int2 *etab, int c) {
   const int D = md.D, n = md.n, L = T.L;
   const uint32_t chain = (uint32_t)c;
   for (int d = 0; d < D; ++d)
-    chain_init(T, nets[d], multi_slice(base, lay, d, cols_g, rows_g, cols_words), c);
+    chain_init(T, nets[d], multi_slice(base, lay, d, cols_g, rows_g, counts_g, cols_words, counts_stride, etab), c);
   double lam_d[kMaxNet];
   double lam_tot = 0.0;
   for (int d = 0; d < D; ++d) {
@@ -40,11 +43,11 @@ static __device__ void run_chain_multi(const Team &T, const DevProblem *nets, co
   long long ms = 0, msd[kMaxNet] = {};
   double t = 0.0;
   double dbuf[kMaxEff];
-  const Slice S0 = multi_slice(base, lay, 0, cols_g, rows_g, cols_words);
-  // network w's rows: rows0 + w*net_stride words (in shared memory the slices
-  // follow one another; in global scratch each network has cols_words)
-  const uint32_t *rows0 = S0.rowsT;
-  const size_t net_stride = rows_g ? cols_words : lay.bytes / 4;
+  const Slice S0 = multi_slice(base, lay, 0, cols_g, rows_g, counts_g, cols_words, counts_stride, etab);
+  // every network's state (in shared memory the slices follow one another; in
+  // global scratch each network has cols_words)
+  const NetBase nb{S0.rows, S0.cols, S0.cm, rows_g ? cols_words : lay.bytes / 4,
+                   cols_g ? cols_words : lay.bytes / 4, counts_stride, S0.misc, lay.bytes / 4, D};
   for (;;) {
     const int slot = (int)(ms & 31);
     if (slot == 0) {
@@ -70,33 +73,26 @@ static __device__ void run_chain_multi(const Team &T, const DevProblem *nets, co
     if (t > 1.0) break;
     const int d = S0.rnet[slot], i = S0.rfocal[slot];
     const DevProblem &P = nets[d];
-    const Slice S = multi_slice(base, lay, d, cols_g, rows_g, cols_words);
-    const int jstar = net_choice<true>(T, P, S, i, ms, chain, dbuf, rows0, net_stride, d);
-    const int aij_star = bit_of(S.rowsT, n, i, jstar);
+    const Slice S = multi_slice(base, lay, d, cols_g, rows_g, counts_g, cols_words, counts_stride, etab);
+    const int rslot = (int)msd[d] & (kRing - 1);
+    const int jstar = net_choice<true>(T, P, S, i, ms, chain, dbuf, &nb, rslot, d);
+    const int aij_star = bit_of(S.rows, n, i, jstar);
     T.sync();
-    if (T.tl < P.k) {
-      const int e = T.tl;
-      const double s0 = S.red[32 * T.G], se = S.red[32 * T.G + 1 + e];
-      S.sc[e] = __dadd_rn(S.sc[e], __dsub_rn(S.dstar[e], __ddiv_rn(se, s0)));
-    }
+    score_slot(T, P, S, rslot);
     ++ms;
     ++msd[d];
-    if (jstar != i && T.tl == 0) {
-      const int j = jstar, dl = 1 - 2 * aij_star;
-      S.rowsT[(j >> 5) * n + i] ^= 1u << (j & 31);
-      S.colsT[(i >> 5) * n + j] ^= 1u << (i & 31);
-      S.indeg[j] += dl;
-      S.outdeg[i] += dl;
-      if (P.symflag) {
-        S.rowsT[(i >> 5) * n + j] ^= 1u << (i & 31);
-        S.colsT[(j >> 5) * n + i] ^= 1u << (j & 31);
-        S.indeg[i] += dl;
-        S.outdeg[j] += dl;
-      }
-    }
+    if (P.cnt.ntask && jstar != i) counts_toggle(T, P, nb, i, jstar, 1 - 2 * aij_star);
+    if (jstar != i) toggle_tie(T, S, n, i, jstar, 1 - 2 * aij_star, P.symflag);
     T.sync();
     if (ms >= kMaxSteps) break;
   }
+  T.sync();
+  for (int d = 0; d < D; ++d) {
+    const Slice S = multi_slice(base, lay, d, cols_g, rows_g, counts_g, cols_words, counts_stride, etab);
+    if ((msd[d] & (kRing - 1)) && ring_scores(nets[d], S))
+      scores_flush(T, S, nets[d].k, (int)msd[d] & (kRing - 1));
+  }
+  T.sync();
   // outputs (src/libcusna_saom_cpu.cpp:549-551, :594-600)
   if (T.tl == 0) {
     if (md.ntim) md.ntim[c] = t;
@@ -107,7 +103,7 @@ static __device__ void run_chain_multi(const Team &T, const DevProblem *nets, co
             (float)__dsub_rn(__ddiv_rn((double)msd[d], lam_d[d]), (double)md.nact);
   }
   for (int d = 0; d < D; ++d) {
-    const Slice S = multi_slice(base, lay, d, cols_g, rows_g, cols_words);
+    const Slice S = multi_slice(base, lay, d, cols_g, rows_g, counts_g, cols_words, counts_stride, etab);
     if (md.scores)
       for (int q = T.tl; q < md.goff[d + 1] - md.goff[d]; q += L)
         md.scores[(size_t)c * md.k + md.gidx[md.goff[d] + q]] = (float)S.sc[q];
@@ -115,7 +111,7 @@ static __device__ void run_chain_multi(const Team &T, const DevProblem *nets, co
       uint8_t *out = md.a_ends + ((size_t)c * D + d) * n * n;
       for (size_t x = T.tl; x < (size_t)n * n; x += L) {
         const int r = (int)(x / n), col = (int)(x % n);
-        out[x] = (uint8_t)bit_of(S.rowsT, n, r, col);
+        out[x] = (uint8_t)bit_of(S.rows, n, r, col);
       }
     }
   }
@@ -126,8 +122,11 @@ template <int MAXT>
 __global__ void __launch_bounds__(MAXT, 1)
 multi_kernel(const DevProblem *__restrict__ nets, MultiDev md, int M,
              unsigned long long *counter, SliceLayout lay, int G, uint32_t *cols_scratch,
-             uint32_t *rows_scratch, size_t cols_words) {
+             uint32_t *rows_scratch, size_t cols_words, uint16_t *counts_scratch,
+             size_t counts_stride) {
   extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ int2 etab[256];
+  load_exp_table(etab, nets);
   Team T;
   T.G = G;
   T.L = 32 * G;
@@ -141,10 +140,8 @@ multi_kernel(const DevProblem *__restrict__ nets, MultiDev md, int M,
   unsigned char *base = smem + (size_t)tw * lay.bytes * md.D;
   uint32_t *cg = cols_scratch ? cols_scratch + slot * md.D * cols_words : nullptr;
   uint32_t *rg = rows_scratch ? rows_scratch + slot * md.D * cols_words : nullptr;
-  const Slice S0 = multi_slice(base, lay, 0, cg, rg, cols_words);
-  // each network's exponential table (ordered before use by chain_init's barriers)
-  for (int d = 0; d < md.D; ++d)
-    fill_exp_table(multi_slice(base, lay, d, cg, rg, cols_words).etab, T.tl, T.L);
+  uint16_t *pg = counts_scratch ? counts_scratch + slot * md.D * counts_stride : nullptr;
+  const Slice S0 = multi_slice(base, lay, 0, cg, rg, pg, cols_words, counts_stride, etab);
   for (;;) {
     long long u = 0;
     if (T.tl == 0) u = (long long)atomicAdd(counter, 1ull);
@@ -157,7 +154,7 @@ multi_kernel(const DevProblem *__restrict__ nets, MultiDev md, int M,
       T.sync();
     }
     if (u >= M) break;
-    run_chain_multi(T, nets, md, base, lay, cg, rg, cols_words, (int)u);
+    run_chain_multi(T, nets, md, base, lay, cg, rg, pg, cols_words, counts_stride, etab, (int)u);
   }
 }
 

@@ -17,16 +17,16 @@ __device__ void chain_finish(const Team &T, const DevProblem &P, const Slice &S,
     for (int i = 0; i < n; ++i) {
       if (!((P.inact[i >> 5] >> (i & 31)) & 1u)) continue;
       for (int w = T.tl; w < W; w += T.L) {
-        S.rowsT[w * n + i] = P.x0T[w * n + i];
-        S.colsT[w * n + i] = P.x0cT[w * n + i];
+        S.rows[w * n + i] = P.x0r[w * n + i];
+        S.cols[w * n + i] = P.x0c[w * n + i];
       }
       T.sync();
       const uint32_t bit = 1u << (i & 31);
       const int wi = i >> 5;
       for (int j = T.tl; j < n; j += T.L) {
         if (j == i) continue;
-        S.rowsT[wi * n + j] = (S.rowsT[wi * n + j] & ~bit) | (P.x0T[wi * n + j] & bit);
-        S.colsT[wi * n + j] = (S.colsT[wi * n + j] & ~bit) | (P.x0cT[wi * n + j] & bit);
+        S.rows[wi * n + j] = (S.rows[wi * n + j] & ~bit) | (P.x0r[wi * n + j] & bit);
+        S.cols[wi * n + j] = (S.cols[wi * n + j] & ~bit) | (P.x0c[wi * n + j] & bit);
       }
       T.sync();
     }
@@ -43,14 +43,14 @@ __device__ void chain_finish(const Team &T, const DevProblem &P, const Slice &S,
         for (int b = 0; b < 4; ++b) {
           const size_t x = 4 * q + b;
           const int i = (int)(x / n), j = (int)(x % n);
-          v |= (uint32_t)bit_of(S.rowsT, n, i, j) << (8 * b);
+          v |= (uint32_t)bit_of(S.rows, n, i, j) << (8 * b);
         }
         o4[q] = v;
       }
     } else {
       for (size_t x = T.tl; x < nn; x += T.L) {
         const int i = (int)(x / n), j = (int)(x % n);
-        out[x] = (uint8_t)bit_of(S.rowsT, n, i, j);
+        out[x] = (uint8_t)bit_of(S.rows, n, i, j);
       }
     }
   }
@@ -59,7 +59,7 @@ __device__ void chain_finish(const Team &T, const DevProblem &P, const Slice &S,
   for (int i = T.tl; i < n; i += T.L) {
     int cnt = 0;
     for (int w = 0; w < W; ++w)
-      cnt += __popc((S.rowsT[w * n + i] ^ P.x0T[w * n + i]) & P.kdistT[w * n + i]);
+      cnt += __popc((S.rows[w * n + i] ^ P.x0r[w * n + i]) & P.kdistr[w * n + i]);
     if (P.actor_dist) P.actor_dist[(size_t)c * n + i] = cnt;
     ds += cnt;
   }
@@ -70,15 +70,15 @@ __device__ void chain_finish(const Team &T, const DevProblem &P, const Slice &S,
   if (P.stats) {
     T.sync();
     for (int x = T.tl; x < W * n; x += T.L) {
-      S.rowsT[x] = (S.rowsT[x] & P.keepT[x]) | P.forceT[x];
-      S.colsT[x] = (S.colsT[x] & P.keepcT[x]) | P.forcecT[x];
+      S.rows[x] = (S.rows[x] & P.keepr[x]) | P.forcer[x];
+      S.cols[x] = (S.cols[x] & P.keepc[x]) | P.forcec[x];
     }
     T.sync();
     for (int x = T.tl; x < n; x += T.L) {
       int od = 0, id = 0;
       for (int w = 0; w < W; ++w) {
-        od += __popc(S.rowsT[w * n + x]);
-        id += __popc(S.colsT[w * n + x]);
+        od += __popc(S.rows[w * n + x]);
+        id += __popc(S.cols[w * n + x]);
       }
       S.outdeg[x] = od;
       S.indeg[x] = id;
@@ -88,7 +88,7 @@ __device__ void chain_finish(const Team &T, const DevProblem &P, const Slice &S,
     D.vmat = P.vmat; D.vb = P.vb; D.wtab = P.wtab; D.p1 = P.p1; D.p2 = P.p2;
     D.vmiss = P.vmiss; D.dyn = P.dyn; D.od0 = P.od0; D.id0 = P.id0; D.type_ids = P.type_ids;
     D.n = n; D.W = W; D.k = k; D.symflag = P.symflag;
-    network_stats_team(T, D, S.rowsT, S.colsT, S.outdeg, S.indeg, S.red, P.stats + (size_t)c * k);
+    network_stats_team(T, D, S.rows, S.cols, S.outdeg, S.indeg, S.red, P.stats + (size_t)c * k);
   }
   if (T.tl == 0) {
     if (P.dist) P.dist[c] = (int)dist;
@@ -128,8 +128,11 @@ template <int MAXT, bool VALID = false>
 __global__ void __launch_bounds__(MAXT, MAXT == 512 ? 1 : CUSNA_MINB_256)
 period_kernel(const DevProblem *__restrict__ probs, const long long *__restrict__ unit_start,
               int nprob, long long total, unsigned long long *counter, SliceLayout lay, int G,
-              uint32_t *cols_scratch, uint32_t *rows_scratch, size_t cols_words) {
+              uint32_t *cols_scratch, uint32_t *rows_scratch, size_t cols_words,
+              uint16_t *counts_scratch, size_t counts_stride) {
   extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ int2 etab[256];
+  load_exp_table(etab, probs);
   Team T;
   T.G = G;
   T.L = 32 * G;
@@ -142,8 +145,8 @@ period_kernel(const DevProblem *__restrict__ probs, const long long *__restrict_
   const size_t slot = (size_t)blockIdx.x * teams_per_cta + tw;
   Slice S = carve(smem + (size_t)tw * lay.bytes, lay,
                   cols_scratch ? cols_scratch + slot * cols_words : nullptr,
-                  rows_scratch ? rows_scratch + slot * cols_words : nullptr);
-  fill_exp_table(S.etab, T.tl, T.L);  // ordered before its first use by chain_init's barriers
+                  rows_scratch ? rows_scratch + slot * cols_words : nullptr,
+                  counts_scratch ? counts_scratch + slot * counts_stride : nullptr, etab);
   for (;;) {
     long long u = 0;
     if (T.tl == 0) u = (long long)atomicAdd(counter, 1ull);

@@ -4,6 +4,7 @@
 #include "saom_period.cuh"
 #include "saom_launch.h"
 
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <utility>
@@ -123,8 +124,8 @@ __global__ void behstats_kernel(const int *__restrict__ z_batch, int n, int M, i
 // Row-major n*W bit rows -> word-major W*n; optionally also the transposed
 // matrix (in-rows) word-major. def_offdiag: when src is null, fill with the
 // all-ones off-diagonal matrix (the reference's default masks).
-__global__ void prep_bits_kernel(const uint32_t *src, int n, int W, uint32_t *dstT,
-                                 uint32_t *dstcT, int def_mode) {
+__global__ void prep_bits_kernel(const uint32_t *src, int n, int W, uint32_t *dst,
+                                 uint32_t *dstc, int def_mode) {
   const size_t total = (size_t)W * n;
   for (size_t x = (size_t)blockIdx.x * blockDim.x + threadIdx.x; x < total;
        x += (size_t)gridDim.x * blockDim.x) {
@@ -143,9 +144,56 @@ __global__ void prep_bits_kernel(const uint32_t *src, int n, int W, uint32_t *ds
       v |= (uint32_t)bit_rq << b;
       vc |= (uint32_t)bit_qr << b;
     }
-    if (dstT) dstT[x] = v;
-    if (dstcT) dstcT[x] = vc;
+    if (dst) dst[x] = v;
+    if (dstc) dstc[x] = vc;
   }
+}
+
+// Start values of the counters that chains hold as matrices, for every problem
+// of a launch (block y = problem): cell (i, j) by popcounts, as count_pc forms it
+// for a ministep of i. Networks w of a multi-network problem are the launch's
+// problems w.
+__global__ void __launch_bounds__(256) counts_init_kernel(const DevProblem *__restrict__ probs,
+                                                          bool multi) {
+  const DevProblem &P = probs[blockIdx.y];
+  const int n = P.n, W = P.W;
+  uint16_t *C = const_cast<uint16_t *>(P.c0);
+  for (int c = 0; c < P.cnt.n; ++c) {
+    if (!((P.cnt.mask >> c) & 1u)) continue;
+    const int list = P.cnt.list[c];
+    const uint32_t *A = list == CL_IN ? P.simc
+                        : (multi && list >= CL_NET) ? probs[list - CL_NET].simr : P.simr;
+    auto rel = [&](int m) -> const uint32_t * {
+      return m == CM_ROWS ? P.simc : ((multi && m >= CM_NCOLS) ? probs[m - CM_NCOLS].simr : P.simr);
+    };
+    const uint32_t *M1 = rel(P.cnt.m1[c]);
+    const uint32_t *M2 = P.cnt.m2[c] == CM_NONE ? nullptr : rel(P.cnt.m2[c]);
+    for (size_t x = (size_t)blockIdx.x * blockDim.x + threadIdx.x; x < (size_t)n * n;
+         x += (size_t)gridDim.x * blockDim.x) {
+      const int i = (int)(x / n), j = (int)(x % n);
+      int v = 0;
+      for (int w = 0; w < W; ++w) {
+        const uint32_t a = A[w * n + i];
+        v += __popc(a & M1[w * n + j]);
+        if (M2) v += __popc(a & M2[w * n + j]);
+      }
+      C[x] = (uint16_t)v;
+    }
+    C += cm_size(n);
+  }
+}
+
+cudaError_t launch_counts_init(const DevProblem *probs, int nprob, int nmax, bool multi,
+                               cudaStream_t st) {
+  const int bx = (int)std::min<size_t>(((size_t)nmax * nmax + 255) / 256, 1024);
+  for (int q = 0; q < nprob; q += 65535) {
+    const dim3 grid(bx, std::min(nprob - q, 65535));
+    counts_init_kernel<<<grid, 256, 0, st>>>(probs + q, multi);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    note_launch();
+  }
+  return cudaSuccess;
 }
 
 // float64 descriptor with the reference's precedence: the *64 array if given,
@@ -215,8 +263,7 @@ int period_blocks_per_sm(int threads, size_t dyn_smem, bool valid) {
 
 cudaError_t launch_period(const LaunchShape &sh, const DevProblem *probs, const long long *unit_start,
                           int nprob, long long total, unsigned long long *counter,
-                          uint32_t *cols_scratch, uint32_t *rows_scratch, size_t cols_words,
-                          cudaStream_t st, bool valid) {
+                          const Scratch &sc, cudaStream_t st, bool valid) {
   const int threads = 32 * sh.G * sh.teams_per_cta;
   const size_t dyn = sh.lay.bytes * sh.teams_per_cta;
   if (valid && threads > 256) return cudaErrorInvalidConfiguration;
@@ -225,7 +272,7 @@ cudaError_t launch_period(const LaunchShape &sh, const DevProblem *probs, const 
   cudaError_t e = raise_dyn_smem((const void *)kern, dyn);
   if (e != cudaSuccess) return e;
   kern<<<sh.ctas, threads, dyn, st>>>(probs, unit_start, nprob, total, counter, sh.lay, sh.G,
-                                      cols_scratch, rows_scratch, cols_words);
+                                      sc.cols, sc.rows, sc.cols_words, sc.counts, sc.counts_stride);
   return counted(cudaGetLastError());
 }
 
@@ -301,13 +348,13 @@ cudaError_t launch_behstats(const int *z, int n, int M, int kb, const int *bty, 
   return counted(cudaGetLastError());
 }
 
-cudaError_t launch_prep_bits(const uint32_t *src, int n, int W, uint32_t *dstT, uint32_t *dstcT,
+cudaError_t launch_prep_bits(const uint32_t *src, int n, int W, uint32_t *dst, uint32_t *dstc,
                              int def_mode, cudaStream_t st) {
   const size_t total = (size_t)W * n;
   int blocks = (int)((total + 255) / 256);
   if (blocks > 1024) blocks = 1024;
   if (blocks < 1) blocks = 1;
-  prep_bits_kernel<<<blocks, 256, 0, st>>>(src, n, W, dstT, dstcT, def_mode);
+  prep_bits_kernel<<<blocks, 256, 0, st>>>(src, n, W, dst, dstc, def_mode);
   return counted(cudaGetLastError());
 }
 

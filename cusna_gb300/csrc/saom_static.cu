@@ -19,6 +19,7 @@
 // overwrite each other's scratch and race. Callers must serialise them.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdio>
@@ -31,7 +32,8 @@ namespace cusna {
 namespace {
 
 constexpr size_t kStaticScratchBytes = (size_t)16 << 20;  // 16 MiB per device
-static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
+constexpr size_t kStaticExtra = 4096;   // the exponential's table and the effects' bounds
+static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes + kStaticExtra];
 
 constexpr int kMaxDevices = 64;
 std::atomic<unsigned char *> g_scratch_addr[kMaxDevices];
@@ -67,9 +69,78 @@ cusna_status scratch_address(unsigned char **out) {
 }
 
 // Any self-tie (a_ii) in word-major rows: flag[0] = 1.
-__global__ void self_tie_kernel(const uint32_t *rowsT, int n, int *flag) {
+__global__ void self_tie_kernel(const uint32_t *rows, int n, int *flag) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    if ((rowsT[(i >> 5) * n + i] >> (i & 31)) & 1u) flag[0] = 1;
+    if ((rows[(i >> 5) * n + i] >> (i & 31)) & 1u) flag[0] = 1;
+}
+
+// Bytes per team of the scratch rule (see the launch shape below): the state of
+// a chain of this size in a fixed accounting.
+size_t scratch_rule_slice(int n, int W, int k, int kb, int nr, int G, bool cols, bool tp, bool gw,
+                          bool tq) {
+  size_t o = 0;
+  auto put = [&](size_t bytes) { o = al16(o + bytes); };
+  const size_t N = (size_t)n, K = (size_t)k;
+  put(W * N * 4);
+  put(cols ? W * N * 4 : 0);
+  put(N * 2); put(N * 2); put(N * 4); put(N * 4);
+  put((N + 31) / 32 * 2 * (K + 1) * 4);
+  put((size_t)W * 4);
+  put(tp || gw ? N * 4 : 0);
+  put(tq ? N * 4 : 0);
+  put(tp ? (size_t)W * 8 : 0);
+  put(nr > 0 ? N * 8 : 0);
+  put((size_t)32 * G * 8 + 32 * 8);
+  for (int x = 0; x < 3; ++x) put(K * 8);
+  put((size_t)(kb + 1) * 8); put((size_t)(kb + 1) * 8); put((size_t)(nr + 1) * 8);
+  put(K * 8); put(K * 8);
+  for (int x = 0; x < 6; ++x) put(K * 4);
+  put((size_t)(kb + 1) * 4); put((size_t)(nr + 1) * 4);
+  put(64); put(256); put(128); put(128); put(128);
+  for (int x = 0; x < 4; ++x) put(K * 4);
+  put(K * 32); put(K * 32); put(K * 4);
+  for (int x = 0; x < 4; ++x) put(K * 16);
+  put(512);
+  return al16(o);
+}
+
+// Bounds on |d_e| (effect_bound) from the prepared descriptors, an effect per block.
+__global__ void bounds_kernel(const int *tid, const int *dyn, const double *vmat, const double *wtab,
+                              const double *p1, const double *p2, const int *z0, double zbar, int kb,
+                              int zmin, int zmax, int n, double *bound) {
+  const int e = blockIdx.x;
+  double v = 0.0, w = 0.0;
+  bool finite = true;
+  for (int j = threadIdx.x; j <= n; j += 32) {
+    const double x = wtab[(size_t)e * (n + 1) + j];
+    w = fmax(w, fabs(x));
+    finite = finite && isfinite(x);
+    if (j == n) continue;
+    const double y = dyn[e] ? (double)z0[j] - zbar : vmat[(size_t)e * n + j];
+    v = fmax(v, fabs(y));
+    finite = finite && isfinite(y);
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    v = fmax(v, __shfl_xor_sync(kFull, v, o));
+    w = fmax(w, __shfl_xor_sync(kFull, w, o));
+  }
+  finite = __all_sync(kFull, finite) && isfinite(p1[e]) && isfinite(p2[e]);
+  if (dyn[e] && kb > 0) v = fmax(v, fmax(fabs((double)zmin - zbar), fabs((double)zmax - zbar)));
+  if (threadIdx.x == 0) bound[e] = finite ? effect_bound(tid[e], n, v, w, p1[e], p2[e]) : INFINITY;
+}
+
+// exp_fx's table as the kernels read it.
+const uint64_t *exp_table() {
+  static const struct Table {
+    uint64_t q[256];
+    Table() {
+      for (int x = 0; x < 256; ++x) {
+        const int2 t = exp_fx_entry(std::exp2(x / 256.0));
+        q[x] = (uint64_t)(uint32_t)t.x | (uint64_t)(uint32_t)t.y << 32;
+      }
+    }
+  } T;
+  return T.q;
 }
 
 struct Bump {
@@ -154,6 +225,9 @@ extern "C" CUSNA_API cusna_status cusna_saom_simulate_period_static(
   int kind[CUSNA_MAXEFF], cfn[CUSNA_MAXEFF];
   int fl = 0;
   bool has_dyn = false;
+  CounterSet cnt;
+  int pk[CUSNA_MAXEFF];
+  plan_counters(tid, k, false, nullptr, cnt, pk);
   for (int e = 0; e < k; ++e) {
     const int t = tid[e];
     kind[e] = K_GEN; cfn[e] = 0;
@@ -161,20 +235,17 @@ extern "C" CUSNA_API cusna_status cusna_saom_simulate_period_static(
     switch (t) {
       case 0: kind[e] = K_CNT; cfn[e] = 0; break;
       case 1: kind[e] = K_CNT; cfn[e] = 1; break;
-      case 2: kind[e] = K_CNT; cfn[e] = 2; fl |= F_PC_RI_CJ | F_PC_RI_RJ; break;
-      case 3: case 23: kind[e] = K_CNT; cfn[e] = 3; fl |= F_PC_RJ_CI; break;
+      case 2: kind[e] = K_CNT; cfn[e] = 2; break;
+      case 3: case 23: kind[e] = K_CNT; cfn[e] = 3; break;
       case 4: kind[e] = K_CNT; cfn[e] = 4; break;
       case 5: kind[e] = K_CNT; cfn[e] = 5; fl |= F_NEED_TP; break;
-      case 6: kind[e] = K_CNT; cfn[e] = 6; fl |= F_PC_RI_CJ | F_PC_RICIRJ; break;
+      case 6: kind[e] = K_CNT; cfn[e] = 6; break;
       case 8: kind[e] = K_CNT; cfn[e] = 7; break;
       case 10: case 14: case 15: case 16: case 17: case 18:
         kind[e] = K_STEP; fl |= F_HAS_STEP; break;
       case 19: kind[e] = K_STEP; fl |= F_HAS_STEP | F_NEED_RDEG; break;
       case 22: kind[e] = K_ZERO; break;
-      case 24: fl |= F_PC_RI_CJ; break;
-      case 26: fl |= F_PC_RI_RJ; break;
-      case 27: fl |= F_PC_CI_CJ; break;
-      case 28: fl |= F_PC_CI_RJ; break;
+      case 24: case 26: case 27: case 28: break;
       case 29: fl |= F_NEED_GW29; break;
       case 30: fl |= F_NEED_GW30; break;
       case 32:
@@ -188,19 +259,48 @@ extern "C" CUSNA_API cusna_status cusna_saom_simulate_period_static(
       default: kind[e] = K_ZERO; break;
     }
   }
+  for (int e = 0; e < k; ++e) cfn[e] |= pk[e] & ~0xFF;  // the counters each effect reads
   if (kb > 0 || has_dyn) fl |= F_HAS_Z;
   if (r->want_end_nets && r->a_ends) fl |= F_WANT_ENDS;
   if (!r->scores) fl |= F_NO_SCORES;  // no score sums without scores
 
   // ---- launch shape (as the autotuned entry points choose it) ------------
-  int dev = 0, sms = 0, smem_optin = 0;
+  int dev = 0, sms = 0, smem_optin = 0, smem_sm = 0;
   SCU(cudaGetDevice(&dev));
   SCU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   SCU(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  const bool need_tp = (fl & F_NEED_TP) != 0, need_gw = (fl & (F_NEED_GW29 | F_NEED_TP)) != 0;
+  SCU(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
+  const bool need_tp = (fl & F_NEED_TP) != 0, need_gw = (fl & F_NEED_GW29) != 0;
   const bool need_tq = (fl & F_NEED_GW30) != 0;
   LaunchShape best{};
   double best_score = -1.0;
+  // Which problems fit is a rule of its own, not of the kernel's footprint in
+  // this build: the in-rows' scratch is counted for the teams that a kernel of
+  // 128 registers (512 threads per SM) and scratch_rule_slice() bytes per team
+  // would keep resident. The launch below never has more teams than that.
+  double rule_score = -1.0;
+  size_t rule_teams = 0;
+  bool rule_cols_smem = false;
+  for (int G = 1; G <= 16; G *= 2)
+    for (int cs = 1; cs >= 0; --cs) {
+      const size_t sl = scratch_rule_slice(n, W, k, kb, nr, G, cs, need_tp, need_gw, need_tq);
+      for (int tpc = 1; tpc <= 16 && sl <= (size_t)smem_optin; tpc *= 2) {
+        const int threads = 32 * G * tpc;
+        if (threads > 512 || (G > 1 && tpc > 15) || sl * tpc > (size_t)smem_optin) continue;
+        const int per_sm = (int)std::min<size_t>(512 / threads, (size_t)smem_sm / (sl * tpc + 1024));
+        if (per_sm < 1) continue;
+        const double teams_sm = (double)per_sm * tpc, want_sm = std::max((double)M / sms, 1.0);
+        const double busy = (teams_sm < (double)M / sms ? teams_sm : want_sm) * G;
+        const double score = (busy < 48 ? busy : 48) * 100.0 - G - (cs ? 0.0 : 50.0) - tpc * 0.01;
+        if (score > rule_score) {
+          rule_score = score;
+          rule_cols_smem = cs;
+          rule_teams = (size_t)std::min<long long>(((long long)M + tpc - 1) / tpc,
+                                                   (long long)sms * per_sm) * tpc;
+        }
+      }
+    }
+  if (rule_score < 0) { set_last_error("no launch shape fits this n in shared memory"); return CUSNA_ERR_UNSUPPORTED; }
   for (int G = 1; G <= 16; G *= 2)
     for (int cs = 1; cs >= 0; --cs) {
       LaunchShape sh{};
@@ -245,15 +345,27 @@ extern "C" CUSNA_API cusna_status cusna_saom_simulate_period_static(
                oOffd = b.take((size_t)k * 4), oTab = b.take(8);
   const size_t oProb = b.take(sizeof(DevProblem)), oUnits = b.take(2 * sizeof(long long)),
                oCnt = b.take(sizeof(unsigned long long)), oFlag = b.take(sizeof(int));
-  const size_t teams = (size_t)best.ctas * best.teams_per_cta;
-  const size_t oCols = best.cols_in_smem ? 0 : b.take(teams * (size_t)W * n * 4);
-  if (b.off > kStaticScratchBytes) {
+  // (beside the fixed-point table and bounds below, which the rule does not count)
+  const size_t need = b.off + (rule_cols_smem ? 0 : rule_teams * bits);
+  const size_t oTabq = b.take(256 * 8), oBound = b.take((size_t)k * 8);
+  if (need > kStaticScratchBytes) {
     char buf[200];
     snprintf(buf, sizeof buf,
              "this problem needs %zu bytes of scratch; the no-allocation entry point holds %zu",
-             b.off, kStaticScratchBytes);
+             need, kStaticScratchBytes);
     set_last_error(buf);
     return CUSNA_ERR_UNSUPPORTED;
+  }
+  // as many CTAs as the array holds in-rows for
+  size_t oCols = 0;
+  if (!best.cols_in_smem) {
+    const size_t per_cta = (size_t)best.teams_per_cta * bits;
+    best.ctas = (int)std::min<size_t>(best.ctas, (kStaticScratchBytes + kStaticExtra - b.off) / per_cta);
+    if (best.ctas < 1) {
+      set_last_error("the no-allocation entry point's scratch holds no team of this problem");
+      return CUSNA_ERR_UNSUPPORTED;
+    }
+    oCols = b.take((size_t)best.ctas * per_cta);
   }
   auto U32 = [&](size_t o) { return (uint32_t *)(base + o); };
   auto I32 = [&](size_t o) { return (int *)(base + o); };
@@ -308,6 +420,11 @@ extern "C" CUSNA_API cusna_status cusna_saom_simulate_period_static(
   SCU(cudaMemcpyAsync(I32(oOffd), zeros, (size_t)k * 4, cudaMemcpyHostToDevice, s));
   SCU(cudaMemsetAsync(base + oTab, 0, 8, s));
 
+  SCU(cudaMemcpyAsync(base + oTabq, exp_table(), 256 * 8, cudaMemcpyHostToDevice, s));
+  bounds_kernel<<<k, 32, 0, s>>>(p->type_ids, I32(oDy), F64(oV), F64(oWt), F64(o1), F64(o2), I32(oZ0),
+                                 (double)p->zbar, kb, p->zmin, p->zmax, n, F64(oBound));
+  SCU(cudaGetLastError());
+
   DevProblem D;
   std::memset(&D, 0, sizeof D);
   D.n = n; D.W = W; D.k = k; D.kb = kb; D.nrate = nr; D.M = M;
@@ -325,14 +442,16 @@ extern "C" CUSNA_API cusna_status cusna_saom_simulate_period_static(
   D.vb = F64(oVb); D.od0 = p->od0; D.id0 = p->id0; D.bty = p->bty; D.rkind = p->rkind;
   D.ralpha = F64(oRa); D.ru = F64(oRu); D.act = I32(oAct); D.inact = U32(oIn);
   D.z0 = I32(oZ0); D.bkdist = I32(oBk);
-  D.x0T = U32(oX); D.x0cT = U32(oXc); D.simT = U32(oS); D.simcT = U32(oSc);
-  D.kdistT = U32(oK); D.permT = U32(oP); D.keepT = U32(oKp); D.forceT = U32(oF);
-  D.keepcT = U32(oKc); D.forcecT = U32(oFc);
+  D.x0r = U32(oX); D.x0c = U32(oXc); D.simr = U32(oS); D.simc = U32(oSc);
+  D.kdistr = U32(oK); D.permr = U32(oP); D.keepr = U32(oKp); D.forcer = U32(oF);
+  D.keepc = U32(oKc); D.forcec = U32(oFc);
   D.lam = p->lam; D.theta = p->theta; D.lamb = p->lamb; D.thetab = kb ? p->thetab : nullptr;
   D.prow = 1;
   D.ekind = I32(oKind); D.ecfn = I32(oCfn); D.eoffd = I32(oOffd); D.eofft = I32(oOffd);
+  D.cnt = cnt;
   D.tab = F64(oTab);
-  D.tab2 = nullptr;  // no lookup tables in this plan
+  D.tabq = (const uint64_t *)(base + oTabq);  // no lookup tables in this plan
+  D.ebound = F64(oBound);
   D.stats = r->stats; D.ntim = r->ntim; D.scores = r->scores; D.dist = r->dist;
   D.dist_stat = r->dist_stat; D.steps = r->steps;
   if (kb) { D.bdist = r->bdist; D.bscores = r->bscores; D.z_end = r->z_end; }
@@ -342,9 +461,10 @@ extern "C" CUSNA_API cusna_status cusna_saom_simulate_period_static(
   SCU(cudaMemcpyAsync(base + oProb, &D, sizeof D, cudaMemcpyHostToDevice, s));
   SCU(cudaMemcpyAsync(base + oUnits, units, sizeof units, cudaMemcpyHostToDevice, s));
   SCU(cudaMemsetAsync(base + oCnt, 0, sizeof(unsigned long long), s));  // work counter starts at 0
+  const Scratch sc{best.cols_in_smem ? nullptr : U32(oCols), nullptr, nullptr, bits / 4, 0};
   SCU(launch_period(best, (const DevProblem *)(base + oProb), (const long long *)(base + oUnits), 1,
                     (long long)M, (unsigned long long *)(base + oCnt),
-                    best.cols_in_smem ? nullptr : U32(oCols), nullptr, (size_t)W * n, s));
+                    sc, s));
   SCU(cudaStreamSynchronize(s));
   return CUSNA_OK;
 }
