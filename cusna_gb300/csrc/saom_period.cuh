@@ -88,7 +88,9 @@ __device__ void chain_finish(const Team &T, const DevProblem &P, const Slice &S,
     D.vmat = P.vmat; D.vb = P.vb; D.wtab = P.wtab; D.p1 = P.p1; D.p2 = P.p2;
     D.vmiss = P.vmiss; D.dyn = P.dyn; D.od0 = P.od0; D.id0 = P.id0; D.type_ids = P.type_ids;
     D.n = n; D.W = W; D.k = k; D.symflag = P.symflag;
-    network_stats_team(T, D, S.rows, S.cols, S.outdeg, S.indeg, S.red, P.stats + (size_t)c * k);
+    // S.red: 32 G + 64 doubles
+    network_stats_team(T, D, S.rows, S.cols, S.outdeg, S.indeg, S.red, (32 * T.G + 56) / kStatRow,
+                       P.stats + (size_t)c * k);
   }
   if (T.tl == 0) {
     if (P.dist) P.dist[c] = (int)dist;
