@@ -254,11 +254,25 @@ class SimPlan:
             pass
 
 
+def _u8(x):
+    """x != 0 as contiguous bytes of 0 and 1. Arrays that hold just that already
+    (bool, or uint8 up to 1) are passed as they are: for the 1000 networks of
+    100 actors of a goodness-of-fit call the comparison and the copy were 1.9 of 4.3 ms."""
+    if x is None:
+        return None
+    x = np.asarray(x)
+    if x.dtype == np.bool_:
+        return np.ascontiguousarray(x).view(np.uint8)
+    if x.dtype == np.uint8 and (x.size == 0 or x.max() <= 1):
+        return np.ascontiguousarray(x)
+    return np.ascontiguousarray(x != 0, dtype=np.uint8)
+
+
 def network_stats(a, n, k, type_ids, p1, p2, vmat, vmiss, dyn_flags, vb, od0, id0, wtab,
                   symflag) -> np.ndarray:
     """Statistics of one or more networks on the GPU (a: (n,n) or (M,n,n))."""
     lib = load_library()
-    A = np.ascontiguousarray(np.asarray(a) != 0, dtype=np.uint8)
+    A = _u8(a)
     single = A.ndim == 2
     if single:
         A = A[None]
@@ -289,11 +303,11 @@ def cross_stats(a_batch, wp, t, parm=0.0) -> np.ndarray:
     """Cross-network statistic of type t (33..37) of own networks a_batch
     ((n,n) or (M,n,n)) against the source predictor wp, on the GPU."""
     lib = load_library()
-    a = np.ascontiguousarray(np.asarray(a_batch) != 0, dtype=np.uint8)
+    a = _u8(a_batch)
     if a.ndim == 2:
         a = a[None]
     M, n = a.shape[0], a.shape[1]
-    w = np.ascontiguousarray(np.asarray(wp) != 0, dtype=np.uint8)
+    w = _u8(wp)
     out = np.zeros(M)
     st = lib.cusna_cross_stats(a.ctypes.data, w.ctypes.data, n, M, int(t), float(parm),
                                out.ctypes.data)
@@ -301,8 +315,6 @@ def cross_stats(a_batch, wp, t, parm=0.0) -> np.ndarray:
     return out
 
 
-def _u8(x):
-    return None if x is None else np.ascontiguousarray(np.asarray(x) != 0, dtype=np.uint8)
 
 
 def typed_stats(a_batch, etype, F, x0, keep=None, force=None, keepS=None, forceS=None,
@@ -348,7 +360,7 @@ def behavior_stats(z_batch, bty, xnet, bkdist, zbar, brange, bsimmean) -> np.nda
     z = np.ascontiguousarray(np.atleast_2d(np.asarray(z_batch, dtype=np.int32)))
     M, n = z.shape
     b = np.ascontiguousarray(np.asarray(bty, dtype=np.int32))
-    x = np.ascontiguousarray(np.asarray(xnet) != 0, dtype=np.uint8)
+    x = _u8(xnet)
     bk = None if bkdist is None else np.ascontiguousarray(np.asarray(bkdist, dtype=np.int32))
     out = np.zeros((M, len(b)))
     st = lib.cusna_behavior_stats_gpu(z.ctypes.data, n, M, len(b), b.ctypes.data, x.ctypes.data,
