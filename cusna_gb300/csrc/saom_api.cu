@@ -762,9 +762,11 @@ cusna_status fetch_outputs(Job &J) {
 
 // Chooses which two-path counters the chains hold as matrices. A popcount takes
 // W words per alter, a matrix one read per alter and, per toggle, one update for
-// each tie of the two actors: from kCountsMinW words on the matrices win (the figures
-// below), if the resident teams' matrices stay within
-// kCountsMaxBytes of device memory.
+// each tie of the two actors. They win where the chip is full of chains (1216 chains
+// with scores: n = 384 93 against 115 ms, n = 448 115 against 170, n = 225 no
+// difference), but not for rounds of a few hundred (512 chains of n = 300 without
+// scores: 15.0 against 13.1 ms), so the line is at kCountsMinW words; and only while
+// the resident teams' matrices stay within kCountsMaxBytes of device memory.
 constexpr int kCountsMinW = 12;
 constexpr size_t kCountsMaxBytes = (size_t)8 << 30;
 constexpr size_t kResidentTeams = 152 * 32;
