@@ -30,7 +30,7 @@
 namespace cusna {
 
 // ---- generated source --------------------------------------------------------
-// Each effect becomes the branch of change_stats32 / change_stats
+// Each effect becomes the branch of change_fixed / change_stats
 // (saom_kernel.cuh) that its kind selects, with the kind, count function,
 // type, creation/endowment type and interaction components as constants.
 // Offsets, theta and every table stay run-time values, so one compiled plan
@@ -171,7 +171,8 @@ void gen_cross(Gen &g, int e, int cfn, int ca) {
   else g.put("    const int c = cross_count(P, S, X, n, %d, S.eoffd[%d], 255, i, j);\n", cfn, e);
 }
 
-// jit_change_stats32<sfx> and jit_change_stats<sfx><TERMS> of one effect plan
+// jit_change_fixed<sfx>, jit_sums_add<sfx> and jit_change_stats<sfx><TERMS> of one
+// effect plan
 void gen_functions(Gen &g, const JitPlan &J, const std::string &sfx, bool multi) {
   const int k = (int)J.kind.size();
   const char *x = sfx.c_str();
@@ -612,9 +613,8 @@ Compiled compile_spec(const std::string &spec) {
   for (int q = 0; q < 2; ++q) N.add_name(prog, kNames[q]);
   // CUSNA_JIT_MINB: resident 256-thread CTAs per SM the register budget of
   // the 256-thread instantiation allows (default 2: 128 registers). Measured
-  // on the n=200, 4096-chain workload: with the double-float score sums 2
-  // gives 90.3 ms against 92.9 for 3 (80 registers, which spill); the earlier
-  // float32 sums ran best with 3.
+  // on the n=200, 4096-chain workload: 2 gives 67 ms, 3 (80 registers) 80 and 4
+  // (64 registers) 94.
   const std::string minb = compile_options_text();
   const char *opts[] = {"--gpu-architecture=sm_103a", "-std=c++17", "--fmad=false",
                         "-default-device", "-DLIBCUSNA_BUILD", minb.c_str()};

@@ -1,10 +1,10 @@
 // saom_jit.h -- the period kernel specialised to one effect plan, compiled at
 // run time with NVRTC (saom_jit.cu).
 //
-// The float32 pass over the alters evaluates every effect of the model for
+// The pass over the alters evaluates every effect of the model for
 // every alter. The library's kernel reads each effect's kind from shared memory
 // and dispatches per alter; the specialised kernel has the effect plan written
-// out as straight-line code (the same float32 operations in the same order, so
+// out as straight-line code (the same operations, so
 // every output is bit-identical to the library kernel's). A plan is compiled in
 // a background thread once it has been used a few times (CUSNA_JIT_AFTER,
 // default 3); until then, and whenever NVRTC is unavailable, the library kernel
