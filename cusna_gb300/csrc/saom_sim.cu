@@ -18,7 +18,7 @@ namespace cusna {
 // columns by ballots over 32 x 32 bits of the rows), then the same statistic code
 // as the period kernel. With one warp per network, whose lane 0 formed and added
 // every order-dependent term, 1000 networks of 100 actors and 11 statistics took
-// 2.5 ms of the kernel.
+// 2.5 ms of the kernel; so 0.59.
 constexpr int kNetWarps = 4;
 __global__ void __launch_bounds__(32 * kNetWarps) netstats_kernel(
     const uint8_t *__restrict__ a_batch, int M, StatDesc D, double *out, int rows) {
