@@ -94,21 +94,20 @@ def smem_bytes_per_network_ministep(n, W):
 
 
 # Warp-instructions the period kernel executes per network ministep, from ncu
-# captures of the bench's own launches (smsp__inst_executed.sum over the
-# launch's 6,557,430 network ministeps; n=200, k=8, 4096 chains), keyed by
-# workload, kernel specialised to the effect plan, and warps per chain of the
-# tuned shape (one warp per chain, columns in shared memory or in global
-# scratch: 44,515,682,075 per launch), and per ministep (network and
-# behaviour, 6,146,609 a launch) of the n=1000 co-evolution workload's
-# specialised kernel (16 warps per chain: 186,772,337,633 per launch; 8:
-# 153,974,457,454).
-INST_PER_MINISTEP = {("c2", True, 1): 6789.0, ("c4", True, 16): 30387.0, ("c4", True, 8): 25050.0}
+# captures (smsp__inst_executed.sum over the launch's ministeps; n=200, k=8, 4096
+# chains, one warp per chain: 29,522,698,877 over 6,552,142), keyed by workload,
+# kernel specialised to the effect plan, and warps per chain of the tuned shape;
+# and per ministep (network and behaviour) of the n=1000 co-evolution workload's
+# specialised kernel (152 chains, 910,095 ministeps: 19,326,942,106 with 16 warps
+# per chain, 12,697,377,001 with 8, 9,986,250,617 with 4, 8,834,848,175 with 2).
+INST_PER_MINISTEP = {("c2", True, 1): 4506.0, ("c4", True, 16): 21236.0, ("c4", True, 8): 13952.0,
+                     ("c4", True, 4): 10973.0, ("c4", True, 2): 9708.0}
 # DRAM bytes of one period-kernel launch of the bench workload (the problem, its
 # tables, the column bitsets' global scratch and the outputs), measured by ncu
-# on the bench's own timed launch (dram__bytes_read.sum 5,991,168 +
-# dram__bytes_write.sum 8,859,392 at 4096 chains, specialised kernel, one warp
+# on a launch of that workload and shape (dram__bytes_read.sum 1,278,464 +
+# dram__bytes_write.sum 4,920,832 at 4096 chains, specialised kernel, one warp
 # per chain, 16 chains per CTA).
-DRAM_BYTES_PER_LAUNCH = {("c2", 4096): 5991168.0 + 8859392.0}
+DRAM_BYTES_PER_LAUNCH = {("c2", 4096): 1278464.0 + 4920832.0}
 
 
 def period_roofline(workload, n, W, k, net_steps, kernel_ms, sm_count, clk, specialised=True,
@@ -141,8 +140,8 @@ def period_roofline(workload, n, W, k, net_steps, kernel_ms, sm_count, clk, spec
     return {"bound": "issue", "achieved": achieved, "peak": peak,
             "unit": "G warp-instructions/s", "frac": achieved / peak if achieved else None,
             "traffic": traffic,
-            "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of the bench's "
-                              "timed launch (4096 chains)",
+            "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of a launch of "
+                              "this workload and shape (4096 chains)",
             "kernel_ms": kernel_ms, "network_ministeps_per_s": rate,
             "inst_per_ministep": ipm, "sm_mhz": mhz,
             "peak_source": "4 warp-instructions per cycle per SM x SMs x sampled SM clock",
