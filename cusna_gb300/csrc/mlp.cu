@@ -188,11 +188,10 @@ __device__ __forceinline__ void epilogue_store(int m, int n, float v, int ldc,
 }
 
 // C[M x N] = A[M x K] . B[N x K]^T (bf16 operands, fp32 accumulation), a CTA
-// per 128 x BN tile (BN = 16, 32 or 64), 128 threads. EPI_STORE products may split
-// K over a cluster (gridDim.z = its size): each CTA multiplies its share of the
-// chunks, and the accumulators are added over the cluster's shared memory, each
-// CTA a share of the rows, in rank order. The K
-// chunks stream through kStages shared-memory stages with cp.async: chunk c +
+// per 128 x BN tile (BN = 16, 32 or 64), 128 threads. Every tile adds its products
+// along K whole and in order, whatever BN: a weight gradient cut into shares of K
+// has other roundings, which a few training steps carry from 1e-6 to 7e-5 of the
+// parameters' moments. The K chunks stream through kStages shared-memory stages with cp.async: chunk c +
 // kStages - 1 is in flight while the tensor cores multiply chunk c. The host
 // checks K % 16 == 0, 16-byte aligned operand rows and BN. *err receives 1 if
 // an mbarrier wait gave up.
@@ -207,7 +206,6 @@ __global__ void __launch_bounds__(128) gemm_tc05(
   __shared__ uint32_t tmem_slot;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int m0 = blockIdx.y * kBM, n0 = blockIdx.x * BN;
-  const int split = EPI == EPI_STORE ? (int)gridDim.z : 1;
   const uint32_t a_bytes = kBM * kKC * 2, b_bytes = (uint32_t)BN * kKC * 2;
   const uint32_t stage_bytes = a_bytes + b_bytes, sbase = smem_u32(dsm);
   // tensor memory: a power of two of at least 32 columns, one f32 column per
@@ -231,15 +229,12 @@ __global__ void __launch_bounds__(128) gemm_tc05(
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_slot;
   const uint32_t idesc = mma_idesc(kBM, BN, A_MN, B_MN);
-  // this CTA's chunks: cb .. cb + nchunks - 1
-  const int all = (K + kKC - 1) / kKC, per = (all + split - 1) / split;
-  const int cb = split > 1 ? (int)blockIdx.z * per : 0;
-  const int nchunks = max(0, min(per, all - cb));
+  const int nchunks = (K + kKC - 1) / kKC;
   const int lg_nb = __ffs(BN >> 3) - 1;   // BN is a power of two
   auto issue = [&](int c) {
     const uint32_t sa = sbase + (uint32_t)(c % kStages) * stage_bytes;
-    stage_tile<A_MN>(A, lda, m0, M, (cb + c) * kKC, K, 4, sa);   // 128 rows: 16 row groups
-    stage_tile<B_MN>(B, ldb, n0, N, (cb + c) * kKC, K, lg_nb, sa + a_bytes);
+    stage_tile<A_MN>(A, lda, m0, M, c * kKC, K, 4, sa);   // 128 rows: 16 row groups
+    stage_tile<B_MN>(B, ldb, n0, N, c * kKC, K, lg_nb, sa + a_bytes);
   };
   // the first kAhead chunks in flight
   for (int c = 0; c < kAhead; ++c) {
@@ -255,7 +250,7 @@ __global__ void __launch_bounds__(128) gemm_tc05(
     if (tid == 0) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t sa = sbase + (uint32_t)(c % kStages) * stage_bytes, sb = sa + a_bytes;
-      const int left = K - (cb + c) * kKC, steps = left >= kKC ? 4 : left / 16;
+      const int left = K - c * kKC, steps = left >= kKC ? 4 : left / 16;
       for (int s = 0; s < steps; ++s) {
         const uint64_t da = step_desc<A_MN>(sa, kBM, s);
         const uint64_t db = step_desc<B_MN>(sb, BN, s);
@@ -288,29 +283,9 @@ __global__ void __launch_bounds__(128) gemm_tc05(
                    (uint32_t)(((nchunks - 1) / kStages) & 1));
   ok = __syncthreads_and(ok) != 0;
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if (!ok && lane == 0) atomicExch(err, 1);
-  if (EPI == EPI_STORE && split > 1) {
-    // the CTA's tile to its shared memory (the stages are free), a row a thread
-    float *tile = reinterpret_cast<float *>(dsm), *mine = tile + tid * (BN + 1);
-    for (int c0 = 0; c0 < BN; c0 += 16) {
-      uint32_t r[16];
-      const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0;
-      tmem_load16(taddr, r);
-#pragma unroll
-      for (int j = 0; j < 16; ++j) mine[c0 + j] = ok && nchunks > 0 ? __uint_as_float(r[j]) : 0.f;
-    }
-    const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
-    cl.sync();
-    const int rows = kBM / split, r0 = (int)blockIdx.z * rows;
-    for (int x = tid; x < rows * BN; x += 128) {
-      const int row = r0 + x / BN, col = x % BN;
-      if (m0 + row >= M || n0 + col >= N) continue;
-      float v = 0.f;
-      for (int q = 0; q < split; ++q) v += *cl.map_shared_rank(tile + row * (BN + 1) + col, q);
-      Cf[(size_t)(m0 + row) * ldc + n0 + col] = v;
-    }
-    cl.sync();   // no CTA leaves while its tile is read
-  } else if (ok) {
+  if (!ok) {
+    if (lane == 0) atomicExch(err, 1);
+  } else {
     // accumulator rows to the warp's 32 x 33 staging area in shared memory (the
     // stages are free now), then out a row at a time, lane = column
     float *stg = reinterpret_cast<float *>(dsm) + warp * 32 * 33;
@@ -608,33 +583,21 @@ cudaError_t gemm(const __nv_bfloat16 *A, int lda, const __nv_bfloat16 *B, int ld
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
-  // Few tiles leave the chip idle: weight gradients (K = the batch) split K over a
-  // cluster of up to 8 CTAs, and tiles are halved, which shares the epilogue among
-  // more CTAs, as long as every CTA still has an SM of its own. An epoch of 12
-  // steps at batch 1024, width 256: 1.61 ms with 2 to 32 CTAs a product, 1.09 so.
-  const int tm = (M + kBM - 1) / kBM, chunks = (K + kKC - 1) / kKC;
-  int BN = tile_n(N), S = 1;
-  auto ctas = [&](int bn, int split) { return (long long)tm * ((N + bn - 1) / bn) * split; };
-  if (EPI == EPI_STORE)
-    while (S < 8 && 2 * S <= chunks && ctas(BN, 2 * S) <= sms) S *= 2;
-  while (BN > 16 && ctas(BN / 2, S) <= sms) BN /= 2;
+  // Few tiles leave the chip idle: tiles are halved, which shares the epilogue
+  // among more CTAs, as long as every CTA still has an SM of its own. An
+  // epoch of 12 steps at batch 1024, width 256: 1.56 ms with 2 to 32 CTAs a product,
+  // 1.31 so.
+  const int tm = (M + kBM - 1) / kBM;
+  int BN = tile_n(N);
+  while (BN > 16 && (long long)tm * ((N + BN / 2 - 1) / (BN / 2)) <= sms) BN /= 2;
   const size_t smem =
       (size_t)kStages * ((size_t)kBM * kKC * 2 + (size_t)BN * kKC * 2) + (size_t)kSlack;
   const void *fn = (const void *)gemm_tc05<EPI, A_MN, B_MN>;
   if ((e = raise_dyn_smem(fn, smem)) != cudaSuccess) return e;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((N + BN - 1) / BN, tm, S);
-  cfg.blockDim = dim3(128);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = at.val.clusterDim.y = 1;
-  at.val.clusterDim.z = S;
-  cfg.attrs = &at;
-  cfg.numAttrs = S > 1 ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, gemm_tc05<EPI, A_MN, B_MN>, A, lda, B, ldb, M, N, K, BN, bias, Zin,
-                            Cf, Cb, Zout, ldc, w.err);
+  const dim3 grid((N + BN - 1) / BN, tm);
+  gemm_tc05<EPI, A_MN, B_MN><<<grid, 128, smem, st>>>(A, lda, B, ldb, M, N, K, BN, bias, Zin, Cf,
+                                                      Cb, Zout, ldc, w.err);
+  return cudaGetLastError();
 }
 
 bool dims_ok(int n_in, int H, int n_out) {
