@@ -101,13 +101,10 @@ __device__ __forceinline__ void chain_init(const Team &T, const DevProblem &P, c
       const int cls = fx_class(kind, S.ecfn[e] & 0xFF, S.tid[e], S.ety[e]);
       double bound = P.ebound[e];
       int sd = fx_scale(bound);
-      if (S.tid[e] == 32 && kind != K_ZERO) {   // products: bounds and scales of the components
+      if (S.tid[e] == 32 && kind != K_ZERO) {   // products: the components' bounds
         bound = __dmul_rn(S.dstar[S.i0[e]], S.dstar[S.i1[e]]);
-        sd = S.esd[S.i0[e]] + S.esd[S.i1[e]] - 64;
-        if (S.i2[e] >= 0) {
-          bound = __dmul_rn(bound, S.dstar[S.i2[e]]);
-          sd += S.esd[S.i2[e]] - 64;
-        }
+        if (S.i2[e] >= 0) bound = __dmul_rn(bound, S.dstar[S.i2[e]]);
+        sd = fx_scale(bound);
       }
       S.dstar[e] = bound;
       S.esd[e] = sd;

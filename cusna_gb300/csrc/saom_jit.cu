@@ -216,9 +216,14 @@ void gen_functions(Gen &g, const JitPlan &J, const std::string &sfx, bool multi)
         else std::snprintf(b, sizeof b, "(int64_t)0");
         return std::string(b);
       };
-      g.put("    int64_t p = __mul64hi(%s, %s);\n", mag(J.i0[e]).c_str(), mag(J.i1[e]).c_str());
-      if (J.i2[e] >= 0) g.put("    p = __mul64hi(p, %s);\n", mag(J.i2[e]).c_str());
-      g.s += "    const uint64_t m = (uint64_t)(p + (1LL << 62));\n";
+      const int a = J.i0[e], b = J.i1[e], c = J.i2[e];
+      if (c < 0)
+        g.put("    const uint64_t m = (1ull << 62) + product_fx(%s, %s,\n"
+              "        S.esd[%d] + S.esd[%d] - 62, S.esd[%d]);\n", mag(a).c_str(), mag(b).c_str(), a, b, e);
+      else
+        g.put("    const uint64_t m = (1ull << 62) + product_fx(%s, %s, %s,\n"
+              "        S.esd[%d] + S.esd[%d] + S.esd[%d] - 124, S.esd[%d]);\n", mag(a).c_str(),
+              mag(b).c_str(), mag(c).c_str(), a, b, c, e);
     } else if (cfn == 16) {
       g.put("    const uint64_t m = gw_fixed(S, X, n, W, %d, %d, j, aij);\n", e, t);
     } else {

@@ -710,6 +710,18 @@ __device__ __forceinline__ int64_t base_fx(uint64_t thr, int cls) {
   return signed_fx(thr >> 2, (cls >> 8) ^ 1);
 }
 
+// The magnitude of a product from its components' a, b and (of three) c, each below
+// 2^62 at its scale: ab 2^-62 has scale sa + sb - 62 and is shifted up to the
+// product's own scale, which follows from the product of the bounds (fx_scale; at
+// most 2 above), so that |theta| 2^(110 - sd) stays below 2^63 as for any other effect.
+__device__ __forceinline__ uint64_t product_fx(int64_t a, int64_t b, int have, int want) {
+  const int up = want > have ? (want - have < 63 ? want - have : 63) : 0;
+  return (uint64_t)__mul64hi((int64_t)((uint64_t)a << 1), (int64_t)((uint64_t)b << 1)) << up;
+}
+__device__ __forceinline__ uint64_t product_fx(int64_t a, int64_t b, int64_t c, int have, int want) {
+  return product_fx(__mul64hi((int64_t)((uint64_t)a << 1), (int64_t)((uint64_t)b << 1)), c, have, want);
+}
+
 // Magnitudes of toggling i -> j for the effects of classes FX_CNT (the count) and
 // FX_REAL (|d| 2^sd + 2^62) into v, 0 for an effect that its creation or
 // endowment type rules out, and the predictor without its sign (f_j = delta
@@ -776,9 +788,10 @@ __device__ __forceinline__ int64_t change_fixed(const DevProblem &P, const Slice
         if (cl == FX_UNI) return (int64_t)(S.stepq[4 * q] - (1ull << 62));
         return cl == FX_REAL && v[q] ? (int64_t)(v[q] - (1ull << 62)) : 0;
       };
-      int64_t p = __mul64hi(mag(S.i0[e]), mag(S.i1[e]));
-      if (S.i2[e] >= 0) p = __mul64hi(p, mag(S.i2[e]));
-      m = (uint64_t)(p + (1LL << 62));
+      const int a = S.i0[e], b = S.i1[e], c = S.i2[e], have = S.esd[a] + S.esd[b] - 62;
+      m = (c < 0 ? product_fx(mag(a), mag(b), have, S.esd[e])
+                 : product_fx(mag(a), mag(b), mag(c), have + S.esd[c] - 62, S.esd[e])) +
+          (1ull << 62);
     } else if (cfn == 16) {
       m = gw_fixed(S, X, n, P.W, e, S.tid[e], j, aij);
     } else {
