@@ -1100,6 +1100,7 @@ static __device__ void run_chain(const Team &T, const DevProblem &P, const Slice
         dist += (uint32_t)aij_star == ((x0 >> (j & 31)) & 1u) ? chg : -chg;
     }
     if (T.tl == 0) trace_put<VALID>(P, c, ms - 1, i, jstar, dist - dist0);
+    if (P.nrate > 0) T.sync();   // the degrees below are the toggled ones (toggle_tie's lanes)
     if (P.nrate > 0 && T.tl == 0) {
       for (int q = 0; q < P.nrate; ++q) {
         const int rk = S.rkind[q];
