@@ -94,7 +94,7 @@ __device__ __forceinline__ void chain_init(const Team &T, const DevProblem &P, c
   if (T.tl == 0) {
     // fixed-point scales, classes and parameters; the pass over the alters needs
     // every |f_j| < 2^14 (S.fx[1]), else the chain runs on the float64 path
-    int64_t f0 = 0;
+    uint64_t f0 = 0;
     double range = 0.0;
     for (int e = 0; e < k; ++e) {
       const int kind = S.ekind[e];
@@ -115,12 +115,12 @@ __device__ __forceinline__ void chain_init(const Team &T, const DevProblem &P, c
     if (in_range)
       for (int e = 0; e < k; ++e) {
         S.thq[e] = theta_fx(S.th[e], S.ecls[e] & 0xFF, S.esd[e]);
-        if ((S.ecls[e] & 0xFF) == FX_DELTA) f0 += (int64_t)S.thq[e];
+        if ((S.ecls[e] & 0xFF) == FX_DELTA) f0 += S.thq[e];
         // the part of a real magnitude's 2^62, for every alter alike
         if ((S.ecls[e] & 0xFF) == FX_UNI || ((S.ecls[e] & 0xFF) == FX_REAL && S.ety[e] == 0))
-          f0 += base_fx(S.thq[e], S.ecls[e]);
+          f0 += (uint64_t)base_fx(S.thq[e], S.ecls[e]);
       }
-    S.fx[0] = f0;
+    S.fx[0] = (int64_t)f0;
     S.fx[1] = in_range;
   }
   for (int x = T.tl; x < n; x += L) {
@@ -508,36 +508,36 @@ static __device__ __noinline__ void lse_float64(const Team T, const DevProblem &
 
 // Adds alter j's weight W and magnitudes v to the lane's accumulators.
 template <int V>
-__device__ __forceinline__ void sums_add(const Slice &S, int k, int64_t (&acc)[V], uint64_t W,
+__device__ __forceinline__ void sums_add(const Slice &S, int k, uint64_t (&acc)[V], uint64_t W,
                                          int aij, const uint64_t *v) {
-  const int64_t wd = signed_fx(W, aij);
+  const uint64_t wd = (uint64_t)signed_fx(W, aij);
   const uint64_t w6 = W << 6;
-  acc[0] += (int64_t)W;
+  acc[0] += W;
   acc[1] += wd;
 #pragma unroll
   for (int e = 0; e < V - 2; ++e) {
     if (e >= k) continue;
     const int cls = S.ecls[e] & 0xFF;
     if (cls == FX_CNT) {
-      acc[2 + e] += wd * (int64_t)v[e];
+      acc[2 + e] += wd * v[e];
     } else if (cls == FX_REAL) {
-      acc[2 + e] += signed_fx(mulhi_fx(w6, v[e]), aij);
+      acc[2 + e] += (uint64_t)signed_fx(mulhi_fx(w6, v[e]), aij);
     }
   }
 }
 
 // The warp's sums: afterwards lane q holds quantity q's total as lo + 2^48 hi.
 template <int V>
-__device__ __forceinline__ void sums_reduce(const int64_t (&acc)[V], int lane, int64_t &lo, int &hi) {
+__device__ __forceinline__ void sums_reduce(const uint64_t (&acc)[V], int lane, int64_t &lo, int &hi) {
   lo = 0;
   hi = 0;
 #pragma unroll
   for (int q = 0; q < V; ++q) {
     if (!((CUSNA_FX_MASK >> q) & 1u)) continue;
-    const uint64_t a = (uint64_t)acc[q];
+    const uint64_t a = acc[q];
     const unsigned s0 = __reduce_add_sync(kFull, (unsigned)a & 0xFFFFFFu);
     const unsigned s1 = __reduce_add_sync(kFull, (unsigned)(a >> 24) & 0xFFFFFFu);
-    const int s2 = __reduce_add_sync(kFull, (int)(acc[q] >> 48));
+    const int s2 = __reduce_add_sync(kFull, (int)((int64_t)a >> 48));
     if (lane == q) {
       lo = (int64_t)s0 + ((int64_t)s1 << 24);
       hi = s2;
@@ -627,7 +627,7 @@ static __device__ __noinline__ void scores_flush(const ScoreRing R, const int *e
         __dmul_rn(__dadd_rn((double)lo, __dmul_rn((double)hi, 281474976710656.0)), inv),
         __dmul_rn(pow2(58), back));
     // (a magnitude of 0 marks one that the type rules out)
-    const double ds = m ? __dmul_rn(__dmul_rn(dl, (double)(m - (1LL << 62))), back) : 0.0;
+    const double ds = m ? __dmul_rn(__dmul_rn(dl, (double)(int64_t)((uint64_t)m + kMinus62)), back) : 0.0;
     return __dsub_rn(ds, mean);
   };
   for (int e0 = 0; e0 < k; e0 += 8) {   // two effects at once: their chains overlap
@@ -710,7 +710,7 @@ __device__ __forceinline__ int alter_pass(const Team &T, const DevProblem &P, co
 #else
   const int KS = k;
 #endif
-  int64_t acc[V];
+  uint64_t acc[V];
 #pragma unroll
   for (int q = 0; q < V; ++q) acc[q] = 0;
   int fmax = 0;
@@ -752,7 +752,7 @@ __device__ __forceinline__ int alter_pass(const Team &T, const DevProblem &P, co
       uint64_t W = exp_fx(f, sh, S.etab);
       if (!ok) W = 0;
       if (stay) {
-        acc[0] += (int64_t)W;
+        acc[0] += W;
       } else {
 #if defined(CUSNA_JIT_SPEC)
         jit_sums_add(acc, W, aij, v);
@@ -859,7 +859,8 @@ __device__ __forceinline__ int net_choice(const Team &T, const DevProblem &P, co
     if (ranged)
       for (int e = 0; e < k; ++e)
         if ((S.ecls[e] & 0xFF) == FX_UNI)
-          X.f0 += term_fx(S.thq[e], S.ecls[e], S.stepq[4 * e]);
+          X.f0 = (int64_t)((uint64_t)X.f0 +
+                           (uint64_t)term_fx(S.thq[e], S.ecls[e], S.stepq[4 * e]));
   }
 
   // ---- one pass over the alters (alter_pass) -------------------------------

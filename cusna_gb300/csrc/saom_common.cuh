@@ -289,10 +289,15 @@ __host__ __device__ __forceinline__ uint64_t mulhi_fx(uint64_t a, uint64_t b) {
 #endif
 }
 
-// x, or -x for neg = 1. Written with the bits' complement: subtractions and
-// negations of 64-bit values inside a chain of additions lost a borrow in code
-// compiled for sm_103a (nvcc 13.0) when the subtracted value's low word was 0, so
-// the fixed-point code adds only.
+// -2^62: taken off a magnitude by an addition.
+constexpr uint64_t kMinus62 = 3ull << 62;
+
+// x, or -x for neg = 1. Written with the bits' complement: the negation 0 - (a - b)
+// of a difference inside a chain of additions loses a borrow in code compiled for
+// sm_103a (nvcc 13.0) when low words are 0 (27,296 of 65,536 sums wrong, in unsigned
+// arithmetic throughout, so no undefined behaviour enters; a - b and b - a in its
+// place, or this form, 0 wrong). The fixed-point code therefore negates here only,
+// and its sums, which may wrap on the way, are unsigned.
 __host__ __device__ __forceinline__ int64_t signed_fx(uint64_t x, int neg) {
   const uint32_t s = 0u - (uint32_t)neg;
   return (int64_t)((x ^ ((uint64_t)s << 32 | s)) + (uint32_t)neg);
@@ -311,17 +316,18 @@ __host__ __device__ __forceinline__ uint64_t exp_fx(int64_t f, int sh, const int
   // N = round(f 256/ln2): 256/ln2 = 369.3299304675746 at 2^-20
   const int N = (int)(((int64_t)fh * 387270501 + ((int64_t)1 << 33)) >> 34);
   // ln2/256 at 2^-62
-  const int64_t r = (int64_t)((uint64_t)f << 16) + (int64_t)N * -12486629536330718LL;
+  const int64_t r =
+      (int64_t)(((uint64_t)f << 16) + (uint64_t)(int64_t)N * (uint64_t)-12486629536330718LL);
   const int s = (int)(r >> 22);    // scale 2^-40
   const float rf = (float)s * 9.094947017729282e-13f;
   const int c3 = (int)(rf * rf * rf * (rf * 0.041666668f + 0.16666667f) * 1.152921504606847e18f);
-  const int64_t e = r + (((int64_t)s * s) >> 19) + ((int64_t)c3 << 2);   // c3 at 2^-60
+  const int64_t e = r + (((int64_t)s * s) >> 19) + (int64_t)c3 * 4;   // c3 at 2^-60
   const int2 t = tab[N & 255];
-  const int64_t T = ((int64_t)t.x << 32) + t.y;
+  const int64_t T = (int64_t)((uint64_t)(uint32_t)t.x << 32) + t.y;
   const int eh = (int)(e >> 32);
   const uint32_t el = (uint32_t)e;
   const int64_t lowp = (int64_t)t.x * el + (int64_t)t.y * eh;
-  const uint64_t m = (uint64_t)(T + (((int64_t)t.x * eh) << 2) + (lowp >> 30));
+  const uint64_t m = (uint64_t)(T + (int64_t)t.x * eh * 4 + (lowp >> 30));
   int k = 17 - (N >> 8) + sh;      // one less than the shift, for the rounding
   if (k > 62) return 0;
   if (k < 0) k = 0;                // out of range: the caller repeats with a larger sh

@@ -183,7 +183,7 @@ void gen_functions(Gen &g, const JitPlan &J, const std::string &sfx, bool multi)
   gen_shape(g, J);
   g.s += "  (void)n; (void)W; (void)i; (void)aji; (void)v;\n";
   gen_counts(g, J);
-  g.s += "  int64_t f = X.f0;\n";
+  g.s += "  uint64_t f = (uint64_t)X.f0;\n";
   for (int e = 0; e < k; ++e) {
     const int kind = J.kind[e], pk = J.cfn[e], cfn = pk & 0xFF, ca = (pk >> 8) & 0xFF, t = J.tid[e];
     const int cls = fx_class(kind, cfn, t, J.ety[e]);
@@ -196,8 +196,8 @@ void gen_functions(Gen &g, const JitPlan &J, const std::string &sfx, bool multi)
       if (off) g.put("    const int m = %s ? 0 : c;\n", off);
       else g.s += "    const int m = c;\n";
       g.put("    v[%d] = (uint64_t)m;\n", e);
-      if (kind == K_CNT && cfn == 1) g.put("    f += m ? (int64_t)S.thq[%d] : 0;\n  }\n", e);
-      else g.put("    f += (int64_t)S.thq[%d] * m;\n  }\n", e);
+      if (kind == K_CNT && cfn == 1) g.put("    f += m ? S.thq[%d] : 0;\n  }\n", e);
+      else g.put("    f += S.thq[%d] * (uint32_t)m;\n  }\n", e);
       continue;
     }
     if (kind == K_LOOK) {
@@ -210,9 +210,9 @@ void gen_functions(Gen &g, const JitPlan &J, const std::string &sfx, bool multi)
         const int cl = fx_class(J.kind[q], J.cfn[q] & 0xFF, J.tid[q], J.ety[q]);
         char b[128];
         if (cl == FX_DELTA) std::snprintf(b, sizeof b, "((int64_t)1 << S.esd[%d])", q);
-        else if (cl == FX_CNT) std::snprintf(b, sizeof b, "((int64_t)v[%d] << S.esd[%d])", q, q);
-        else if (cl == FX_UNI) std::snprintf(b, sizeof b, "(int64_t)(S.stepq[%d] - (1ull << 62))", 4 * q);
-        else if (cl == FX_REAL) std::snprintf(b, sizeof b, "(v[%d] ? (int64_t)(v[%d] - (1ull << 62)) : 0)", q, q);
+        else if (cl == FX_CNT) std::snprintf(b, sizeof b, "(int64_t)(v[%d] << S.esd[%d])", q, q);
+        else if (cl == FX_UNI) std::snprintf(b, sizeof b, "(int64_t)(S.stepq[%d] + kMinus62)", 4 * q);
+        else if (cl == FX_REAL) std::snprintf(b, sizeof b, "(v[%d] ? (int64_t)(v[%d] + kMinus62) : 0)", q, q);
         else std::snprintf(b, sizeof b, "(int64_t)0");
         return std::string(b);
       };
@@ -231,28 +231,28 @@ void gen_functions(Gen &g, const JitPlan &J, const std::string &sfx, bool multi)
             "    const uint64_t m = real_fx(aij ? -d : d, S.esd[%d]);\n", e, gen_cnt_arg(ca).c_str(), e);
     }
     char tb[96];
-    std::snprintf(tb, sizeof tb, "term_fx(S.thq[%d], S.ecls[%d], m)", e, e);
+    std::snprintf(tb, sizeof tb, "(uint64_t)term_fx(S.thq[%d], S.ecls[%d], m)", e, e);
     if (off) {
-      g.put("    v[%d] = %s ? 0 : m;\n    if (!(%s)) f += %s + base_fx(S.thq[%d], S.ecls[%d]);\n  }\n", e,
+      g.put("    v[%d] = %s ? 0 : m;\n    if (!(%s)) f += %s + (uint64_t)base_fx(S.thq[%d], S.ecls[%d]);\n  }\n", e,
             off, off, tb, e, e);
     } else {
       g.put("    v[%d] = m;\n    f += %s;\n  }\n", e, tb);
     }
   }
-  g.s += "  return f;\n}\n";
+  g.s += "  return (int64_t)f;\n}\n";
   // the score sums (sums_add)
-  g.put("template <int V>\n__device__ __forceinline__ void jit_sums_add%s(int64_t (&acc)[V], uint64_t W, int aij,\n"
+  g.put("template <int V>\n__device__ __forceinline__ void jit_sums_add%s(uint64_t (&acc)[V], uint64_t W, int aij,\n"
         "    const uint64_t *v) {\n"
-        "  const int64_t wd = signed_fx(W, aij);\n  const uint64_t w6 = W << 6;\n"
-        "  (void)v; (void)w6;\n  acc[0] += (int64_t)W;\n  acc[1] += wd;\n", x);
+        "  const uint64_t wd = (uint64_t)signed_fx(W, aij);\n  const uint64_t w6 = W << 6;\n"
+        "  (void)v; (void)w6;\n  acc[0] += W;\n  acc[1] += wd;\n", x);
   for (int e = 0; e < k; ++e) {
     const int cfn = J.cfn[e] & 0xFF, cls = fx_class(J.kind[e], cfn, J.tid[e], J.ety[e]);
     if (cls == FX_CNT && J.kind[e] == K_CNT && cfn == 1)
       g.put("  acc[%d] += v[%d] ? wd : 0;\n", 2 + e, e);
     else if (cls == FX_CNT)
-      g.put("  acc[%d] += wd * (int64_t)(uint32_t)v[%d];\n", 2 + e, e);
+      g.put("  acc[%d] += wd * (uint32_t)v[%d];\n", 2 + e, e);
     else if (cls == FX_REAL)
-      g.put("  acc[%d] += signed_fx(mulhi_fx(w6, v[%d]), aij);\n", 2 + e, e);
+      g.put("  acc[%d] += (uint64_t)signed_fx(mulhi_fx(w6, v[%d]), aij);\n", 2 + e, e);
   }
   g.s += "}\n";
   // float64 evaluation (change_stats): the chosen alter and uncertified choices
@@ -341,7 +341,7 @@ std::string jit_multi_spec_source(const std::vector<JitPlan> &nets) {
   for (int d = 0; d < D; ++d)
     g.put("    case %d: return jit_change_fixed_n%d(P, S, X, j, aij, aji, v);\n", d, d);
   g.s += "    default: return 0;\n  }\n}\n";
-  g.s += "template <int V>\n__device__ __forceinline__ void jit_sums_add(int net, int64_t (&acc)[V],\n"
+  g.s += "template <int V>\n__device__ __forceinline__ void jit_sums_add(int net, uint64_t (&acc)[V],\n"
          "    uint64_t W, int aij, const uint64_t *v) {\n  switch (net) {\n";
   for (int d = 0; d < D; ++d) g.put("    case %d: jit_sums_add_n%d(acc, W, aij, v); break;\n", d, d);
   g.s += "    default: break;\n  }\n}\n";

@@ -732,7 +732,7 @@ __device__ __forceinline__ int64_t change_fixed(const DevProblem &P, const Slice
                                                 const StepCtx &X, int j, int aij, int aji,
                                                 uint64_t *v) {
   const int n = P.n, k = P.k, i = X.i;
-  int64_t f = X.f0;
+  uint64_t f = (uint64_t)X.f0;   // partial sums may wrap
 #pragma unroll 1
   for (int e = 0; e < k; ++e) {
     const int cls = S.ecls[e] & 0xFF;
@@ -761,7 +761,7 @@ __device__ __forceinline__ int64_t change_fixed(const DevProblem &P, const Slice
         }
       }
       v[e] = (uint64_t)c;
-      f += (int64_t)S.thq[e] * c;
+      f += S.thq[e] * (uint32_t)c;
       continue;
     }
     uint64_t m;
@@ -784,9 +784,9 @@ __device__ __forceinline__ int64_t change_fixed(const DevProblem &P, const Slice
       auto mag = [&](int q) -> int64_t {
         const int cl = S.ecls[q] & 0xFF;
         if (cl == FX_DELTA) return (int64_t)1 << S.esd[q];
-        if (cl == FX_CNT) return (int64_t)v[q] << S.esd[q];
-        if (cl == FX_UNI) return (int64_t)(S.stepq[4 * q] - (1ull << 62));
-        return cl == FX_REAL && v[q] ? (int64_t)(v[q] - (1ull << 62)) : 0;
+        if (cl == FX_CNT) return (int64_t)(v[q] << S.esd[q]);
+        if (cl == FX_UNI) return (int64_t)(S.stepq[4 * q] + kMinus62);
+        return cl == FX_REAL && v[q] ? (int64_t)(v[q] + kMinus62) : 0;
       };
       const int a = S.i0[e], b = S.i1[e], c = S.i2[e], have = S.esd[a] + S.esd[b] - 62;
       m = (c < 0 ? product_fx(mag(a), mag(b), have, S.esd[e])
@@ -799,10 +799,10 @@ __device__ __forceinline__ int64_t change_fixed(const DevProblem &P, const Slice
       m = real_fx(aij ? -g : g, S.esd[e]);
     }
     v[e] = m;
-    f += term_fx(S.thq[e], S.ecls[e], m);
-    if (ety) f += base_fx(S.thq[e], S.ecls[e]);
+    f += (uint64_t)term_fx(S.thq[e], S.ecls[e], m);
+    if (ety) f += (uint64_t)base_fx(S.thq[e], S.ecls[e]);
   }
-  return f;
+  return (int64_t)f;
 }
 
 // Behaviour change statistic, src/libcusna_saom_cpu.cpp:103-113.
