@@ -427,15 +427,17 @@ __device__ __forceinline__ double f64_of(const DevProblem &P, const Slice &S, co
 // permitted alter (at least the "no change" alter's 0), then sume = sum of
 // exp(f_j - lmax) and wsum_e = sum of exp(f_j - lmax) d_je over permitted
 // alters, every f_j and d_je the reference's float64 value. The sums run per
-// 32-alter block (fixed warp reduction) and over blocks in order, so they do
-// not depend on the team size; quantity 0 (the weights) and 1 + e land in
-// S.red[32G + q]. Then score_e += d_{jstar,e} - wsum_e / sume. Used by chains whose parameters exceed the fixed-point range
-// and at every ministep under F_LSE64. Called by the whole team.
+// 32-alter block (fixed warp reduction), every 32nd block's in order, then over
+// those 32, so they do not depend on the team size; quantity 0 (the weights) and
+// 1 + e land in S.red[32G + q]. Then score_e += d_{jstar,e} - wsum_e / sume. Used
+// by chains whose parameters exceed the fixed-point range, by ministeps with a sum
+// of few bits (sums_short), and at every ministep under F_LSE64. Called by the whole team.
 template <bool MULTI, int VQ>
 static __device__ __noinline__ void lse_float64(const Team T, const DevProblem &P, const Slice S,
                                                 const StepCtx X, double *d, int net, int jstar) {
   constexpr int V = VQ <= 8 ? 8 : (VQ <= 16 ? 16 : 32);  // warp_multi_sum's power of two
   const int n = P.n, k = P.k, L = T.L, i = X.i;
+  double *rec = reinterpret_cast<double *>(S.ring + ring_bytes(k));
   long long mk = dkey(0.0);
   for (int j = T.tl; j < n; j += L) {
     if (j == i || !((S.okbits[j >> 5] >> (j & 31)) & 1u)) continue;
@@ -446,7 +448,6 @@ static __device__ __noinline__ void lse_float64(const Team T, const DevProblem &
     }
   }
   const double lmax = dunkey(team_max_ll(T, mk, S.red));
-  double *rec64 = S.blk;
   for (int jb = 32 * T.warp; jb < n; jb += L) {
     const int j = jb + T.lane;
     double w = 0.0;
@@ -465,18 +466,17 @@ static __device__ __noinline__ void lse_float64(const Team T, const DevProblem &
     for (int q = 1; q < V; ++q) v[q] = (weighted && q - 1 < k) ? __dmul_rn(w, d[q - 1]) : 0.0;
     const int q = warp_multi_sum<V>(v, T.lane);
     const bool writer = (V >= 32) || ((T.lane & ((32 / V) - 1)) == 0);
-    if (writer && q <= k) rec64[(size_t)(jb >> 5) * (k + 1) + q] = v[0];
+    if (writer && q <= k) {   // block b and b + 32 are the same warp's and lane's
+      double *r = rec + ((jb >> 5) & 31) * (k + 1) + q;
+      *r = jb < 1024 ? v[0] : __dadd_rn(*r, v[0]);
+    }
   }
   T.sync();
   if (T.warp == 0) {
-    const int nb = (n + 31) >> 5;
     double v[V];
 #pragma unroll
-    for (int q = 0; q < V; ++q) v[q] = 0.0;
-    for (int b = T.lane; b < nb; b += 32)
-#pragma unroll
-      for (int q = 0; q < V; ++q)
-        if (q <= k) v[q] = __dadd_rn(v[q], rec64[(size_t)b * (k + 1) + q]);
+    for (int q = 0; q < V; ++q)
+      v[q] = q <= k && T.lane < ((n + 31) >> 5) ? __dadd_rn(0.0, rec[T.lane * (k + 1) + q]) : 0.0;
     const int q = warp_multi_sum<V>(v, T.lane);
     const bool writer = (V >= 32) || ((T.lane & ((32 / V) - 1)) == 0);
     if (writer && q <= k) S.red[32 * T.G + q] = v[0];
@@ -498,7 +498,7 @@ static __device__ __noinline__ void lse_float64(const Team T, const DevProblem &
 // Quantities: 0 the weights w_j (every permitted alter, "no change" included), 1
 // delta_j w_j, 2 + e the weighted magnitude delta_j w_j |d_je| of an effect of
 // class FX_CNT or FX_REAL. Each lane adds its alters in 64-bit integers (scale
-// 2^-(44 - sh); real statistics as mulhi_fx(w 2^6, m)), the warp adds its lanes'
+// 2^-(44 - sh); real statistics as mulround_fx(w 2^6, m)), the warp adds its lanes'
 // accumulators as three integer limbs, and the warps' sums are added as integers:
 // no order matters. kFxRoom bounds a lane's sums (see step_guard).
 // A specialised build fixes the number (CUSNA_FX_V) and the ones in use.
@@ -521,7 +521,7 @@ __device__ __forceinline__ void sums_add(const Slice &S, int k, uint64_t (&acc)[
     if (cls == FX_CNT) {
       acc[2 + e] += wd * v[e];
     } else if (cls == FX_REAL) {
-      acc[2 + e] += (uint64_t)signed_fx(mulhi_fx(w6, v[e]), aij);
+      acc[2 + e] += (uint64_t)signed_fx(mulround_fx(w6, v[e]), aij);
     }
   }
 }
@@ -547,7 +547,8 @@ __device__ __forceinline__ void sums_reduce(const uint64_t (&acc)[V], int lane, 
 
 // The ring: ministep slot's score sums as they left the pass (quantity q as lo +
 // 2^48 hi), the chosen alter's magnitudes (v of change_fixed; a FX_UNI effect's
-// float64 magnitude) and meta = 4 sh + 2 a_ij + ("no change" chosen). Divisions
+// float64 magnitude) and meta = 4 sh + 2 a_ij + ("no change" chosen), -1 where the
+// ministep's scores were formed in float64. Divisions
 // and float64 arithmetic wait for scores_flush: on this chip a dependent FP64
 // operation is tens of cycles and a division hundreds, 2,700 of the 8,800 cycles
 // of a ministep of one warp (n = 50) when every ministep did its own; eight at
@@ -558,11 +559,37 @@ struct ScoreRing {
 };
 __device__ __forceinline__ ScoreRing ring_of(const Slice &S, int k) {
   ScoreRing R;
-  R.lo = reinterpret_cast<int64_t *>(S.blk);
+  R.lo = reinterpret_cast<int64_t *>(S.ring);
   R.dst = R.lo + kRing * (k + 2);
   R.hi = reinterpret_cast<int *>(R.dst + kRing * k);
   R.meta = R.hi + kRing * (k + 2);
   return R;
+}
+
+// The "no change" alter's weight (exp_fx(0, sh)).
+__device__ __forceinline__ int64_t stay_weight(int sh) {
+  return sh <= kWBits ? 1LL << (kWBits - sh) : (sh == kWBits + 1 ? 1 : 0);
+}
+// The ring's sum at index x in float64.
+__device__ __forceinline__ double count_sum(const ScoreRing &R, int x) {
+  return __dadd_rn((double)R.lo[x], __dmul_rn((double)R.hi[x], 281474976710656.0));
+}
+// Quantity q's sum of the slot at x; of a real statistic (real) of creation or
+// endowment type ty less the 2^62 of every magnitude, which added 16 w delta: over
+// all alters, or over those that the creation (no tie) or endowment (tie) type
+// leaves, which is half of w (1 + delta), or of w (delta - 1), without "no change"
+// (stay: its weight). Taken off in integers, so that magnitudes of 0 leave 0.
+__device__ __forceinline__ double sum_value(const ScoreRing &R, int x, int q, bool real, int ty,
+                                            int64_t stay) {
+  if (!real) return count_sum(R, x + q);
+  int64_t minus8;   // a factor that the compiler does not turn into a subtraction (see signed_fx)
+  asm volatile("mov.b64 %0, -8;" : "=l"(minus8));
+  const int64_t cd = ty == 0 ? 2 : 1, cw = ty == 1 ? 1 : (ty == 2 ? -1 : 0),
+                cs = ty == 1 ? -1 : (ty == 2 ? 1 : 0);
+  int64_t lo = R.lo[x + q] + (R.lo[x + 1] * cd + R.lo[x] * cw + stay * cs) * minus8;
+  const int64_t hi = R.hi[x + q] + (R.hi[x + 1] * cd + R.hi[x] * cw) * minus8 + (lo >> 48);
+  lo &= (1LL << 48) - 1;
+  return __dadd_rn((double)lo, __dmul_rn((double)hi, 281474976710656.0));
 }
 
 // Adds the warps' sums into the ring (one warp, lane q).
@@ -588,46 +615,29 @@ static __device__ __noinline__ void scores_flush(const ScoreRing R, const int *e
                                                  const int *ety, const int *esd, double *sc,
                                                  int k, int lane, int cnt) {
   const int slot = lane & (kRing - 1);
-  const bool on = slot < cnt;
-  auto dbl = [&](int q) {
-    const int x = slot * (k + 2) + q;
-    return __dadd_rn((double)R.lo[x], __dmul_rn((double)R.hi[x], 281474976710656.0));
-  };
-  const int meta = on ? R.meta[slot] : 0;
-  const int sh = meta >> 2;
+  const int meta = slot < cnt ? R.meta[slot] : -1;
+  const bool on = meta >= 0;
+  const int sh = on ? meta >> 2 : 0, x = slot * (k + 2);
   const double dl = (meta & 1) ? 0.0 : ((meta & 2) ? -1.0 : 1.0);
-  const double w = on ? dbl(0) : 1.0, dw = on ? dbl(1) : 0.0;
+  const double w = on ? count_sum(R, x) : 1.0, dw = on ? count_sum(R, x + 1) : 0.0;
   const double inv = __ddiv_rn(1.0, w);
-  // the "no change" alter's weight (exp_fx(0, sh)), and a factor that the compiler
-  // does not turn into a subtraction (see signed_fx)
-  const int64_t stay = sh <= kWBits ? 1LL << (kWBits - sh) : (sh == kWBits + 1 ? 1 : 0);
-  int64_t minus8;
-  asm volatile("mov.b64 %0, -8;" : "=l"(minus8));
+  const int64_t stay = stay_weight(sh);
   auto term = [&](int e) -> double {
     if (!on || e >= k) return 0.0;
-    const int cls = ecls[e] & 0xFF, ty = ety[e];
+    const int cls = ecls[e] & 0xFF;
     const int64_t m = R.dst[slot * k + e];
     if (cls == FX_DELTA) return __dsub_rn(dl, __dmul_rn(dw, inv));
     if (cls == FX_UNI)   // a_ij = 0: the magnitude itself
       return __dmul_rn(__longlong_as_double(m), __dsub_rn(dl, __dmul_rn(dw, inv)));
-    if (cls == FX_CNT) return __dsub_rn(__dmul_rn(dl, (double)m), __dmul_rn(dbl(2 + e), inv));
+    if (cls == FX_CNT)
+      return __dsub_rn(__dmul_rn(dl, (double)m), __dmul_rn(count_sum(R, x + 2 + e), inv));
     if (cls != FX_REAL) return 0.0;
-    // the 2^62 of every magnitude added 16 w delta: over all alters, or over those
-    // that the creation (no tie) or endowment (tie) type leaves, which is half of
-    // w (1 + delta), or of w (delta - 1), without "no change". Taken off in
-    // integers, so that magnitudes of 0 leave 0.
-    const int x = slot * (k + 2);
-    const int64_t cd = ty == 0 ? 2 : 1, cw = ty == 1 ? 1 : (ty == 2 ? -1 : 0),
-                  cs = ty == 1 ? -1 : (ty == 2 ? 1 : 0);
-    int64_t lo = R.lo[x + 2 + e] + (R.lo[x + 1] * cd + R.lo[x] * cw + stay * cs) * minus8;
-    const int64_t hi = R.hi[x + 2 + e] + (R.hi[x + 1] * cd + R.hi[x] * cw) * minus8 + (lo >> 48);
-    lo &= (1LL << 48) - 1;
     const double back = pow2(-esd[e]);
-    const double mean = __dmul_rn(
-        __dmul_rn(__dadd_rn((double)lo, __dmul_rn((double)hi, 281474976710656.0)), inv),
-        __dmul_rn(pow2(58), back));
+    const double mean = __dmul_rn(__dmul_rn(sum_value(R, x, 2 + e, true, ety[e], stay), inv),
+                                  __dmul_rn(pow2(58), back));
     // (a magnitude of 0 marks one that the type rules out)
-    const double ds = m ? __dmul_rn(__dmul_rn(dl, (double)(int64_t)((uint64_t)m + kMinus62)), back) : 0.0;
+    const double ds =
+        m ? __dmul_rn(__dmul_rn(dl, (double)(int64_t)((uint64_t)m + kMinus62)), back) : 0.0;
     return __dsub_rn(ds, mean);
   };
   for (int e0 = 0; e0 < k; e0 += 8) {   // two effects at once: their chains overlap
@@ -647,6 +657,25 @@ __device__ __forceinline__ void scores_flush(const Team &T, const Slice &S, int 
   if (T.warp == T.G - 1) scores_flush(ring_of(S, k), S.ecls, S.ety, S.esd, S.sc, k, T.lane, cnt);
 }
 
+constexpr int kLn2 = 11356;   // ln2 at scale 2^-14
+// A predictor this many ln2 (11.8) below sh ln2 has a weight of fewer than 28 bits,
+// whose rounding may exceed 2^-28 of it, a sixteenth of a float32's. From sh = 18 on
+// that is the "no change" alter's, and the sums are formed in float64.
+constexpr int kMaxShift = 17;
+
+// Whether a sum of the ring's slot may have lost a float32's precision to weights of
+// few bits: it is below 2^34 units of the grid (of a real statistic as large as its
+// bound 2^38), where hundreds of weights' roundings stay below 2^-29 of it; or it is 0
+// and a weight was rounded to 0 (zeros). One warp.
+static __device__ __noinline__ bool sums_short(const ScoreRing R, const int *ecls, const int *ety,
+                                               int k, int slot, int sh, int lane, bool zeros) {
+  if (lane >= k + 2) return false;
+  const int x = slot * (k + 2), e = lane - 2, cls = e < 0 ? (int)FX_CNT : ecls[e] & 0xFF;
+  if (cls < FX_CNT) return false;
+  const double v = fabs(sum_value(R, x, lane, cls == FX_REAL, e < 0 ? 0 : ety[e], stay_weight(sh)));
+  return v == 0.0 ? zeros : v < (cls == FX_REAL ? 274877906944.0 : 17179869184.0);
+}
+
 // Largest f (scale 2^-14) for which no lane's sums can leave 63 bits: with nb
 // blocks of 32 alters a lane adds at most nb products w |d| at scale 2^44 (real
 // statistics: w 2^50 at most), so w mb nb <= 2^17 keeps them below 2^61, mb
@@ -658,7 +687,7 @@ __device__ __forceinline__ int step_guard(const DevProblem &P, const Slice &S, c
   // out-degrees of every network (cross effects count another network's ties)
   for (int w = 0; w < X.net.D; ++w) mb = max(mb, X.net.misc[w * X.net.misc_stride + 11] + 1);
   const int lg = 17 - (32 - __clz(mb * nb - 1));   // floor(log2(2^17 / (mb nb)))
-  return lg * 11356;                               // ln2 at 2^-14
+  return lg * kLn2;
 }
 
 // Per-thread scratch of one alter's change statistics in the pass over the
@@ -695,12 +724,12 @@ __device__ __forceinline__ RowWords row_words(const DevProblem &P, const Slice &
 // the magnitudes and the predictor, the float32 Gumbel key with its error bound
 // (into *best and S.gbuf), the permitted-alter bits (S.okbits) and, with sums,
 // the weight exp(f_j) 2^-sh and its products, whose warp sums end in S.red and
-// S.redh. Returns the lane's largest predictor (scale 2^-14). Block b of 32
-// alters belongs to warp b mod G.
+// S.redh. Returns the lane's largest predictor (scale 2^-14), and in fmin its
+// smallest. Block b of 32 alters belongs to warp b mod G.
 template <bool MULTI, bool VALID, int V>
 __device__ __forceinline__ int alter_pass(const Team &T, const DevProblem &P, const Slice &S,
                                           const StepCtx &X, long long ms, uint32_t chain,
-                                          KeyTop &best, bool sums, int sh, int net,
+                                          KeyTop &best, int &fmin, bool sums, int sh, int net,
                                           RowWords words) {
   const int n = prob_n(P), k = prob_k(P), i = X.i;
   (void)net;
@@ -714,6 +743,7 @@ __device__ __forceinline__ int alter_pass(const Team &T, const DevProblem &P, co
 #pragma unroll
   for (int q = 0; q < V; ++q) acc[q] = 0;
   int fmax = 0;
+  fmin = 0;
   const bool full = P.maxdeg > 0 && X.od_i >= P.maxdeg;   // no new tie
   const uint32_t k0 = P.k0, k1 = P.k1;
 #pragma unroll 1
@@ -743,6 +773,7 @@ __device__ __forceinline__ int alter_pass(const Team &T, const DevProblem &P, co
     const float E = fmaf(fabsf(f32), 3.6e-7f, 3e-5f);
     if (ok) {
       fmax = max(fmax, fh);
+      fmin = min(fmin, fh);
       keytop_add(best, gk, E, j);
     }
     if (jl < n) S.gbuf[j] = ok ? __fadd_rn(gk, E) : -INFINITY;
@@ -871,29 +902,37 @@ __device__ __forceinline__ int net_choice(const Team &T, const DevProblem &P, co
   // gbuf[j] keeps the upper bound g_j + E_j. When a predictor exceeds the room
   // that the sums have (step_guard), the pass is repeated with every weight
   // scaled by 2^-sh, sh from the largest predictor (so from the alters alone).
+  // Where an alter's weight then has few bits and a sum is short of them
+  // (sums_short), the ministep's sums are formed in float64: an effect whose
+  // statistics are all at improbable alters has a score of its own size, and a
+  // float32 ulp of that. (The fixed grid alone was 5e-6 of such a score off at
+  // f = -20, and all of it from f = -31 on.)
   // Without requested scores (F_NO_SCORES) no sums are formed.
   const bool want_sums = (fl & F_NO_SCORES) == 0;
   const bool fast_sums = want_sums && (fl & F_LSE64) == 0 && ranged;
   KeyTop top{-INFINITY, 0.f, INFINITY, 0x7FFFFFFF};
   float lb = -INFINITY;
-  int sh = 0;
+  int sh = 0, fn = 0;
+  bool few = false, ring = false;
   if (ranged) {
     const int room = fast_sums ? step_guard(P, S, X) : 0x7FFFFFFF;
     for (;;) {
       KeyTop best{-INFINITY, 0.f, -INFINITY, 0x7FFFFFFF};
       int fm;
 #ifdef CUSNA_FX_V
-      fm = alter_pass<MULTI, VALID, CUSNA_FX_V>(T, P, S, X, ms, chain, best, fast_sums, sh, net, words);
+      fm = alter_pass<MULTI, VALID, CUSNA_FX_V>(T, P, S, X, ms, chain, best, fn, fast_sums, sh, net,
+                                                words);
 #else
       if (k + 2 <= 8)
-        fm = alter_pass<MULTI, VALID, 8>(T, P, S, X, ms, chain, best, fast_sums, sh, net, words);
+        fm = alter_pass<MULTI, VALID, 8>(T, P, S, X, ms, chain, best, fn, fast_sums, sh, net, words);
       else if (k + 2 <= 16)
-        fm = alter_pass<MULTI, VALID, 16>(T, P, S, X, ms, chain, best, fast_sums, sh, net, words);
+        fm = alter_pass<MULTI, VALID, 16>(T, P, S, X, ms, chain, best, fn, fast_sums, sh, net, words);
       else
-        fm = alter_pass<MULTI, VALID, 26>(T, P, S, X, ms, chain, best, fast_sums, sh, net, words);
+        fm = alter_pass<MULTI, VALID, 26>(T, P, S, X, ms, chain, best, fn, fast_sums, sh, net, words);
 #endif
       top = warp_keytop(best, T.lane);
       fm = __reduce_max_sync(kFull, fm);
+      few = __any_sync(kFull, fn < (sh - kMaxShift) * kLn2);
       if (T.G > 1) {
         float *rb = reinterpret_cast<float *>(S.red + 32 * T.G + 32);   // 4 words per warp
         int *ri = reinterpret_cast<int *>(rb);
@@ -902,24 +941,45 @@ __device__ __forceinline__ int net_choice(const Team &T, const DevProblem &P, co
           rb[4 * T.warp + 1] = top.e1;
           rb[4 * T.warp + 2] = top.ub2;
           ri[4 * T.warp + 3] = top.j1;
-          S.rfm[T.warp] = fm;
+          S.rfm[T.warp] = 2 * fm + (int)few;   // fm >= 0, the "no change" alter's
         }
         T.sync();
         top = KeyTop{rb[0], rb[1], rb[2], ri[3]};
         fm = S.rfm[0];
+        int any = fm;
         for (int w = 1; w < T.G; ++w) {
           keytop_merge(top, KeyTop{rb[4 * w], rb[4 * w + 1], rb[4 * w + 2], ri[4 * w + 3]});
           fm = max(fm, S.rfm[w]);
+          any |= S.rfm[w];
         }
+        fm >>= 1;
+        few = any & 1;
       } else {
         __syncwarp();
       }
-      if (fm <= room) break;
-      // the smallest scaling for which the largest predictor fits (ln2 at 2^-14)
-      const int need = (fm - room + 11355) / 11356;
-      if (need <= sh) break;
-      sh = need;
+      if (fm <= room + sh * kLn2 || !fast_sums) break;
+      // the smallest scaling for which the largest predictor fits
+      sh = (fm - room + kLn2 - 1) / kLn2;
+      if (sh > kMaxShift) break;
       T.sync();   // every warp has read the first pass's scratch
+    }
+    ring = fast_sums && sh <= kMaxShift;
+    if (ring && few) {
+      const bool z = __any_sync(kFull, fn < (sh - kWBits + 1) * kLn2);
+      T.sync();   // every warp has read rfm
+      if (T.lane == 0) S.rfm[T.warp] = z;
+      T.sync();
+      if (T.warp == 0) {
+        int zeros = 0;
+        for (int w = 0; w < T.G; ++w) zeros |= S.rfm[w];
+        sums_combine(T, S, ring_of(S, k), k, slot);
+        __syncwarp();
+        const bool s = __any_sync(kFull, sums_short(ring_of(S, k), S.ecls, S.ety, k, slot, sh, T.lane,
+                                                    zeros != 0));
+        if (T.lane == 0) S.rfm[0] = s;
+      }
+      T.sync();
+      ring = S.rfm[0] == 0;
     }
     lb = __fsub_rn(top.b1, top.e1);
   } else {
@@ -939,7 +999,8 @@ __device__ __forceinline__ int net_choice(const Team &T, const DevProblem &P, co
   // the score sums into the ring by a warp other than the chosen alter's owner,
   // which meanwhile forms the chosen alter's magnitudes; on the float64 path, the
   // scores by the whole team
-  if (want_sums && !fast_sums) {
+  if (want_sums && !ring) {
+    if (fast_sums && T.tl == 0) ring_of(S, k).meta[slot] = -1;
 #ifdef CUSNA_JIT_K
     lse_float64<MULTI, CUSNA_JIT_K + 1>(T, P, S, X, d, net, jstar);
 #else
@@ -947,7 +1008,7 @@ __device__ __forceinline__ int net_choice(const Team &T, const DevProblem &P, co
     else if (k + 1 <= 16) lse_float64<MULTI, 16>(T, P, S, X, d, net, jstar);
     else lse_float64<MULTI, 32>(T, P, S, X, d, net, jstar);
 #endif
-  } else if (fast_sums) {
+  } else if (ring) {
     const ScoreRing R = ring_of(S, k);
     const int owner = jstar & (L - 1);   // L and G are powers of two
     if (T.warp == (((owner >> 5) + 1) & (T.G - 1))) sums_combine(T, S, R, k, slot);

@@ -260,7 +260,10 @@ __device__ __forceinline__ float gumbel_est(uint32_t x) {
 // exact whatever the order, so any split of the alters over warps gives the
 // same bits, and a count's term is one 64-bit multiply-add.
 //   predictor f_j          scale 2^-46 (kFBits)
-//   weight exp(f_j)        scale 2^-44 (kWBits), "no change" weighs 1
+//   weight exp(f_j)        scale 2^-(44 - sh) (kWBits): "no change" weighs 1; sh
+//                          follows the ministep's largest predictor. Where the
+//                          grid is too coarse for a sum, the ministep's sums are
+//                          formed in float64 (net_choice)
 //   real statistic d_e     |d_e| 2^sd + 2^62 as an unsigned number, sd_e from
 //                          the effect's largest |d_e| (fx_scale)
 constexpr int kFBits = 46, kWBits = 44;
@@ -278,7 +281,7 @@ __host__ __device__ inline int fx_scale(double bound) {
 }
 
 // High 64 bits of a * b without the product of the low halves (at most 3 below
-// the exact ones).
+// the exact ones): a predictor's terms.
 __host__ __device__ __forceinline__ uint64_t mulhi_fx(uint64_t a, uint64_t b) {
   const uint32_t ah = (uint32_t)(a >> 32), al = (uint32_t)a;
   const uint32_t bh = (uint32_t)(b >> 32), bl = (uint32_t)b;
@@ -287,6 +290,16 @@ __host__ __device__ __forceinline__ uint64_t mulhi_fx(uint64_t a, uint64_t b) {
 #else
   return (uint64_t)ah * bh + (((uint64_t)ah * bl) >> 32) + (((uint64_t)al * bh) >> 32);
 #endif
+}
+
+// a * b 2^-64, rounded to nearest: the score sums add a product per alter, and a
+// cut to one side would add up over the alters and ministeps.
+__host__ __device__ __forceinline__ uint64_t mulround_fx(uint64_t a, uint64_t b) {
+  const uint32_t ah = (uint32_t)(a >> 32), al = (uint32_t)a;
+  const uint32_t bh = (uint32_t)(b >> 32), bl = (uint32_t)b;
+  const uint64_t p = (uint64_t)ah * bl + (((uint64_t)al * bl) >> 32);
+  const uint64_t q = (uint64_t)al * bh + (uint32_t)p;
+  return (uint64_t)ah * bh + (p >> 32) + (q >> 32) + ((uint32_t)q >> 31);
 }
 
 // -2^62: taken off a magnitude by an addition.

@@ -252,7 +252,7 @@ void gen_functions(Gen &g, const JitPlan &J, const std::string &sfx, bool multi)
     else if (cls == FX_CNT)
       g.put("  acc[%d] += wd * (uint32_t)v[%d];\n", 2 + e, e);
     else if (cls == FX_REAL)
-      g.put("  acc[%d] += (uint64_t)signed_fx(mulhi_fx(w6, v[%d]), aij);\n", 2 + e, e);
+      g.put("  acc[%d] += (uint64_t)signed_fx(mulround_fx(w6, v[%d]), aij);\n", 2 + e, e);
   }
   g.s += "}\n";
   // float64 evaluation (change_stats): the chosen alter and uncertified choices

@@ -39,8 +39,8 @@ struct Slice {
   short *indeg, *outdeg;  // n each (degrees < 2^15 as n <= 8192)
   int *z;
   float *gbuf;       // n   upper bounds of the float32 Gumbel keys
-  double *blk;       // ceil(n/32)*(k+1)  per 32-alter block: the score sums of the
-                     //   float64 path; the same bytes hold the ring (ScoreRing)
+  unsigned char *ring;  // the score sums of the last ministeps (ScoreRing), then
+                     //   min(32, ceil(n/32))*(k+1) sums of the float64 path
   uint32_t *okbits;  // W
   int *tp;           // n   (gwdspFF)
   int *tq;           // n   (gwdspFB)
@@ -49,7 +49,7 @@ struct Slice {
   double *crate;     // n   (non-basic rates)
   double *red;       // 32*G + 64 reduction scratch
   int *redh;         // 32*G  high parts of the warps' score sums
-  int *rfm;          // G    the warps' largest predictors
+  int *rfm;          // G    the warps' largest predictors (and flags)
   double *th;        // k  parameters of the current chain
   uint64_t *thq;     // k  the same in fixed point (theta_fx)
   int *esd, *ecls;   // k  scale of a real statistic, class (FX_*) of an effect
@@ -72,7 +72,7 @@ struct Slice {
 
 struct SliceLayout {
   size_t bytes;  // per team
-  size_t o_rows, o_cols, o_indeg, o_outdeg, o_z, o_g, o_blk, o_ok, o_tp, o_tq, o_tpeq, o_crate, o_red, o_th, o_sc, o_dstar, o_thb, o_bsc, o_rsc, o_p1, o_p2, o_tid,
+  size_t o_rows, o_cols, o_indeg, o_outdeg, o_z, o_g, o_ring, o_ok, o_tp, o_tq, o_tpeq, o_crate, o_red, o_th, o_sc, o_dstar, o_thb, o_bsc, o_rsc, o_p1, o_p2, o_tid,
       o_ety, o_dyn, o_i0, o_i1, o_i2, o_bty, o_rkind, o_misc, o_rtau, o_rnet, o_rfocal, o_rr3, o_ekind, o_ecfn, o_eoffd, o_eofft,
       o_stepd, o_stept, o_stepq, o_thq, o_esd, o_ecls, o_fx, o_redh, o_rfm;
 };
@@ -82,7 +82,7 @@ __host__ __device__ inline size_t al16(size_t x) { return (x + 15) & ~(size_t)15
 // Ministeps whose score sums wait for one flush (scores_flush).
 constexpr int kRing = 8;
 __host__ __device__ inline size_t ring_bytes(int k) {
-  return (size_t)kRing * ((k + 2) * 12 + k * 8 + 4);
+  return al16((size_t)kRing * ((k + 2) * 12 + k * 8 + 4));
 }
 
 // Layout of one team slice for maxima (n, k, ...) over the launch.
@@ -98,9 +98,7 @@ __host__ __device__ inline SliceLayout make_layout(int n, int W, int k, int kb, 
   put(s.o_outdeg, (size_t)n * 2);
   put(s.o_z, (size_t)n * 4);
   put(s.o_g, (size_t)n * 4);
-  // the score sums of the float64 path, or the ring of the fixed-point one
-  const size_t blk = (size_t)((n + 31) / 32) * (k + 1) * 8, ring = ring_bytes(k);
-  put(s.o_blk, blk > ring ? blk : ring);
+  put(s.o_ring, ring_bytes(k) + (size_t)(n > 992 ? 32 : (n + 31) / 32) * (k + 1) * 8);
   put(s.o_ok, (size_t)W * 4);
   put(s.o_tp, need_gw ? (size_t)n * 4 : 0);
   put(s.o_tq, need_tq ? (size_t)n * 4 : 0);
@@ -156,7 +154,7 @@ __device__ __forceinline__ Slice carve(unsigned char *base, const SliceLayout &L
   s.outdeg = (short *)(base + L.o_outdeg);
   s.z = (int *)(base + L.o_z);
   s.gbuf = (float *)(base + L.o_g);
-  s.blk = (double *)(base + L.o_blk);
+  s.ring = base + L.o_ring;
   s.okbits = (uint32_t *)(base + L.o_ok);
   s.tp = (int *)(base + L.o_tp);
   s.tq = (int *)(base + L.o_tq);
