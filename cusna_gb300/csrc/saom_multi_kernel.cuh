@@ -33,6 +33,9 @@ static __device__ void run_chain_multi(const Team &T, const DevProblem *nets, co
   const uint32_t chain = (uint32_t)c;
   for (int d = 0; d < D; ++d)
     chain_init(T, nets[d], multi_slice(base, lay, d, cols_g, rows_g, counts_g, cols_words, counts_stride, etab), c);
+  if (T.tl == 0)
+    for (int d = 0; d < D; ++d)
+      multi_slice(base, lay, d, cols_g, rows_g, counts_g, cols_words, counts_stride, etab).misc[14] = 0;
   double lam_d[kMaxNet];
   double lam_tot = 0.0;
   for (int d = 0; d < D; ++d) {
@@ -75,9 +78,11 @@ static __device__ void run_chain_multi(const Team &T, const DevProblem *nets, co
     const DevProblem &P = nets[d];
     const Slice S = multi_slice(base, lay, d, cols_g, rows_g, counts_g, cols_words, counts_stride, etab);
     const int rslot = (int)msd[d] & (kRing - 1);
-    const int jstar = net_choice<true>(T, P, S, i, ms, chain, dbuf, &nb, rslot, d);
+    int keep = S.misc[14];   // the score sums' scaling to begin with (net_choice)
+    const int jstar = net_choice<true>(T, P, S, i, ms, chain, dbuf, &nb, rslot, keep, d);
     const int aij_star = bit_of(S.rows, n, i, jstar);
     T.sync();
+    if (T.tl == 0) S.misc[14] = keep;
     score_slot(T, P, S, rslot);
     ++ms;
     ++msd[d];
