@@ -963,7 +963,7 @@ __device__ __forceinline__ int net_choice(const Team &T, const DevProblem &P, co
       } else {
         __syncwarp();
       }
-      if (fm <= room + sh * kLn2 || !fast_sums) break;
+      if (__builtin_expect(fm <= room + sh * kLn2 || !fast_sums, 1)) break;
       // the smallest scaling for which the largest predictor fits
       sh = (fm - room + kLn2 - 1) / kLn2;
       if (sh > kMaxShift) break;
@@ -971,7 +971,7 @@ __device__ __forceinline__ int net_choice(const Team &T, const DevProblem &P, co
     }
     ring = fast_sums && sh <= kMaxShift;
     keep = max(min(sh, kKeepShift) - (int)(((int)ms & (kShiftLife - 1)) == 0), 0);
-    if (ring && few) {
+    if (__builtin_expect(ring && few, 0)) {
       const bool z = __any_sync(kFull, fn < (sh - kWBits + 1) * kLn2);
       T.sync();   // every warp has read rfm
       if (T.lane == 0) S.rfm[T.warp] = z;
