@@ -37,6 +37,62 @@ __device__ __forceinline__ void load_exp_table(int2 *etab, const DevProblem *pro
   __syncthreads();
 }
 
+// Fixed-point scales, classes and parameters (one lane). The pass over the alters
+// needs every |f_j| < 2^14, by bounds on the statistics: of the own network's counts
+// and degrees a cap, S.fx[2], which starts as what n allows and is halved until the
+// parameters fit, while it is above the counts that the chain starts with (mb). A
+// chain that nears its cap (cap_check), or that none fits, runs in float64
+// (S.fx[1] = 0). With the bounds of n alone, chains of large sparse networks did from
+// the start: transTrip's at n = 8192 alone allowed |theta| < 1.
+__device__ __forceinline__ void chain_scales(const DevProblem &P, const Slice &S, int mb) {
+  const int k = prob_k(P);
+  double range = 0.0;
+  int cap = max(16, 2 * P.n + 2);
+  for (;; cap /= 2) {
+    range = 0.0;
+    for (int e = 0; e < k; ++e) {
+      const int kind = S.ekind[e], t = S.tid[e];
+      const int cls = fx_class(kind, S.ecfn[e] & 0xFF, t, S.ety[e]);
+      double bound = P.ebound[e];
+      if (kind == K_CNT || (kind == K_STEP && t >= 14 && t <= 19 && t != 18))
+        bound = bound > (double)cap ? (double)cap : bound;
+      if (t == 32 && kind != K_ZERO) {   // products: the components' bounds
+        bound = __dmul_rn(S.dstar[S.i0[e]], S.dstar[S.i1[e]]);
+        if (S.i2[e] >= 0) bound = __dmul_rn(bound, S.dstar[S.i2[e]]);
+      }
+      S.dstar[e] = bound;
+      S.esd[e] = fx_scale(bound);
+      S.ecls[e] = cls | (S.th[e] < 0.0 ? 256 : 0);
+      if (cls != FX_ZERO) range = __dadd_rn(range, __dmul_rn(fabs(S.th[e]), bound));
+    }
+    if (range < 16384.0 || !(cap / 2 >= mb)) break;
+  }
+  uint64_t f0 = 0;
+  const bool in_range = range < 16384.0;      // false for a NaN
+  if (in_range)
+    for (int e = 0; e < k; ++e) {
+      S.thq[e] = theta_fx(S.th[e], S.ecls[e] & 0xFF, S.esd[e]);
+      if ((S.ecls[e] & 0xFF) == FX_DELTA) f0 += S.thq[e];
+      // the part of a real magnitude's 2^62, for every alter alike
+      if ((S.ecls[e] & 0xFF) == FX_UNI || ((S.ecls[e] & 0xFF) == FX_REAL && S.ety[e] == 0))
+        f0 += (uint64_t)base_fx(S.thq[e], S.ecls[e]);
+    }
+  S.fx[0] = (int64_t)f0;
+  S.fx[1] = in_range;
+  S.fx[2] = cap >= 2 * P.n + 2 ? 0x7FFFFFFF : cap;
+  S.misc[15] = in_range;
+}
+
+// Before every 32nd ministep (one lane): whether the next 32 toggles keep the counts
+// and degrees below the cap.
+constexpr int kCapEvery = 32;
+__device__ __forceinline__ int capped_counts(int max_out, int max_in) {
+  return max(16, max(2 * (max_out + kCapEvery) + 2, max_in + kCapEvery + 1));
+}
+__device__ __forceinline__ void cap_check(const Slice &S) {
+  if (capped_counts(S.misc[11], S.misc[10]) > (int)S.fx[2]) S.fx[1] = 0;
+}
+
 // Load the chain's start state and parameters into the team slice.
 __device__ __forceinline__ void chain_init(const Team &T, const DevProblem &P, const Slice &S,
                                            int c) {
@@ -91,38 +147,6 @@ __device__ __forceinline__ void chain_init(const Team &T, const DevProblem &P, c
     for (int x = T.tl; x < n; x += L) S.crate[x] = 1.0;
   if (T.tl == 0) S.misc[13] = c;   // the chain's index within its problem (validation words)
   T.sync();
-  if (T.tl == 0) {
-    // fixed-point scales, classes and parameters; the pass over the alters needs
-    // every |f_j| < 2^14 (S.fx[1]), else the chain runs on the float64 path
-    uint64_t f0 = 0;
-    double range = 0.0;
-    for (int e = 0; e < k; ++e) {
-      const int kind = S.ekind[e];
-      const int cls = fx_class(kind, S.ecfn[e] & 0xFF, S.tid[e], S.ety[e]);
-      double bound = P.ebound[e];
-      int sd = fx_scale(bound);
-      if (S.tid[e] == 32 && kind != K_ZERO) {   // products: the components' bounds
-        bound = __dmul_rn(S.dstar[S.i0[e]], S.dstar[S.i1[e]]);
-        if (S.i2[e] >= 0) bound = __dmul_rn(bound, S.dstar[S.i2[e]]);
-        sd = fx_scale(bound);
-      }
-      S.dstar[e] = bound;
-      S.esd[e] = sd;
-      S.ecls[e] = cls | (S.th[e] < 0.0 ? 256 : 0);
-      if (cls != FX_ZERO) range = __dadd_rn(range, __dmul_rn(fabs(S.th[e]), bound));
-    }
-    const bool in_range = range < 16384.0;      // false for a NaN
-    if (in_range)
-      for (int e = 0; e < k; ++e) {
-        S.thq[e] = theta_fx(S.th[e], S.ecls[e] & 0xFF, S.esd[e]);
-        if ((S.ecls[e] & 0xFF) == FX_DELTA) f0 += S.thq[e];
-        // the part of a real magnitude's 2^62, for every alter alike
-        if ((S.ecls[e] & 0xFF) == FX_UNI || ((S.ecls[e] & 0xFF) == FX_REAL && S.ety[e] == 0))
-          f0 += (uint64_t)base_fx(S.thq[e], S.ecls[e]);
-      }
-    S.fx[0] = (int64_t)f0;
-    S.fx[1] = in_range;
-  }
   for (int x = T.tl; x < n; x += L) {
     int od = 0, id = 0;
     for (int w = 0; w < W; ++w) {
@@ -145,6 +169,7 @@ __device__ __forceinline__ void chain_init(const Team &T, const DevProblem &P, c
   if (T.tl == 0) {
     S.misc[10] = mi;
     S.misc[11] = mo;
+    chain_scales(P, S, capped_counts(mo, mi));
   }
   T.sync();
 }
@@ -681,7 +706,8 @@ static __device__ __noinline__ bool sums_short(const ScoreRing R, const int *ecl
 // Largest f (scale 2^-14) for which no lane's sums can leave 63 bits: with nb
 // blocks of 32 alters a lane adds at most nb products w |d| at scale 2^44 (real
 // statistics: w 2^50 at most), so w mb nb <= 2^17 keeps them below 2^61, mb
-// being the largest count that the ministep can meet (at least 16).
+// being
+// the largest count or degree that the ministep can meet (at least 16).
 __device__ __forceinline__ int step_guard(const DevProblem &P, const Slice &S, const StepCtx &X) {
   const int nb = (P.n + 31) >> 5;
   int mb = max(16, max(2 * X.od_i + 2, X.id_i + 1));
@@ -850,7 +876,7 @@ static __device__ __noinline__ int choice_float64(const Team T, const DevProblem
 
 // The chain's scores go through the ring.
 __device__ __forceinline__ bool ring_scores(const DevProblem &P, const Slice &S) {
-  return (P.flags & (F_NO_SCORES | F_LSE64)) == 0 && S.fx[1] != 0;
+  return (P.flags & (F_NO_SCORES | F_LSE64)) == 0 && S.misc[15] != 0;
 }
 // After ministep slot's choice and a team barrier: a full ring into the scores.
 __device__ __forceinline__ void score_slot(const Team &T, const DevProblem &P, const Slice &S,
@@ -1007,7 +1033,7 @@ __device__ __forceinline__ int net_choice(const Team &T, const DevProblem &P, co
   // which meanwhile forms the chosen alter's magnitudes; on the float64 path, the
   // scores by the whole team
   if (want_sums && !ring) {
-    if (fast_sums && T.tl == 0) ring_of(S, k).meta[slot] = -1;
+    if (T.tl == 0) ring_of(S, k).meta[slot] = -1;
 #ifdef CUSNA_JIT_K
     lse_float64<MULTI, CUSNA_JIT_K + 1>(T, P, S, X, d, net, jstar);
 #else
@@ -1101,6 +1127,7 @@ static __device__ void run_chain(const Team &T, const DevProblem &P, const Slice
     if (P.nrate > 0) {
       uint32_t rr[4];
       step_words<VALID>(P, S, ms, chain, rr);
+      if (((int)ms & (kCapEvery - 1)) == 0 && T.tl == 0) cap_check(S);
       i = rate_draw(T, P, S, rr, lam, t, rho);
       if (i < 0) break;
       is_net = true;
@@ -1120,6 +1147,7 @@ static __device__ void run_chain(const Team &T, const DevProblem &P, const Slice
           if (idx >= P.nact) idx = P.nact - 1;
           S.rfocal[T.lane] = P.act[idx];
           S.rr3[T.lane] = rr[3];
+          if (T.lane == 0) cap_check(S);
         }
         T.sync();
         tnext = __dadd_rn(t, S.rtau[0]);

@@ -368,7 +368,7 @@ __host__ __device__ inline double effect_bound(int t, int n, double vmax, double
     case 3: case 23: case 4: case 5: case 8: case 14: case 36: case 37: return N + 1.0;
     case 7: case 9: case 15: return N + 1.0;
     case 17: return 2.0 * N + 2.0;    // 1.5 sqrt(n + 1) at most
-    case 18: return N + 1.0 + a1;
+    case 18: return 1.0;              // min(d +- 1, p) - min(d, p)
     case 10: case 11: return vmax;
     case 12: return 1.0 + 2.0 * vmax * a1 + a2;
     case 21: return vmax * vmax;

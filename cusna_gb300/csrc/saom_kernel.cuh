@@ -53,7 +53,7 @@ struct Slice {
   double *th;        // k  parameters of the current chain
   uint64_t *thq;     // k  the same in fixed point (theta_fx)
   int *esd, *ecls;   // k  scale of a real statistic, class (FX_*) of an effect
-  int64_t *fx;       // 2  constant part of the predictor; chain in range (0/1)
+  int64_t *fx;       // 3  constant part of the predictor; in range (0/1); bound on counts
   double *sc;        // k  scores
   double *dstar;     // k  change statistics of the chosen alter
   double *thb, *bsc; // kb
@@ -136,7 +136,7 @@ __host__ __device__ inline SliceLayout make_layout(int n, int W, int k, int kb, 
   put(s.o_thq, (size_t)k * 8);
   put(s.o_esd, (size_t)k * 4);
   put(s.o_ecls, (size_t)k * 4);
-  put(s.o_fx, 16);
+  put(s.o_fx, 24);
   put(s.o_redh, (size_t)32 * G * 4);
   put(s.o_rfm, (size_t)G * 4);
   s.bytes = al16(o);

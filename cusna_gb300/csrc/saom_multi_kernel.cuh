@@ -69,6 +69,8 @@ static __device__ void run_chain_multi(const Team &T, const DevProblem *nets, co
         long long idx = (long long)__dmul_rn(unif01(rr[2]), (double)md.nact);
         if (idx >= md.nact) idx = md.nact - 1;
         S0.rfocal[T.lane] = md.act[idx];
+        if (T.lane < D)
+          cap_check(multi_slice(base, lay, T.lane, cols_g, rows_g, counts_g, cols_words, counts_stride, etab));
       }
       T.sync();
     }
