@@ -32,7 +32,9 @@ namespace cusna {
 namespace {
 
 constexpr size_t kStaticScratchBytes = (size_t)16 << 20;  // 16 MiB per device
-constexpr size_t kStaticExtra = 4096;   // the exponential's table and the effects' bounds
+constexpr size_t kStaticExtra = 4096;   // the problem, the exponential's table and the effects' bounds
+constexpr size_t kRuleProblemBytes = 576;   // a problem's descriptor in the scratch rule's accounting
+static_assert(sizeof(DevProblem) + 256 * 8 + CUSNA_MAXEFF * 8 + 3 * 256 <= kStaticExtra, "scratch beside the rule");
 static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes + kStaticExtra];
 
 constexpr int kMaxDevices = 64;
@@ -301,32 +303,35 @@ extern "C" CUSNA_API cusna_status cusna_saom_simulate_period_static(
       }
     }
   if (rule_score < 0) { set_last_error("no launch shape fits this n in shared memory"); return CUSNA_ERR_UNSUPPORTED; }
-  for (int G = 1; G <= 16; G *= 2)
-    for (int cs = 1; cs >= 0; --cs) {
-      LaunchShape sh{};
-      sh.G = G;
-      sh.cols_in_smem = cs;
-      sh.rows_in_smem = true;
-      sh.lay = make_layout(n, W, k, kb, nr, G, true, cs, need_tp, need_gw, need_tq);
-      if (sh.lay.bytes > (size_t)smem_optin) continue;
-      for (int tpc = 1; tpc <= 16; tpc *= 2) {
-        const int threads = 32 * G * tpc;
-        if (threads > 512 || (G > 1 && tpc > 15) || sh.lay.bytes * tpc > (size_t)smem_optin) continue;
-        const int per_sm = period_blocks_per_sm(threads, sh.lay.bytes * tpc);
-        if (per_sm < 1) continue;
-        const double teams_sm = (double)per_sm * tpc;
-        const double busy = (teams_sm < (double)M / sms ? teams_sm : ((double)M / sms > 1 ? (double)M / sms : 1.0)) * G;
-        const double score = (busy < 48 ? busy : 48) * 100.0 - G - (cs ? 0.0 : 50.0) - tpc * 0.01;
-        if (score > best_score) {
-          best_score = score;
-          best = sh;
-          best.teams_per_cta = tpc;
-          const long long want = ((long long)M + tpc - 1) / tpc;
-          const long long cap = (long long)sms * per_sm;
-          best.ctas = (int)(want < cap ? want : cap);
-        }
+  // (the out-rows in scratch as well only where the slice, somewhat larger than the
+  // rule's, does not fit with them)
+  for (int x = 0; x < 15 && !(x >= 10 && best_score >= 0); ++x) {
+    const int G = 1 << x % 5, cs = x < 5, rs = x < 10;
+    LaunchShape sh{};
+    sh.G = G;
+    sh.cols_in_smem = cs;
+    sh.rows_in_smem = rs;
+    sh.lay = make_layout(n, W, k, kb, nr, G, rs, cs, need_tp, need_gw, need_tq);
+    if (sh.lay.bytes > (size_t)smem_optin) continue;
+    for (int tpc = 1; tpc <= 16; tpc *= 2) {
+      const int threads = 32 * G * tpc;
+      if (threads > 512 || (G > 1 && tpc > 15) || sh.lay.bytes * tpc > (size_t)smem_optin) continue;
+      const int per_sm = period_blocks_per_sm(threads, sh.lay.bytes * tpc);
+      if (per_sm < 1) continue;
+      const double teams_sm = (double)per_sm * tpc;
+      const double busy = (teams_sm < (double)M / sms ? teams_sm : ((double)M / sms > 1 ? (double)M / sms : 1.0)) * G;
+      // (ties as the nested loop over G, then the in-rows' place, decided them)
+      const double score = (busy < 48 ? busy : 48) * 100.0 - G - (cs ? 0.0 : 50.0) - tpc * 0.01;
+      if (score > best_score || (score == best_score && G < best.G)) {
+        best_score = score;
+        best = sh;
+        best.teams_per_cta = tpc;
+        const long long want = ((long long)M + tpc - 1) / tpc;
+        const long long cap = (long long)sms * per_sm;
+        best.ctas = (int)(want < cap ? want : cap);
       }
     }
+  }
   if (best_score < 0) { set_last_error("no launch shape fits this n in shared memory"); return CUSNA_ERR_UNSUPPORTED; }
 
   // ---- scratch layout ----------------------------------------------------
@@ -343,10 +348,12 @@ extern "C" CUSNA_API cusna_status cusna_saom_simulate_period_static(
                oZ0 = b.take((size_t)n * 4), oBk = b.take((size_t)n * 4), oIn = b.take((size_t)W * 4);
   const size_t oKind = b.take((size_t)k * 4), oCfn = b.take((size_t)k * 4),
                oOffd = b.take((size_t)k * 4), oTab = b.take(8);
-  const size_t oProb = b.take(sizeof(DevProblem)), oUnits = b.take(2 * sizeof(long long)),
+  const size_t oRuleProb = b.take(kRuleProblemBytes), oUnits = b.take(2 * sizeof(long long)),
                oCnt = b.take(sizeof(unsigned long long)), oFlag = b.take(sizeof(int));
-  // (beside the fixed-point table and bounds below, which the rule does not count)
+  (void)oRuleProb;
+  // (beside the problem, the fixed-point table and bounds below, which the rule does not count)
   const size_t need = b.off + (rule_cols_smem ? 0 : rule_teams * bits);
+  const size_t oProb = b.take(sizeof(DevProblem));
   const size_t oTabq = b.take(256 * 8), oBound = b.take((size_t)k * 8);
   if (need > kStaticScratchBytes) {
     char buf[200];
@@ -356,10 +363,10 @@ extern "C" CUSNA_API cusna_status cusna_saom_simulate_period_static(
     set_last_error(buf);
     return CUSNA_ERR_UNSUPPORTED;
   }
-  // as many CTAs as the array holds in-rows for
+  // as many CTAs as the array holds in-rows (and out-rows) for
   size_t oCols = 0;
   if (!best.cols_in_smem) {
-    const size_t per_cta = (size_t)best.teams_per_cta * bits;
+    const size_t per_cta = (size_t)best.teams_per_cta * bits * (best.rows_in_smem ? 1 : 2);
     best.ctas = (int)std::min<size_t>(best.ctas, (kStaticScratchBytes + kStaticExtra - b.off) / per_cta);
     if (best.ctas < 1) {
       set_last_error("the no-allocation entry point's scratch holds no team of this problem");
@@ -461,7 +468,9 @@ extern "C" CUSNA_API cusna_status cusna_saom_simulate_period_static(
   SCU(cudaMemcpyAsync(base + oProb, &D, sizeof D, cudaMemcpyHostToDevice, s));
   SCU(cudaMemcpyAsync(base + oUnits, units, sizeof units, cudaMemcpyHostToDevice, s));
   SCU(cudaMemsetAsync(base + oCnt, 0, sizeof(unsigned long long), s));  // work counter starts at 0
-  const Scratch sc{best.cols_in_smem ? nullptr : U32(oCols), nullptr, nullptr, bits / 4, 0};
+  const size_t teams = (size_t)best.ctas * best.teams_per_cta;
+  const Scratch sc{best.cols_in_smem ? nullptr : U32(oCols),
+                   best.rows_in_smem ? nullptr : U32(oCols + teams * bits), nullptr, bits / 4, 0};
   SCU(launch_period(best, (const DevProblem *)(base + oProb), (const long long *)(base + oUnits), 1,
                     (long long)M, (unsigned long long *)(base + oCnt),
                     sc, s));
