@@ -78,6 +78,7 @@ cusna_status ensure_ctx() {
   return CUSNA_OK;
 }
 
+size_t arena_bytes(size_t bytes) { return std::max(bytes + bytes / 4, (size_t)64 << 20); }
 cusna_status ensure_arena(size_t bytes) {
   Ctx &c = g_ctx;
   if (bytes <= c.cap) return CUSNA_OK;
@@ -87,8 +88,7 @@ cusna_status ensure_arena(size_t bytes) {
     c.arena = nullptr;
     c.cap = 0;
   }
-  size_t want = std::max(bytes, (size_t)64 << 20);
-  want = std::max(want, bytes + bytes / 4);
+  const size_t want = arena_bytes(bytes);
   CU(cudaMalloc(&c.arena, want));
   c.cap = want;
   return CUSNA_OK;
@@ -760,30 +760,22 @@ cusna_status fetch_outputs(Job &J) {
   return CUSNA_OK;
 }
 
-// Chooses which two-path counters the chains hold as matrices. A popcount takes
-// W words per alter, a matrix one read per alter and, per toggle, one update for
-// each tie of the two actors. They win where the chip is full of chains (1216 chains
-// with scores: n = 384 93 against 115 ms, n = 448 115 against 170, n = 225 no
-// difference), but not for rounds of a few hundred (512 chains of n = 300 without
-// scores: 15.0 against 13.1 ms), so the line is at kCountsMinW words; and only while
-// the resident teams' matrices stay within kCountsMaxBytes of device memory.
+// Chooses which two-path counters the chains hold as matrices (on; false: none). A
+// popcount takes W words per alter, a matrix one read per alter and, per toggle, one
+// update for each tie of the two actors. Measured: 1216 chains with scores, n = 384 93
+// against 115 ms, n = 448 115 against 170, n = 225 no difference; below twelve words
+// 512 chains of n = 300 without scores 15.0 against 13.1 ms; 1,024 groups of up to
+// 400 actors, one chain each, 36.7 against 37.5 ms with matrices in the largest. So
+// the line is at kCountsMinW words.
 constexpr int kCountsMinW = 12;
-constexpr size_t kCountsMaxBytes = (size_t)8 << 30;
-constexpr size_t kResidentTeams = 152 * 32;
-void choose_counts(std::vector<Job> &jobs, long long total_units, int nets) {
-  size_t per_team = 0;
+void choose_counts(std::vector<Job> &jobs, int nets, bool on) {
   for (Job &J : jobs) {
     CounterSet &C = J.F.cnt;
     C.mask = 0;
-    if (J.p->W >= kCountsMinW)
+    if (on && J.p->W >= kCountsMinW)
       for (int c = 0; c < C.n; ++c)
         if (C.list[c] == CL_OUT || C.list[c] == CL_IN || C.list[c] >= CL_NET) C.mask |= 1u << c;
-    per_team = std::max(per_team, counts_words(C, J.p->n) * 2 * nets);
   }
-  const size_t teams = std::min<size_t>((size_t)total_units, kResidentTeams);
-  const bool fits = per_team * teams <= kCountsMaxBytes;
-  if (!fits)
-    for (Job &J : jobs) J.F.cnt.mask = 0;
   std::vector<const CounterSet *> all;
   for (Job &J : jobs) all.push_back(&J.F.cnt);
   for (size_t q = 0; q < jobs.size(); ++q) {
@@ -814,6 +806,37 @@ struct Needs {
     counts = std::max(counts, counts_words(F.cnt, n));
   }
 };
+
+// The matrices are optional: a launch whose resident teams' matrices exceed
+// counts_cap() (CUSNA_COUNTS_MAX_MB, default 8 GiB), or whose scratch the device has
+// not free, runs with popcounts, which need none of it.
+size_t counts_cap() {
+  const char *e = std::getenv("CUSNA_COUNTS_MAX_MB");
+  const long long mb = e ? std::atoll(e) : 8192;
+  return (size_t)(mb < 0 ? 0 : mb) << 20;
+}
+size_t team_counts_bytes(const Needs &nd, const LaunchShape &x, int nets) {
+  return (size_t)x.ctas * x.teams_per_cta * nd.counts * 2 * nets;
+}
+// The shapes whose matrices the cap allows (all of them without matrices).
+std::vector<LaunchShape> within_cap(const std::vector<LaunchShape> &shapes, const Needs &nd, int nets) {
+  if (!nd.counts) return shapes;
+  std::vector<LaunchShape> out;
+  const size_t cap = counts_cap();
+  for (const LaunchShape &x : shapes)
+    if (team_counts_bytes(nd, x, nets) <= cap) out.push_back(x);
+  return out;
+}
+// Whether an allocation that holds matrices can be made beside `held` bytes that it
+// replaces.
+bool device_has(size_t bytes, size_t held) {
+  size_t free = 0, total = 0;
+  if (cudaMemGetInfo(&free, &total) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return bytes <= free + held;
+}
 
 // ---- launch-shape autotuner ---------------------------------------------------
 // The simulator is bound by the float64 pipe, whose instructions have long
@@ -1015,8 +1038,9 @@ void tuner_record(const TuneKey &key, int trial, float ms) {
 
 // Register limit check of a shape: the kernel is compiled for 512 threads with
 // the full register file, so any CTA size up to 512 fits.
-cusna_status run_jobs(std::vector<Job> &jobs, bool dev, cusna_gpu_options *opts,
-                      const cusna_validation_options *vo = nullptr) {
+// *retry: the matrices do not fit (nothing has run).
+cusna_status run_jobs_as(std::vector<Job> &jobs, bool dev, cusna_gpu_options *opts,
+                         const cusna_validation_options *vo, bool *retry) {
   cusna_status s;
   if ((s = ensure_ctx()) != CUSNA_OK) return s;
   if (opts && opts->stream) {
@@ -1044,9 +1068,14 @@ cusna_status run_jobs(std::vector<Job> &jobs, bool dev, cusna_gpu_options *opts,
   JitKernel jk;
   // the validation build is the library kernel's
   const bool use_jit = !valid && jit_for(jobs, opts ? opts->specialise : 0, &jk);
-  std::vector<LaunchShape> ranked =
+  const std::vector<LaunchShape> fitting =
       rank_shapes(nmax, Wmax, kmax, kbmax, nrmax, nd, total, fG, fT, 1,
                   use_jit ? &jk : nullptr, valid);
+  const std::vector<LaunchShape> ranked = within_cap(fitting, nd, 1);
+  if (!fitting.empty() && ranked.empty()) {
+    *retry = true;
+    return CUSNA_OK;
+  }
   if (ranked.empty()) {
     set_err("no launch shape fits n=%d in shared memory", nmax);
     return CUSNA_ERR_UNSUPPORTED;
@@ -1073,7 +1102,14 @@ cusna_status run_jobs(std::vector<Job> &jobs, bool dev, cusna_gpu_options *opts,
   const size_t o_cols = sh.cols_in_smem ? NONE : pl.take(teams * cols_words * 4);
   const size_t o_rows = sh.rows_in_smem ? NONE : pl.take(teams * cols_words * 4);
   const size_t o_counts = nd.counts ? pl.take(teams * nd.counts * 2) : NONE;
-  if ((s = ensure_arena(pl.off)) != CUSNA_OK) return s;
+  if (nd.counts && pl.off > g_ctx.cap && !device_has(arena_bytes(pl.off), g_ctx.cap)) {
+    *retry = true;
+    return CUSNA_OK;
+  }
+  if ((s = ensure_arena(pl.off)) != CUSNA_OK) {
+    *retry = nd.counts > 0;
+    return s;
+  }
 
   std::vector<DevProblem> hp(jobs.size());
   std::vector<long long> units(jobs.size() + 1, 0);
@@ -1134,13 +1170,19 @@ cusna_status run_jobs(std::vector<Job> &jobs, bool dev, cusna_gpu_options *opts,
   return CUSNA_OK;
 }
 
-void order_longest_first(std::vector<Job> &jobs);
-
-long long total_chains(const std::vector<Job> &jobs) {
-  long long t = 0;
-  for (const Job &J : jobs) t += J.p->M;
-  return t;
+cusna_status run_jobs(std::vector<Job> &jobs, bool dev, cusna_gpu_options *opts,
+                      const cusna_validation_options *vo = nullptr) {
+  bool retry = false;
+  choose_counts(jobs, 1, true);
+  cusna_status s = run_jobs_as(jobs, dev, opts, vo, &retry);
+  if (!retry) return s;
+  cudaGetLastError();
+  g_err.clear();
+  choose_counts(jobs, 1, false);
+  return run_jobs_as(jobs, dev, opts, vo, &retry);
 }
+
+void order_longest_first(std::vector<Job> &jobs);
 
 cusna_status simulate(const cusna_saom_problem *problems, cusna_saom_result *results, int count,
                       cusna_gpu_options *opts) {
@@ -1163,7 +1205,6 @@ cusna_status simulate(const cusna_saom_problem *problems, cusna_saom_result *res
   }
   if ((s = ensure_ctx()) != CUSNA_OK) return s;
   order_longest_first(jobs);
-  choose_counts(jobs, total_chains(jobs), 1);
   s = run_jobs(jobs, dev, opts);
   if (s == CUSNA_OK && opts) {
     long long tot = 0;
@@ -1203,9 +1244,10 @@ struct MultiNet {
 
 // check_only: validate and compile the specialised kernel (no device), with
 // the compiler log in *log and the compile time in *seconds.
-cusna_status simulate_multi(const cusna_saom_multi_problem *pb, cusna_saom_multi_result *r,
-                            bool check_only = false, std::string *log = nullptr,
-                            double *seconds = nullptr) {
+// counts: with count matrices; *retry: they do not fit (nothing has run).
+cusna_status simulate_multi_as(const cusna_saom_multi_problem *pb, cusna_saom_multi_result *r,
+                               bool check_only, std::string *log, double *seconds, bool counts,
+                               bool *retry) {
   if (!pb || !r) { set_err("problem or result is NULL"); return CUSNA_ERR_NULL_ARG; }
   if (pb->struct_version != CUSNA_ABI_VERSION || r->struct_version != CUSNA_ABI_VERSION) {
     set_err("struct_version %d/%d != %d", pb->struct_version, r->struct_version, CUSNA_ABI_VERSION);
@@ -1302,7 +1344,7 @@ cusna_status simulate_multi(const cusna_saom_multi_problem *pb, cusna_saom_multi
     if (s != CUSNA_OK) return s;
     kmax = std::max(kmax, kd);
   }
-  choose_counts(jobs, M, D);
+  choose_counts(jobs, D, counts);
   for (const Job &J : jobs) nd.add(J.F, n);
   // the multi-network kernel specialised to the networks' effect plans
   std::vector<JitPlan> jplans;
@@ -1323,8 +1365,13 @@ cusna_status simulate_multi(const cusna_saom_multi_problem *pb, cusna_saom_multi
   cudaStream_t st = g_ctx.stream;
   JitKernel jk;
   const bool use_jit = jit_get(mspec, &jk);
-  const std::vector<LaunchShape> ranked =
+  const std::vector<LaunchShape> fitting =
       rank_shapes(n, W, kmax, 0, 0, nd, M, 0, 0, D, use_jit ? &jk : nullptr);
+  const std::vector<LaunchShape> ranked = within_cap(fitting, nd, D);
+  if (!fitting.empty() && ranked.empty()) {
+    *retry = true;
+    return CUSNA_OK;
+  }
   if (ranked.empty()) {
     set_err("no launch shape fits %d networks of n=%d", D, n);
     return CUSNA_ERR_UNSUPPORTED;
@@ -1351,7 +1398,14 @@ cusna_status simulate_multi(const cusna_saom_multi_problem *pb, cusna_saom_multi
   const size_t o_cols = sh.cols_in_smem ? NONE : pl.take(teams * D * cols_words * 4);
   const size_t o_rows = sh.rows_in_smem ? NONE : pl.take(teams * D * cols_words * 4);
   const size_t o_counts = nd.counts ? pl.take(teams * D * nd.counts * 2) : NONE;
-  if ((s = ensure_arena(pl.off)) != CUSNA_OK) return s;
+  if (nd.counts && pl.off > g_ctx.cap && !device_has(arena_bytes(pl.off), g_ctx.cap)) {
+    *retry = true;
+    return CUSNA_OK;
+  }
+  if ((s = ensure_arena(pl.off)) != CUSNA_OK) {
+    *retry = nd.counts > 0;
+    return s;
+  }
   std::vector<DevProblem> hp(D);
   for (int d = 0; d < D; ++d)
     if ((s = prepare(jobs[d], false, hp[d], 0)) != CUSNA_OK) return s;
@@ -1402,6 +1456,17 @@ cusna_status simulate_multi(const cusna_saom_multi_problem *pb, cusna_saom_multi
   return CUSNA_OK;
 }
 
+cusna_status simulate_multi(const cusna_saom_multi_problem *pb, cusna_saom_multi_result *r,
+                            bool check_only = false, std::string *log = nullptr,
+                            double *seconds = nullptr) {
+  bool retry = false;
+  const cusna_status s = simulate_multi_as(pb, r, check_only, log, seconds, true, &retry);
+  if (!retry) return s;
+  cudaGetLastError();
+  g_err.clear();
+  return simulate_multi_as(pb, r, check_only, log, seconds, false, &retry);
+}
+
 }  // namespace
 
 }  // namespace cusna
@@ -1446,8 +1511,9 @@ void plan_free(cusna_saom_plan *P) {
   delete P;
 }
 
-cusna_status plan_create(const cusna_saom_problem *problems, cusna_saom_result *results, int count,
-                         int shared_params, cusna_saom_plan **out) {
+// counts: with count matrices; *retry: they do not fit (nothing has been made).
+cusna_status plan_create_as(const cusna_saom_problem *problems, cusna_saom_result *results, int count,
+                            int shared_params, cusna_saom_plan **out, bool counts, bool *retry) {
   if (!problems || !results || !out) { set_err("problems, results and plan are required"); return CUSNA_ERR_NULL_ARG; }
   *out = nullptr;
   if (count < 1) { set_err("count %d < 1", count); return CUSNA_ERR_SHAPE; }
@@ -1464,7 +1530,7 @@ cusna_status plan_create(const cusna_saom_problem *problems, cusna_saom_result *
     if (!one) jobs[q].F.flags &= ~F_THETA_TAB;
   }
   order_longest_first(jobs);
-  choose_counts(jobs, total_chains(jobs), 1);
+  choose_counts(jobs, 1, counts);
   int nmax = 0, Wmax = 0, kmax = 0, kbmax = 0, nrmax = 0;
   Needs nd;
   long long total = 0;
@@ -1474,8 +1540,13 @@ cusna_status plan_create(const cusna_saom_problem *problems, cusna_saom_result *
     nd.add(J.F, J.p->n);
     total += J.p->M;
   }
-  const std::vector<LaunchShape> ranked =
+  const std::vector<LaunchShape> fitting =
       rank_shapes(nmax, Wmax, kmax, kbmax, nrmax, nd, total, 0, 0);
+  const std::vector<LaunchShape> ranked = within_cap(fitting, nd, 1);
+  if (!fitting.empty() && ranked.empty()) {
+    *retry = true;
+    return CUSNA_OK;
+  }
   if (ranked.empty()) { set_err("no launch shape fits n=%d", nmax); return CUSNA_ERR_UNSUPPORTED; }
   std::vector<LaunchShape> cand = tuning_candidates(ranked);
   {
@@ -1483,7 +1554,8 @@ cusna_status plan_create(const cusna_saom_problem *problems, cusna_saom_result *
     const TuneKey key = tune_key(nmax, Wmax, kmax, kbmax, nrmax, nd, total);
     std::lock_guard<std::mutex> lk(g_tune_mu);
     for (auto &e : g_tune)
-      if (std::memcmp(&e.key, &key, sizeof key) == 0 && e.next >= e.cand.size() && e.best >= 0)
+      if (std::memcmp(&e.key, &key, sizeof key) == 0 && e.next >= e.cand.size() && e.best >= 0 &&
+          !within_cap({e.cand[e.best]}, nd, 1).empty())
         cand = {e.cand[e.best]};
   }
   if (!tuning_enabled()) cand.resize(1);
@@ -1525,9 +1597,10 @@ cusna_status plan_create(const cusna_saom_problem *problems, cusna_saom_result *
     return CUSNA_ERR_CUDA;
   }
   P->device = g_ctx.device;
-  if (cudaMalloc(&P->mem, pl.off) != cudaSuccess) {
+  if ((nd.counts && !device_has(pl.off, 0)) || cudaMalloc(&P->mem, pl.off) != cudaSuccess) {
     cudaGetLastError();
     plan_free(P);
+    *retry = nd.counts > 0;
     set_err("plan: cudaMalloc of %zu bytes failed", pl.off);
     return CUSNA_ERR_CUDA;
   }
@@ -1583,6 +1656,15 @@ cusna_status plan_create(const cusna_saom_problem *problems, cusna_saom_result *
   P->spec = launch_spec(jobs);
   *out = P;
   return CUSNA_OK;
+}
+
+cusna_status plan_create(const cusna_saom_problem *problems, cusna_saom_result *results, int count,
+                         int shared_params, cusna_saom_plan **out) {
+  bool retry = false;
+  const cusna_status s = plan_create_as(problems, results, count, shared_params, out, true, &retry);
+  if (!retry) return s;
+  g_err.clear();
+  return plan_create_as(problems, results, count, shared_params, out, false, &retry);
 }
 
 // Kernel launches only (capture-safe): epoch and term tables, work counter,
@@ -1731,7 +1813,6 @@ CUSNA_API cusna_status cusna_saom_simulate_period_validate(const cusna_saom_prob
   if (s != CUSNA_OK) return s;
   if ((s = ensure_ctx()) != CUSNA_OK) return s;
   std::vector<Job> jobs(1, J);
-  choose_counts(jobs, total_chains(jobs), 1);
   return run_jobs(jobs, false, nullptr, vo);
 }
 
@@ -1755,7 +1836,7 @@ CUSNA_API cusna_status cusna_saom_specialise_check(const cusna_saom_problem *pro
   jobs[0].r = &dummy;
   cusna_status s = validate(problem, &dummy, false, jobs[0].F);
   if (s != CUSNA_OK) return s;
-  choose_counts(jobs, problem->M, 1);
+  choose_counts(jobs, 1, true);
   std::string text;
   double sec = 0.0;
   const int st = jit_compile_only(jobs[0].F.spec_w, &text, &sec);
