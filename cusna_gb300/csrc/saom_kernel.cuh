@@ -396,7 +396,8 @@ __device__ __forceinline__ void tp_masks(const Team &T, const DevProblem &P, con
   const CountRow R = count_row(P, S, X, n, W, c);
   for (int hb = 32 * T.warp; hb < W * 32; hb += T.L) {
     const int h = hb + T.lane;
-    const int v = h < n ? count_of(R, n, W, h) : -1;
+    // (a matrix's diagonal is not kept up; the actor itself counts where it has a self-tie)
+    const int v = h >= n ? -1 : (R.cm && h == X.i ? pc2(S.rows, h, S.cols, h, n, W) : count_of(R, n, W, h));
     const uint32_t z0 = __ballot_sync(kFull, v == 0), z1 = __ballot_sync(kFull, v == 1);
     if (T.lane == 0) { S.tpeq[hb >> 5] = z0; S.tpeq[W + (hb >> 5)] = z1; }
   }
