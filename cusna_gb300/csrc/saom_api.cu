@@ -839,9 +839,8 @@ bool device_has(size_t bytes, size_t held) {
 }
 
 // ---- launch-shape autotuner ---------------------------------------------------
-// The simulator is bound by the float64 pipe, whose instructions have long
-// latencies, so the shape that wins keeps the most warps resident per SM while
-// every resident team has a chain to run. For each team size G (warps per
+// The simulator is bound by instruction latency, so the shape that wins tends to keep
+// the most warps resident per SM while every resident team has a chain to run. For each team size G (warps per
 // chain), chain state in shared memory or in-rows in global scratch, and teams
 // per CTA, the CUDA occupancy calculator gives the resident CTAs per SM (shared
 // memory, registers and warps all count). The score is the number of warps that

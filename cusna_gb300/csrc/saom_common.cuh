@@ -215,8 +215,8 @@ __device__ __forceinline__ double dunkey(long long k) {
   return __longlong_as_double(b);
 }
 
-// float32 estimate of log(-log(u)), u = (x + 0.5) 2^-32, used to shortlist the
-// Gumbel-max candidates. Error bound (from the documented <= 1 ulp error of
+// float32 estimate of log(-log(u)), u = (x + 0.5) 2^-32, by CUDA's logf and log1pf: the
+// yardstick in float32 of gumbel_est below, which the kernels use. Error bound (from the documented <= 1 ulp error of
 // logf/log1pf and the 2^-24 rounding of the inputs):
 //   L = -log(u) is estimated with relative error < 5e-7 (for u >= 1/2 through
 //   log1p of v = 1 - u, which is formed exactly from ~x), and log(L) lies in

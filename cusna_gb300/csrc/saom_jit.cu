@@ -287,8 +287,8 @@ void gen_functions(Gen &g, const JitPlan &J, const std::string &sfx, bool multi)
       g.s += "    v = 0.0;\n    has_term = false;\n";
     } else if (multi && kind == K_CROSS) {
       gen_cross(g, e, cfn, ca);
-      g.put("    v = flip((%d == 36 && S.p1[%d] >= 2.0) ? sqrt(i2d(c)) : i2d(c), sg);\n"
-            "    if (TERMS) term = __dmul_rn(S.th[%d], v);\n", cfn, e, e);
+      g.put("    v = flip(i2d(c), sg);\n"
+            "    if (TERMS) term = __dmul_rn(S.th[%d], v);\n", e);
     } else {
       g.put("    v = gen_stat(P, S, X, %d, j, aij, aji, %s, d);\n"
             "    if (TERMS) term = __dmul_rn(S.th[%d], v);\n", e, gen_cnt_arg(ca).c_str(), e);

@@ -661,8 +661,7 @@ __device__ __forceinline__ double change_stats(const DevProblem &P, const Slice 
       v = 0.0;
       has_term = false;
     } else if (MULTI && kind == K_CROSS) {
-      const int c = cross_count(P, S, X, n, cfn, S.eoffd[e], ca, i, j);
-      v = flip((cfn == 36 && S.p1[e] >= 2.0) ? sqrt(i2d(c)) : i2d(c), sg);
+      v = flip(i2d(cross_count(P, S, X, n, cfn, S.eoffd[e], ca, i, j)), sg);
       if (TERMS) term = __dmul_rn(S.th[e], v);
     } else {
       v = gen_stat(P, S, X, e, j, aij, aji, ca != 0xFF ? cnt(ca) : 0, d);

@@ -121,7 +121,7 @@ __device__ void chain_finish(const Team &T, const DevProblem &P, const Slice &S,
 // Persistent period kernel: every team repeatedly takes the next chain of the
 // launch's work list (all chains of all problems) until the list is empty.
 // MAXT is the largest CTA the instantiation serves: 256 threads with a register
-// budget for three CTAs per SM (teams of up to 8 warps), or 512 (16-warp teams).
+// budget for two CTAs per SM (CUSNA_MINB_256), or 512.
 #ifndef CUSNA_MINB_256
 #define CUSNA_MINB_256 2  // resident 256-thread CTAs per SM the register budget allows
 #endif

@@ -160,7 +160,7 @@ __global__ void prep_bits_kernel(const uint32_t *src, int n, int W, uint32_t *ds
 }
 
 // Start values of the counters that chains hold as matrices, for every problem
-// of a launch (block y = problem): cell (i, j) by popcounts, as count_pc forms it
+// of a launch (block y = problem): cell (i, j) by popcounts, as count_of forms it
 // for a ministep of i. Networks w of a multi-network problem are the launch's
 // problems w.
 __global__ void __launch_bounds__(256) counts_init_kernel(const DevProblem *__restrict__ probs,
@@ -334,7 +334,8 @@ cudaError_t launch_netstats(const uint8_t *a, int M, const StatDesc &D, double *
                             cudaStream_t st) {
   const size_t nets = al16((size_t)2 * D.W * D.n * 4 + (size_t)2 * D.n * 4) + 16;
   if (nets + 304 > 200 * 1024) return cudaErrorInvalidValue;
-  // scratch for as many statistics at a time as fit (at least two)
+  // scratch for as many statistics at a time as fit (at least two: with them a network
+  // that just passes takes 288 bytes more than 200 KiB, which an SM has)
   int rows = D.k < 32 ? D.k : 32;
   while (rows > 2 && nets + stat_scratch(rows) * 8 > 200 * 1024) --rows;
   if (rows < 2) rows = 2;

@@ -279,7 +279,8 @@ extern "C" CUSNA_API cusna_status cusna_saom_simulate_period_static(
   // Which problems fit is a rule of its own, not of the kernel's footprint in
   // this build: the in-rows' scratch is counted for the teams that a kernel of
   // 128 registers (512 threads per SM) and scratch_rule_slice() bytes per team
-  // would keep resident. The launch below never has more teams than that.
+  // would keep resident. The launch's own CTAs are bounded by the bytes that are left
+  // (below), so it may have fewer or more teams.
   double rule_score = -1.0;
   size_t rule_teams = 0;
   bool rule_cols_smem = false;
