@@ -255,8 +255,9 @@ CUSNA_API cusna_status cusna_saom_simulate_batch(
  * (alter j's Gumbel draw). Later ministeps draw from Philox as usual.
  *
  * lse64 = 1 forms the score sums in float64 at every ministep, as the
- * reference does (otherwise in 64-bit fixed point, with float64 only for
- * chains whose parameters leave its range). warps_per_chain / chains_per_cta (0: chosen by
+ * reference does (otherwise in 64-bit fixed point, with float64 for
+ * chains whose parameters leave its range and for ministeps with a sum that is short
+ * of bits). warps_per_chain / chains_per_cta (0: chosen by
  * the library) force the launch shape; the validation build runs CTAs of at
  * most 256 threads. The call runs the library's own kernel, never a
  * specialised one, and no result depends on the launch shape. */
