@@ -233,7 +233,9 @@ cusna_status build_plan(const cusna_saom_problem *p, bool dev, Facts &F, bool on
       top = std::max(top, std::fabs(v));
       finite = finite && std::isfinite(v);
     }
-    F.bound[e] = finite ? top : INFINITY;   // not finite: the chains run in float64
+    // not finite, or beyond the scales: the chains run in float64
+    finite = finite && (top == 0.0 || (top >= 1e-250 && top <= 1e250));
+    F.bound[e] = finite ? top : INFINITY;
     const double scale = std::ldexp(1.0, fx_scale(finite ? top : 1.0));
     F.poolq.resize(F.pool.size(), 0);
     for (size_t x = 0; x < size; ++x)

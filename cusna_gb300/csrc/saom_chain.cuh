@@ -63,7 +63,10 @@ __device__ __forceinline__ void chain_scales(const DevProblem &P, const Slice &S
       S.dstar[e] = bound;
       S.esd[e] = fx_scale(bound);
       S.ecls[e] = cls | (S.th[e] < 0.0 ? 256 : 0);
-      if (cls != FX_ZERO) range = __dadd_rn(range, __dmul_rn(fabs(S.th[e]), bound));
+      // (scales of bounds beyond these powers of ten would leave pow2's range)
+      const bool scaled = bound == 0.0 || (bound >= 1e-250 && bound <= 1e250);
+      if (cls != FX_ZERO)
+        range = __dadd_rn(range, scaled ? __dmul_rn(fabs(S.th[e]), bound) : (double)INFINITY);
     }
     if (range < 16384.0 || !(cap / 2 >= mb)) break;
   }
